@@ -19,10 +19,29 @@ namespace bfly {
 namespace dev {
 
 // ------------------------------------------------------------------ complex helpers
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
+// Sums, differences and real multiples of a complex value act on both halves alike, so they are
+// issued as packed two-wide fp32 instructions (one per complex value; each half rounds as the
+// scalar instruction does).  Products by +-i and by a general twiddle cross the halves and stay
+// scalar: packing them would spend the saved instruction on register moves.
+__device__ __forceinline__ float2 f2(float s) { return make_float2(s, s); }
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }
+__device__ __forceinline__ float2 cscale(float2 a, float s) { return __fmul2_rn(a, f2(s)); }
+__device__ __forceinline__ float2 cfma(float2 a, float s, float2 c) { return __ffma2_rn(a, f2(s), c); }   // s a + c
 __device__ __forceinline__ float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
+// a + s*d*w and a - s*d*w with w = -i (forward) or +i (INV), s a constant.
+template <bool INV>
+__device__ __forceinline__ void add_sub_i(float2 a, float2 d, float s, float2& plus, float2& minus) {
+    const float h = INV ? -s : s;
+    plus = make_float2(fmaf(h, d.y, a.x), fmaf(-h, d.x, a.y));
+    minus = make_float2(fmaf(-h, d.y, a.x), fmaf(h, d.x, a.y));
+}
+template <bool INV>
+__device__ __forceinline__ void add_sub_i(float2 a, float2 d, float2& plus, float2& minus) {
+    const float2 p = make_float2(a.x + d.y, a.y - d.x), m = make_float2(a.x - d.y, a.y + d.x);
+    plus = INV ? m : p;
+    minus = INV ? p : m;
+}
 // a * w (CONJ=false) or a * conj(w) (CONJ=true)
 template <bool CONJ>
 __device__ __forceinline__ float2 cmul(float2 a, float2 w) {
@@ -84,64 +103,149 @@ template <bool INV> struct DFT<2, INV> {
 template <bool INV> struct DFT<4, INV> {
     static __device__ __forceinline__ void run(float2* v) {
         const float2 t0 = cadd(v[0], v[2]), t1 = csub(v[0], v[2]);
-        const float2 t2 = cadd(v[1], v[3]);
-        float2 t3 = csub(v[1], v[3]);
-        t3 = INV ? make_float2(-t3.y, t3.x) : make_float2(t3.y, -t3.x);  // * (+-i)
+        const float2 t2 = cadd(v[1], v[3]), t3 = csub(v[1], v[3]);
         v[0] = cadd(t0, t2);
         v[2] = csub(t0, t2);
-        v[1] = cadd(t1, t3);
-        v[3] = csub(t1, t3);
+        add_sub_i<INV>(t1, t3, v[1], v[3]);
     }
 };
 
-template <int A, int B, int R, bool INV, int K1 = 0, int N2 = 0>
-__device__ __forceinline__ void twiddle_split_impl(float2* v) {
-    if constexpr (K1 < A) {
-        if constexpr (N2 < B) {
-            v[B * K1 + N2] = rot<K1 * N2, R, INV>(v[B * K1 + N2]);
-            twiddle_split_impl<A, B, R, INV, K1, N2 + 1>(v);
-        } else {
-            twiddle_split_impl<A, B, R, INV, K1 + 1, 0>(v);
+// DFT4 of (a0, w a1, w^2 a2, w^3 a3) for w = W_8: the eighth roots are a sum and a difference
+// times sqrt(1/2), and that factor rides on the sums after them as a multiply-add.
+template <bool INV>
+__device__ __forceinline__ void dft4_w8(float2* v) {
+    constexpr float H = 0.70710678118654752440f;   // sqrt(1/2)
+    float2 t0, t1;
+    add_sub_i<INV>(v[0], v[2], t0, t1);   // W_8^2 = -i (INV: +i)
+    // H*u1 = W_8 a1, H*u3 = W_8^3 a3
+    const float2 u1 = INV ? make_float2(v[1].x - v[1].y, v[1].x + v[1].y) : make_float2(v[1].x + v[1].y, v[1].y - v[1].x);
+    const float2 u3 = INV ? make_float2(-v[3].x - v[3].y, v[3].x - v[3].y) : make_float2(v[3].y - v[3].x, -v[3].x - v[3].y);
+    const float2 s = cadd(u1, u3), d = csub(u1, u3);
+    v[0] = cfma(s, H, t0);
+    v[2] = cfma(s, -H, t0);
+    add_sub_i<INV>(t1, d, H, v[1], v[3]);
+}
+
+// DFT4 of (a0, w a1, w^2 a2, w^3 a3) for w = W_16^K, K = 1 or 3 (w^2 an odd eighth root).
+template <int K, bool INV>
+__device__ __forceinline__ void dft4_w16(float2* v) {
+    constexpr float H = 0.70710678118654752440f;
+    const float2 a = rot<K, 16, INV>(v[1]), b = rot<3 * K, 16, INV>(v[3]);
+    const float x = v[2].x, y = v[2].y;   // H*u = W_16^(2K) a2
+    const float2 u = K == 1 ? (INV ? make_float2(x - y, x + y) : make_float2(x + y, y - x))
+                            : (INV ? make_float2(-x - y, x - y) : make_float2(y - x, -x - y));
+    const float2 t0 = cfma(u, H, v[0]), t1 = cfma(u, -H, v[0]);
+    const float2 t2 = cadd(a, b), t3 = csub(a, b);
+    v[0] = cadd(t0, t2);
+    v[2] = csub(t0, t2);
+    add_sub_i<INV>(t1, t3, v[1], v[3]);
+}
+
+// 8 = 2 x 4 and 16 = 4 x 4 Cooley-Tukey, input n = B n1 + n2, output k = k1 + A k2; the inner
+// twiddles W_R^(n2 k1) are part of the second stage's butterflies.  A DFT16 is 106 fp32
+// instructions (160 with scalar sums): k_c2c n = 4096 executes 21.9 M against 29.1 M per 2^24
+// points, with the constant exchange offsets of Team::at_off.
+template <bool INV> struct DFT<8, INV> {
+    static __device__ __forceinline__ void run(float2* v) {
+        float2 a[4], b[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            a[j] = cadd(v[j], v[4 + j]);
+            b[j] = csub(v[j], v[4 + j]);
+        }
+        DFT<4, INV>::run(a);
+        dft4_w8<INV>(b);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            v[2 * k] = a[k];
+            v[2 * k + 1] = b[k];
         }
     }
-}
-template <int A, int B, int R, bool INV>
-__device__ __forceinline__ void twiddle_split(float2* v) { twiddle_split_impl<A, B, R, INV>(v); }
-
-// R = A*B Cooley-Tukey in registers. Input n = B*n1 + n2, output k = k1 + A*k2.
-template <int A, int B, bool INV>
-__device__ __forceinline__ void dft_split(float2* v) {
-    constexpr int R = A * B;
-#pragma unroll
-    for (int n2 = 0; n2 < B; ++n2) {
-        float2 col[A];
-#pragma unroll
-        for (int n1 = 0; n1 < A; ++n1) col[n1] = v[B * n1 + n2];
-        DFT<A, INV>::run(col);
-#pragma unroll
-        for (int k1 = 0; k1 < A; ++k1) v[B * k1 + n2] = col[k1];
-    }
-    // twiddles w_R^(n2*k1): unrolled with compile-time exponents
-    twiddle_split<A, B, R, INV>(v);
-    float2 out[R];
-#pragma unroll
-    for (int k1 = 0; k1 < A; ++k1) {
-        float2 row[B];
-#pragma unroll
-        for (int n2 = 0; n2 < B; ++n2) row[n2] = v[B * k1 + n2];
-        DFT<B, INV>::run(row);
-#pragma unroll
-        for (int k2 = 0; k2 < B; ++k2) out[k1 + A * k2] = row[k2];
-    }
-#pragma unroll
-    for (int i = 0; i < R; ++i) v[i] = out[i];
-}
-
-template <bool INV> struct DFT<8, INV> {
-    static __device__ __forceinline__ void run(float2* v) { dft_split<2, 4, INV>(v); }
 };
+template <bool INV>
+__device__ __forceinline__ void dft16_rows(float2 (&y)[4][4], float2* v) {   // y[k1][n2]
+    DFT<4, INV>::run(y[0]);
+    dft4_w16<1, INV>(y[1]);
+    dft4_w8<INV>(y[2]);
+    dft4_w16<3, INV>(y[3]);
+#pragma unroll
+    for (int k1 = 0; k1 < 4; ++k1)
+#pragma unroll
+        for (int k2 = 0; k2 < 4; ++k2) v[k1 + 4 * k2] = y[k1][k2];
+}
 template <bool INV> struct DFT<16, INV> {
-    static __device__ __forceinline__ void run(float2* v) { dft_split<4, 4, INV>(v); }
+    static __device__ __forceinline__ void run(float2* v) {
+        float2 y[4][4];
+#pragma unroll
+        for (int n2 = 0; n2 < 4; ++n2) {
+            float2 c[4] = {v[n2], v[4 + n2], v[8 + n2], v[12 + n2]};
+            DFT<4, INV>::run(c);
+#pragma unroll
+            for (int k1 = 0; k1 < 4; ++k1) y[k1][n2] = c[k1];
+        }
+        dft16_rows<INV>(y, v);
+    }
+};
+
+// DFT16 of eight values and eight zeros: v[8..15] are zero whatever they hold.
+template <bool INV>
+__device__ __forceinline__ void dft16_low(float2* v) {
+    float2 y[4][4];
+#pragma unroll
+    for (int n2 = 0; n2 < 4; ++n2) {
+        const float2 a = v[n2], b = v[4 + n2];
+        y[0][n2] = cadd(a, b);
+        y[2][n2] = csub(a, b);
+        add_sub_i<INV>(a, b, y[1][n2], y[3][n2]);
+    }
+    dft16_rows<INV>(y, v);
+}
+
+// a * exp(-+2*pi*i*Q/32), Q compile-time.
+template <int Q, bool INV>
+__device__ __forceinline__ float2 rot32(float2 a) {
+    if constexpr (Q % 2 == 0) {
+        return rot<Q / 2, 16, INV>(a);
+    } else {
+        constexpr int q = Q % 32;
+        constexpr int m = q % 16 > 8 ? 16 - q % 16 : q % 16;   // angle folded into the first quadrant
+        constexpr float C1 = 0.98078528040323044913f, S1 = 0.19509032201612826785f;   // cos, sin of pi/16
+        constexpr float C3 = 0.83146961230254523708f, S3 = 0.55557023301960222474f;   // of 3 pi/16
+        constexpr float c0 = m == 1 ? C1 : m == 3 ? C3 : m == 5 ? S3 : S1;
+        constexpr float s0 = m == 1 ? S1 : m == 3 ? S3 : m == 5 ? C3 : C1;
+        constexpr float c = (q < 8 || q > 24) ? c0 : -c0;
+        constexpr float s = (q < 16) != INV ? s0 : -s0;
+        return make_float2(fmaf(a.x, c, a.y * s), fmaf(a.y, c, -(a.x * s)));
+    }
+}
+template <int K1, bool INV, int N2 = 1>
+__device__ __forceinline__ void twiddle32(float2* v) {   // v[n2] *= W_32^(K1 n2), n2 < 8
+    if constexpr (N2 < 8) {
+        v[N2] = rot32<K1 * N2, INV>(v[N2]);
+        twiddle32<K1, INV, N2 + 1>(v);
+    }
+}
+// 32 = 4 x 8.
+template <bool INV> struct DFT<32, INV> {
+    static __device__ __forceinline__ void run(float2* v) {
+        float2 y[4][8];
+#pragma unroll
+        for (int n2 = 0; n2 < 8; ++n2) {
+            float2 c[4] = {v[n2], v[8 + n2], v[16 + n2], v[24 + n2]};
+            DFT<4, INV>::run(c);
+#pragma unroll
+            for (int k1 = 0; k1 < 4; ++k1) y[k1][n2] = c[k1];
+        }
+        twiddle32<1, INV>(y[1]);
+        twiddle32<2, INV>(y[2]);
+        twiddle32<3, INV>(y[3]);
+#pragma unroll
+        for (int k1 = 0; k1 < 4; ++k1) {
+            DFT<8, INV>::run(y[k1]);
+#pragma unroll
+            for (int k2 = 0; k2 < 8; ++k2) v[k1 + 4 * k2] = y[k1][k2];
+        }
+    }
 };
 
 // ------------------------------------------------------------------ pass schedule
@@ -152,7 +256,7 @@ __host__ __device__ constexpr int ilog2c(int n) { return n <= 1 ? 0 : 1 + ilog2c
 template <int N, int E>
 struct Sched {
     static_assert((N & (N - 1)) == 0 && N >= 2, "N must be a power of two");
-    static_assert(E == 2 || E == 4 || E == 8 || E == 16, "E must be 2,4,8,16");
+    static_assert(E == 2 || E == 4 || E == 8 || E == 16 || E == 32, "E must be 2,4,8,16,32");
     static_assert(N >= E, "N must be >= E");
     static constexpr int T = N / E;                      // threads per transform
     static constexpr int LOGN = ilog2c(N), LOGE = ilog2c(E);
@@ -236,6 +340,25 @@ struct Team {
         else return i * ESTRIDE;
     }
 
+    // Where at(base + off) lies, given a = at(base): the padding adds up exactly when off is a
+    // multiple of 16, or base is one (16 | STEP, the divisor that the caller knows of base), so the
+    // elements of a butterfly are constant offsets from one address.  Other cases recompute.
+    template <int OFFSTEP, int STEP>
+    static __device__ __forceinline__ int at_off(int base, int a, int off) {
+        if constexpr (ESTRIDE != 0) return a + off * ESTRIDE;
+        else if constexpr (OFFSTEP % 16 == 0 || STEP % 16 == 0) return a + spad(off);
+        else return spad(base + off);
+    }
+    // Element r of butterfly j as pass p stores it, and as pass p loads it.
+    template <int p>
+    static __device__ __forceinline__ int out_at(int base, int a, int r) {
+        return at_off<S::ns(p), S::ns(p) == 1 ? S::radix(p) : 1>(base, a, r * S::ns(p));
+    }
+    template <int p>
+    static __device__ __forceinline__ int in_at(int j, int a, int r) {
+        return at_off<N / S::radix(p), 1>(j, a, r * (N / S::radix(p)));
+    }
+
     static __device__ __forceinline__ void sync(int row) { team_sync<SYNC>(row, T); }
 
     template <class Load>
@@ -248,9 +371,11 @@ struct Team {
             for (int r = 0; r < R; ++r) v[s * R + r] = load(t + s * T + r * (N / R));
     }
 
+    // The steps of pass p: twiddles and DFTs in registers, the results to the exchange buffer, the
+    // next pass's inputs back from it.  A kernel may take them apart to hold another t after an
+    // exchange than before it.
     template <int p>
-    static __device__ __forceinline__ void passes(float2 (&v)[E], float2* sm,
-                                                  const float2* __restrict__ tw, int t, int row) {
+    static __device__ __forceinline__ void butterflies(float2 (&v)[E], const float2* __restrict__ tw, int t) {
         constexpr int R = S::radix(p);
         constexpr int B = E / R;
         constexpr int Ns = S::ns(p);
@@ -266,24 +391,81 @@ struct Team {
         }
 #pragma unroll
         for (int s = 0; s < B; ++s) DFT<R, INV>::run(&v[s * R]);
+    }
+    template <int p>
+    static __device__ __forceinline__ void put(const float2 (&v)[E], float2* sm, int t) {
+        constexpr int R = S::radix(p);
+        constexpr int B = E / R;
+        constexpr int Ns = S::ns(p);
+#pragma unroll
+        for (int s = 0; s < B; ++s) {
+            const int j = t + s * T;
+            const int k = j & (Ns - 1);
+            const int base = (j - k) * R + k, a = at(base);
+#pragma unroll
+            for (int r = 0; r < R; ++r) sm[out_at<p>(base, a, r)] = v[s * R + r];
+        }
+    }
+    template <int p>
+    static __device__ __forceinline__ void get(float2 (&v)[E], const float2* sm, int t) {
+        constexpr int R = S::radix(p);
+        constexpr int B = E / R;
+#pragma unroll
+        for (int s = 0; s < B; ++s) {
+            const int j = t + s * T, a = at_off<T, 1>(t, at(t), s * T);
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[s * R + r] = sm[in_at<p>(j, a, r)];
+        }
+    }
+
+    template <int p>
+    static __device__ __forceinline__ void passes(float2 (&v)[E], float2* sm,
+                                                  const float2* __restrict__ tw, int t, int row) {
+        butterflies<p>(v, tw, t);
         if constexpr (p < P - 1) {
-#pragma unroll
-            for (int s = 0; s < B; ++s) {
-                const int j = t + s * T;
-                const int k = j & (Ns - 1);
-                const int base = (j - k) * R + k;
-#pragma unroll
-                for (int r = 0; r < R; ++r) sm[at(base + r * Ns)] = v[s * R + r];
-            }
+            put<p>(v, sm, t);
             sync(row);
-            constexpr int R2 = S::radix(p + 1);
-            constexpr int B2 = E / R2;
-#pragma unroll
-            for (int s = 0; s < B2; ++s)
-#pragma unroll
-                for (int r = 0; r < R2; ++r) v[s * R2 + r] = sm[at(t + s * T + r * (N / R2))];
+            get<p + 1>(v, sm, t);
             if constexpr (p + 1 < P - 1) sync(row);   // next pass writes the buffer again
             passes<p + 1>(v, sm, tw, t, row);
+        }
+    }
+
+    // The transform by the transposed graph: passes P-1 .. 0, pass p a DFT_R of the elements put<p>
+    // writes, then the twiddles of pass p, stored where get<p> reads.  Its input is laid out as
+    // run() leaves a result and its output as run() takes an input (element t + s*T + r*N/R_0),
+    // so a product of spectra goes from one transform into the next without an exchange, on the
+    // same twiddle table.  `sm` may still be read by the team when called.
+    template <int p = P - 1>
+    static __device__ __forceinline__ void passes_transposed(float2 (&v)[E], float2* sm, const float2* __restrict__ tw,
+                                                             int t, int row) {
+        constexpr int R = S::radix(p);
+        constexpr int B = E / R;
+        constexpr int Ns = S::ns(p);
+#pragma unroll
+        for (int s = 0; s < B; ++s) DFT<R, INV>::run(&v[s * R]);
+        if constexpr (p > 0) {
+            const float2* twp = tw + S::twoff(p);
+            sync(row);
+#pragma unroll
+            for (int s = 0; s < B; ++s) {
+                const int j = t + s * T, k = j & (Ns - 1), a = at_off<T, 1>(t, at(t), s * T);
+                sm[a] = v[s * R];
+#pragma unroll
+                for (int r = 1; r < R; ++r)
+                    sm[in_at<p>(j, a, r)] = cmul<INV>(v[s * R + r], __ldg(twp + (r - 1) * Ns + k));
+            }
+            sync(row);
+            constexpr int R2 = S::radix(p - 1);
+            constexpr int B2 = E / R2;
+            constexpr int Ns2 = S::ns(p - 1);
+#pragma unroll
+            for (int s = 0; s < B2; ++s) {
+                const int j = t + s * T, k = j & (Ns2 - 1), base = (j - k) * R2 + k, a = at(base);
+#pragma unroll
+                for (int r = 0; r < R2; ++r) v[s * R2 + r] = sm[out_at<p - 1>(base, a, r)];
+            }
+            passes_transposed<p - 1>(v, sm, tw, t, row);
         }
     }
 
@@ -291,6 +473,12 @@ struct Team {
     static __device__ __forceinline__ int out_index(int t, int s, int r) {
         constexpr int R = S::radix(P - 1);
         return t + s * T + r * (N / R);
+    }
+
+    // Where run() leaves element t + j*T (T = N/E): the slot of v with s + r*B = j.
+    static __host__ __device__ constexpr int slot(int j) {
+        constexpr int R = S::radix(P - 1), B = E / R;
+        return (j % B) * R + j / B;
     }
 
     template <class Load>
@@ -350,6 +538,25 @@ __device__ __forceinline__ float2 ld_stream(const float2* p) { return __ldcs(p);
 // ld_stream.
 __device__ __forceinline__ float2 ld_once_ca(const float2* p) { return __ldca(p); }
 __device__ __forceinline__ void st_stream(float2* p, float2 v) { __stcs(p, v); }
+
+// Loading ahead into L2: a CTA asks for the lines of the tile that the CTA `ahead` places later
+// in the grid will load, so DRAM keeps working while the resident CTAs compute.  Half the CTAs the
+// GPU holds at once (kSms SMs, `perSm` CTAs each) is the distance that measured best; a whole
+// residency costs 1-5 % of the gain and 1.5 residencies most of it.  Plain launches, 2^25 points,
+// without and with: k_c2c n = 4096: 6178 -> 6300 GB/s, 8192: 5049 -> 5433, 16384: 3755 -> 4322;
+// k_cols NY = 512: 5798 -> 6410, 1024: 4002 -> 4928.  The fewer CTAs share an SM, the more it
+// gives.  kSms sets a distance only.
+constexpr unsigned kSms = 148;
+__host__ __device__ constexpr unsigned prefetch_ahead(int perSm) { return perSm * kSms / 2; }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+// The lines of [p, min(p + bytes, end)) by `threads` threads.
+template <int BYTES, int THREADS>
+__device__ __forceinline__ void prefetch_span(const void* p, const void* end) {
+    const char* q = static_cast<const char*>(p) + threadIdx.x * 128;
+#pragma unroll
+    for (int i = 0; i < BYTES; i += THREADS * 128)
+        if ((int)threadIdx.x * 128 + i < BYTES && q + i < static_cast<const char*>(end)) prefetch_l2(q + i);
+}
 
 }  // namespace dev
 }  // namespace bfly

@@ -11,20 +11,13 @@
 namespace bfly {
 namespace dev {
 
-__device__ __forceinline__ float2 mul_i(float2 a, bool neg) {   // -i*a (neg) or +i*a
-    return neg ? make_float2(a.y, -a.x) : make_float2(-a.y, a.x);
-}
-
 template <bool INV>
 __device__ __forceinline__ void dft3(float2& x0, float2& x1, float2& x2) {
     constexpr float kS3 = 0.866025403784438647f;   // sin(2*pi/3)
-    const float2 t1 = cadd(x1, x2);
-    const float2 t2 = make_float2(x1.x - x2.x, x1.y - x2.y);
-    const float2 m = make_float2(x0.x - 0.5f * t1.x, x0.y - 0.5f * t1.y);
-    const float2 r = mul_i(make_float2(kS3 * t2.x, kS3 * t2.y), !INV);
+    const float2 t1 = cadd(x1, x2), t2 = csub(x1, x2);
+    const float2 m = cfma(t1, -0.5f, x0);
     x0 = cadd(x0, t1);
-    x1 = cadd(m, r);
-    x2 = make_float2(m.x - r.x, m.y - r.y);
+    add_sub_i<INV>(m, t2, kS3, x1, x2);
 }
 
 template <bool INV>
@@ -32,16 +25,14 @@ __device__ __forceinline__ void dft5(float2& x0, float2& x1, float2& x2, float2&
     constexpr float kC1 = 0.309016994374947424f, kC2 = -0.809016994374947424f;   // cos(2pi/5), cos(4pi/5)
     constexpr float kS1 = 0.951056516295153572f, kS2 = 0.587785252292473129f;    // sin(2pi/5), sin(4pi/5)
     const float2 t1 = cadd(x1, x4), t2 = cadd(x2, x3);
-    const float2 t3 = make_float2(x1.x - x4.x, x1.y - x4.y), t4 = make_float2(x2.x - x3.x, x2.y - x3.y);
-    const float2 a1 = make_float2(x0.x + kC1 * t1.x + kC2 * t2.x, x0.y + kC1 * t1.y + kC2 * t2.y);
-    const float2 a2 = make_float2(x0.x + kC2 * t1.x + kC1 * t2.x, x0.y + kC2 * t1.y + kC1 * t2.y);
-    const float2 b1 = mul_i(make_float2(kS1 * t3.x + kS2 * t4.x, kS1 * t3.y + kS2 * t4.y), !INV);
-    const float2 b2 = mul_i(make_float2(kS2 * t3.x - kS1 * t4.x, kS2 * t3.y - kS1 * t4.y), !INV);
+    const float2 t3 = csub(x1, x4), t4 = csub(x2, x3);
+    const float2 a1 = cfma(t2, kC2, cfma(t1, kC1, x0));
+    const float2 a2 = cfma(t2, kC1, cfma(t1, kC2, x0));
+    const float2 b1 = cfma(t4, kS2, cscale(t3, kS1));
+    const float2 b2 = cfma(t4, -kS1, cscale(t3, kS2));
     x0 = cadd(x0, cadd(t1, t2));
-    x1 = cadd(a1, b1);
-    x4 = make_float2(a1.x - b1.x, a1.y - b1.y);
-    x2 = cadd(a2, b2);
-    x3 = make_float2(a2.x - b2.x, a2.y - b2.y);
+    add_sub_i<INV>(a1, b1, x1, x4);
+    add_sub_i<INV>(a2, b2, x2, x3);
 }
 
 template <bool INV>
@@ -52,19 +43,16 @@ __device__ __forceinline__ void dft7(float2* x) {
     const float2 d1 = csub(x[1], x[6]), d2 = csub(x[2], x[5]), d3 = csub(x[3], x[4]);
     const float2 x0 = x[0];
     // cos(2 pi k m / 7) and sin(2 pi k m / 7) for k, m in 1..3 reduce to +-C1..C3, +-S1..S3
-    const float2 a1 = make_float2(x0.x + kC1 * t1.x + kC2 * t2.x + kC3 * t3.x, x0.y + kC1 * t1.y + kC2 * t2.y + kC3 * t3.y);
-    const float2 a2 = make_float2(x0.x + kC2 * t1.x + kC3 * t2.x + kC1 * t3.x, x0.y + kC2 * t1.y + kC3 * t2.y + kC1 * t3.y);
-    const float2 a3 = make_float2(x0.x + kC3 * t1.x + kC1 * t2.x + kC2 * t3.x, x0.y + kC3 * t1.y + kC1 * t2.y + kC2 * t3.y);
-    const float2 b1 = mul_i(make_float2(kS1 * d1.x + kS2 * d2.x + kS3 * d3.x, kS1 * d1.y + kS2 * d2.y + kS3 * d3.y), !INV);
-    const float2 b2 = mul_i(make_float2(kS2 * d1.x - kS3 * d2.x - kS1 * d3.x, kS2 * d1.y - kS3 * d2.y - kS1 * d3.y), !INV);
-    const float2 b3 = mul_i(make_float2(kS3 * d1.x - kS1 * d2.x + kS2 * d3.x, kS3 * d1.y - kS1 * d2.y + kS2 * d3.y), !INV);
+    const float2 a1 = cfma(t3, kC3, cfma(t2, kC2, cfma(t1, kC1, x0)));
+    const float2 a2 = cfma(t3, kC1, cfma(t2, kC3, cfma(t1, kC2, x0)));
+    const float2 a3 = cfma(t3, kC2, cfma(t2, kC1, cfma(t1, kC3, x0)));
+    const float2 b1 = cfma(d3, kS3, cfma(d2, kS2, cscale(d1, kS1)));
+    const float2 b2 = cfma(d3, -kS1, cfma(d2, -kS3, cscale(d1, kS2)));
+    const float2 b3 = cfma(d3, kS2, cfma(d2, -kS1, cscale(d1, kS3)));
     x[0] = cadd(x0, cadd(t1, cadd(t2, t3)));
-    x[1] = cadd(a1, b1);
-    x[6] = csub(a1, b1);
-    x[2] = cadd(a2, b2);
-    x[5] = csub(a2, b2);
-    x[3] = cadd(a3, b3);
-    x[4] = csub(a3, b3);
+    add_sub_i<INV>(a1, b1, x[1], x[6]);
+    add_sub_i<INV>(a2, b2, x[2], x[5]);
+    add_sub_i<INV>(a3, b3, x[3], x[4]);
 }
 
 // Odd prime R = 11, 13 by the same symmetric pairs: (R-1)/2 cosine and sine sums per output pair.
@@ -138,16 +126,14 @@ __device__ __forceinline__ void dft_prime(float2* x) {
     for (int m = 1; m <= H; ++m) sum = cadd(sum, t[m]);
 #pragma unroll
     for (int k = 1; k <= H; ++k) {
-        float2 a = x0, b = make_float2(0.f, 0.f);
+        float2 a = x0, b = cscale(d[1], prime_sin<R>(k));
+        a = cfma(t[1], prime_cos<R>(k), a);
 #pragma unroll
-        for (int m = 1; m <= H; ++m) {
-            const float c = prime_cos<R>((k * m) % R), s = prime_sin<R>((k * m) % R);
-            a = make_float2(fmaf(c, t[m].x, a.x), fmaf(c, t[m].y, a.y));
-            b = make_float2(fmaf(s, d[m].x, b.x), fmaf(s, d[m].y, b.y));
+        for (int m = 2; m <= H; ++m) {
+            a = cfma(t[m], prime_cos<R>((k * m) % R), a);
+            b = cfma(d[m], prime_sin<R>((k * m) % R), b);
         }
-        b = mul_i(b, !INV);
-        x[k] = cadd(a, b);
-        x[R - k] = csub(a, b);
+        add_sub_i<INV>(a, b, x[k], x[R - k]);
     }
     x[0] = sum;
 }
