@@ -53,10 +53,112 @@ k_c2c(const float2* __restrict__ in, float2* __restrict__ out, const float2* __r
     if (ok) TM::for_each_out(v, t, [&](int i, float2 x) { st_stream(dst + i, cscale(x, scale)); });
 }
 
+// ------------------------------------------------------------------ real split, by pairs
+// x real [N] viewed as z[m] = x[2m] + i x[2m+1] (M = N/2), Z = FFT_M(z).  With b = conj(Z[M-k]),
+//   e = (Z[k] + b)/2, o = (Z[k] - b)/(2i), p = W_N^k o:   X[k] = e + p, X[M-k] = conj(e - p)
+// (same split as fft_real.cpp:9-14, :139-149), so bins k and M-k come from one pair of values.
+__device__ __forceinline__ void r2c_pair(float2 a, float2 b, float2 w, float2& xk, float2& xm) {
+    const float2 e = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
+    const float2 o = make_float2(0.5f * (a.y + b.y), 0.5f * (b.x - a.x));
+    const float2 p = cmul<false>(o, w);
+    const float2 d = csub(e, p);
+    xk = cadd(e, p);
+    xm = make_float2(d.x, -d.y);
+}
+// The inverse of r2c_pair times 2 out_scale: Z[k] and Z[M-k] of
+//   Z[k] = (Xk + conj Xm) + i (Xk - conj Xm) W_N^-k   (Xm = X[M-k]; k = 0 pairs X[0] with X[M]).
+// Bins 0 and M: imaginary parts ignored (as in the real part extraction of kfft_c2r_post,
+// fft_real.cpp:262-263), weight s_edge; the others s_int.
+__device__ __forceinline__ void c2r_pair(float2 xk, float2 xm, bool edge, float2 w, float s_edge, float s_int,
+                                         float out_scale, float2& zk, float2& zm) {
+    if (edge) {
+        xk = make_float2(xk.x * s_edge, 0.f);
+        xm = make_float2(xm.x * s_edge, 0.f);
+    } else {
+        xk = cscale(xk, s_int);
+        xm = cscale(xm, s_int);
+    }
+    const float2 ev = make_float2(xk.x + xm.x, xk.y - xm.y);
+    const float2 od = cmul<true>(make_float2(xk.x - xm.x, xk.y + xm.y), w);
+    zk = cscale(make_float2(ev.x - od.y, ev.y + od.x), out_scale);
+    zm = cscale(make_float2(ev.x + od.y, od.x - ev.y), out_scale);
+}
+
+// The split of one row held by a team (TM = Team<M, E, ...>), pairs (k, M-k) with k = t + j T,
+// j < E/2, handled by thread t: it holds the values at k itself, and those at M-k belong to
+// thread T - t, so only the upper half of the row crosses shared memory (E/2 stores and loads a
+// thread in place of E and 2 E), and each pair shares its twiddle and its sums.  Every bin on its
+// own / by pairs, ncu: k_istft n = 512, 60008 frames, 72.7 / 57.4 us; k_stft n = 1024, 20032
+// frames, 53.7 / 48.6 us; k_c2r n = 256, 32768 rows, 18.6 / 16.3 us.
+template <class TM, int M, int E>
+struct RealSplit {
+    static constexpr int T = M / E, H = E / 2;
+    // v: a finished transform, as Team leaves it; emit(k, X[k]) for every bin k <= M of the team's
+    // row.  `sm` must be free once the team has synchronised.
+    template <class Emit>
+    static __device__ __forceinline__ void store(float2 (&v)[E], float2* sm, const float2* __restrict__ twr, int t,
+                                                 int row, Emit&& emit) {
+        float2 lo[H], w[H], mid;
+#pragma unroll
+        for (int j = 0; j < H; ++j) w[j] = __ldg(twr + t + j * T);   // in flight over the exchange
+        TM::sync(row);
+        TM::for_each_out(v, t, [&](int i, float2 x) {
+            if (i >= t + H * T) sm[spad(i - M / 2)] = x;   // i - t is a compile-time multiple of T
+        });
+#pragma unroll
+        for (int j = 0; j < H; ++j) lo[j] = v[TM::slot(j)];
+        mid = v[TM::slot(H)];
+        TM::sync(row);
+        if (t == 0) emit(M / 2, cconj(mid));   // bin M/2 pairs with itself
+#pragma unroll
+        for (int j = 0; j < H; ++j) {
+            const int k = t + j * T;
+            const float2 b = k == 0 ? lo[0] : sm[spad(M / 2 - k)];
+            float2 xk, xm;
+            r2c_pair(lo[j], b, w[j], xk, xm);
+            emit(k, xk);
+            emit(M - k, xm);
+        }
+    }
+
+    // Bins of one row as loaded (all loads in flight before the first use).
+    struct Bins {
+        float2 lo[H], hi[H], mid;
+    };
+    template <class Load>
+    static __device__ __forceinline__ Bins bins(int t, Load&& load) {
+        Bins x;
+#pragma unroll
+        for (int j = 0; j < H; ++j) x.lo[j] = load(t + j * T);
+#pragma unroll
+        for (int j = 0; j < H; ++j) x.hi[j] = load(M - t - j * T);
+        x.mid = t == 0 ? load(M / 2) : make_float2(0.f, 0.f);
+        return x;
+    }
+    // Z of the loaded bins into v, as pass 0 of the team wants it: element t + j T in v[j].  `sm`
+    // must be free when called and is free again on return.
+    static __device__ __forceinline__ void load(float2 (&v)[E], float2* sm, const float2* __restrict__ twr, int t,
+                                                int row, const Bins& x, float s_edge, float s_int, float out_scale) {
+        static_assert(TM::S::radix(0) == E, "pass 0 takes element t + r T in v[r]");
+#pragma unroll
+        for (int j = 0; j < H; ++j) {
+            const int k = t + j * T;
+            float2 zm;
+            c2r_pair(x.lo[j], x.hi[j], k == 0, __ldg(twr + k), s_edge, s_int, out_scale, v[j], zm);
+            if (k > 0) sm[spad(M / 2 - k)] = zm;
+        }
+        if (t == 0) {   // bin M/2 pairs with itself
+            const float c = 2.f * s_int * out_scale;
+            sm[0] = make_float2(c * x.mid.x, -c * x.mid.y);
+        }
+        TM::sync(row);
+#pragma unroll
+        for (int j = H; j < E; ++j) v[j] = sm[spad(t + (j - H) * T)];
+        TM::sync(row);
+    }
+};
+
 // ------------------------------------------------------------------ R2C
-// x real [N] viewed as z[m] = x[2m] + i x[2m+1] (M = N/2), Z = FFT_M(z), then for k = 0..M:
-//   a = Z[k mod M], b = conj(Z[(M-k) mod M]), E = (a+b)/2, O = (a-b)/(2i),
-//   X[k] = E + W_N^k O.          (same split as fft_real.cpp:9-14, :139-149)
 // Optional per-bin weights (WEIGHTED): X[k] *= (k==0||k==M ? s_edge : s_int); used by the
 // adjoint of C2R.
 template <int N, int E, int ROWS, bool WEIGHTED>
@@ -78,53 +180,16 @@ k_r2c(const float2* __restrict__ in, float2* __restrict__ out, const float2* __r
     float2* sm = smem + rl * S;
     float2 v[E];
     TM::run(v, sm, tw, t, rl, [&](int i) { return ok ? ld_stream(src + i) : make_float2(0.f, 0.f); });
-    // twiddles of this thread's output bins k = t + i*T (and bin M for t == 0), in flight
-    // while Z goes through shared memory
-    float2 w[E];
-#pragma unroll
-    for (int i = 0; i < E; ++i) w[i] = __ldg(twr + t + i * T);
-    const float2 wm = __ldg(twr + M);
-    TM::sync(rl);
-    TM::for_each_out(v, t, [&](int i, float2 x) { sm[spad(i)] = x; });
-    TM::sync(rl);
     pdl_trigger();
-    if (!ok) return;
-    auto bin = [&](int k, float2 wk) {
-        const float2 a = sm[spad(k & (M - 1))];
-        const float2 b = sm[spad((M - k) & (M - 1))];
-        const float2 e = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
-        const float2 o = make_float2(0.5f * (a.y + b.y), 0.5f * (b.x - a.x));
-        float2 X = cadd(e, cmul<false>(o, wk));
+    RealSplit<TM, M, E>::store(v, sm, twr, t, rl, [&](int k, float2 X) {
         if constexpr (WEIGHTED) X = cscale(X, (k == 0 || k == M) ? s_edge : s_int);
-        st_stream(dst + k, X);
-    };
-#pragma unroll
-    for (int i = 0; i < E; ++i) bin(t + i * T, w[i]);
-    if (t == 0) bin(M, wm);
+        if (ok) st_stream(dst + k, X);
+    });
 }
 
 // ------------------------------------------------------------------ C2R
-// X half spectrum [M+1] (M = N/2), staged once in shared memory.  Imaginary parts of X[0] and
-// X[M] are ignored, as in the real part extraction of kfft_c2r_post (fft_real.cpp:262-263).
-// For k = 0..M-1:
-//   Xk = X[k], Xm = X[M-k] (scaled by s_edge at DC/Nyquist, s_int elsewhere),
-//   Z[k] = (Xk + conj Xm) + i (Xk - conj Xm) W_N^-k,  z = IDFT_M(Z) * out_scale,
+// X half spectrum [M+1] (M = N/2) to Z by pairs of bins, z = IDFT_M(Z),
 //   x[2m] = Re z[m], x[2m+1] = Im z[m].   out_scale = 1/N gives numpy.fft.irfft.
-// C2R split of bin k: xk = X[k], xm = X[M-k] (xm = X[M] for k = 0), twk = W_N^k.
-__device__ __forceinline__ float2 c2r_split(float2 xk, float2 xm, int k, float2 twk, float s_edge, float s_int,
-                                            float out_scale) {
-    if (k == 0) {
-        xk = make_float2(xk.x * s_edge, 0.f);
-        xm = make_float2(xm.x * s_edge, 0.f);
-    } else {
-        xk = cscale(xk, s_int);
-        xm = cscale(xm, s_int);
-    }
-    const float2 ev = make_float2(xk.x + xm.x, xk.y - xm.y);
-    const float2 od = cmul<true>(make_float2(xk.x - xm.x, xk.y + xm.y), twk);
-    return make_float2((ev.x - od.y) * out_scale, (ev.y + od.x) * out_scale);
-}
-
 template <int N, int E, int ROWS>
 __global__ void __launch_bounds__((N / 2 / E) * ROWS, min_blocks_64regs((N / 2 / E) * ROWS))
 k_c2r(const float2* __restrict__ in, float2* __restrict__ out, const float2* __restrict__ tw,
@@ -142,19 +207,10 @@ k_c2r(const float2* __restrict__ in, float2* __restrict__ out, const float2* __r
     const float2* src = in + row * (M + 1);
     float2* dst = out + row * M;
     float2* sm = smem + rl * S;
-    // stage bins 0..M-1 once (coalesced), then pair bin k with bin M-k from shared memory; the
-    // Nyquist bin M pairs only with bin 0 and is read directly
-    const float2 nyq = (ok && t == 0) ? ld_stream(src + M) : make_float2(0.f, 0.f);   // before the barrier
+    using RS = RealSplit<TM, M, E>;
+    const auto x = RS::bins(t, [&](int k) { return ok ? ld_stream(src + k) : make_float2(0.f, 0.f); });
     float2 v[E];
-#pragma unroll
-    for (int i = 0; i < E; ++i) v[i] = ok ? ld_stream(src + t + i * T) : make_float2(0.f, 0.f);   // all loads in flight
-#pragma unroll
-    for (int i = 0; i < E; ++i) sm[spad(t + i * T)] = v[i];
-    TM::sync(rl);
-    TM::load_first(v, t, [&](int k) {
-        return c2r_split(sm[spad(k)], k == 0 ? nyq : sm[spad(M - k)], k, __ldg(twr + k), s_edge, s_int, out_scale);
-    });
-    TM::sync(rl);   // the passes reuse the staging buffer for their exchanges
+    RS::load(v, sm, twr, t, rl, x, s_edge, s_int, out_scale);
     TM::template passes<0>(v, sm, tw, t, rl);
     pdl_trigger();
     if (ok) TM::for_each_out(v, t, [&](int i, float2 x) { st_stream(dst + i, x); });

@@ -108,26 +108,11 @@ k_stft(const float* __restrict__ sig, float2* __restrict__ out, const float2* __
         }
         return z;
     });
-    float2 w[E];
-#pragma unroll
-    for (int i = 0; i < E; ++i) w[i] = __ldg(twr + t + i * T);
-    const float2 wm = __ldg(twr + M);
-    TM::sync(rl);
-    TM::for_each_out(v, t, [&](int i, float2 z) { sm[spad(i)] = z; });
-    TM::sync(rl);
-    if (!ok) return;
-    auto bin = [&](int k, float2 wk) {
-        const float2 a = sm[spad(k & (M - 1))];
-        const float2 b = sm[spad((M - k) & (M - 1))];
-        const float2 e = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
-        const float2 o = make_float2(0.5f * (a.y + b.y), 0.5f * (b.x - a.x));
-        const float2 X = cadd(e, cmul<false>(o, wk));
-        if constexpr (ADJ) st_stream(dst + k, cscale(X, (k == 0 || k == M) ? s_edge : s_int));
-        else st_stream(dst + k, X);
-    };
-#pragma unroll
-    for (int i = 0; i < E; ++i) bin(t + i * T, w[i]);
-    if (t == 0) bin(M, wm);
+    RealSplit<TM, M, E>::store(v, sm, twr, t, rl, [&](int k, float2 X) {
+        if (!ok) return;
+        if constexpr (ADJ) X = cscale(X, (k == 0 || k == M) ? s_edge : s_int);
+        st_stream(dst + k, X);
+    });
 }
 
 // Inverse STFT in one kernel (torch.istft) for power-of-two N: every frame's C2R in registers
@@ -156,6 +141,7 @@ k_istft(const float2* __restrict__ spec, float* __restrict__ out, const float2* 
     static_assert(2 * S >= N, "a row buffer holds one real frame");
     static_assert(VEC == 1 || VEC == 4, "scalar or float4 overlap-add");
     using TM = Team<M, E, true, sync_kind(T, CTA)>;
+    using RS = RealSplit<TM, M, E>;
     extern __shared__ float2 smem[];
     const int rl = threadIdx.x / T;
     const int t = threadIdx.x - rl * T;
@@ -172,19 +158,10 @@ k_istft(const float2* __restrict__ spec, float* __restrict__ out, const float2* 
         // rows past R (a CTA's partial first or last wave) transform frame f0 again and are not
         // read: every row runs the same barriers, rows of one warp included
         const float2* src = src0 + (uint64_t)(f0 + (rl < R ? rl : 0)) * (M + 1);
-        const float2 nyq = t == 0 ? ld_stream(src + M) : make_float2(0.f, 0.f);
-        float2 v[E];
-#pragma unroll
-        for (int i = 0; i < E; ++i) v[i] = ld_stream(src + t + i * T);
+        const auto x = RS::bins(t, [&](int k) { return ld_stream(src + k); });
         __syncthreads();   // the previous wave is done with the row buffers and the carry
-#pragma unroll
-        for (int i = 0; i < E; ++i) sm[spad(t + i * T)] = v[i];
-        TM::sync(rl);
-        TM::load_first(v, t, [&](int k) {
-            return c2r_split(sm[spad(k)], k == 0 ? nyq : sm[spad(M - k)], k, __ldg(twr + k), ADJ ? s_edge : 1.f,
-                             ADJ ? s_int : 1.f, out_scale);
-        });
-        TM::sync(rl);
+        float2 v[E];
+        RS::load(v, sm, twr, t, rl, x, ADJ ? s_edge : 1.f, ADJ ? s_int : 1.f, out_scale);
         TM::template passes<0>(v, sm, tw, t, rl);
         TM::sync(rl);
         TM::for_each_out(v, t, [&](int i, float2 z) {   // windowed frame: samples 2i, 2i+1 at sm[i]

@@ -260,8 +260,8 @@ __global__ void __launch_bounds__(512, 2) k_mixed(const float2* __restrict__ in,
 // Real transforms of even length N = 2M on the mixed-radix passes of the M-point complex row
 // (M 13-smooth).  twr[k] = W_N^k, k <= M.
 // R2C (numpy.fft.rfft): z[m] = x[2m] + i x[2m+1] read as complex, Z = FFT_M(z) left unpadded in
-// shared memory, then per bin k <= M: a = Z[k mod M], b = conj(Z[(M-k) mod M]),
-// X[k] = (a+b)/2 + W_N^k (a-b)/(2i), times s_edge at bins 0 and M and s_int elsewhere.
+// shared memory, then bins k and M - k by pairs (r2c_pair), times s_edge at bins 0 and M and s_int
+// elsewhere.
 template <class ROWS>
 __global__ void __launch_bounds__(512, 2) k_r2c_mixed(const float2* __restrict__ in, float2* __restrict__ out,
                                                       const float2* __restrict__ tw, const float2* __restrict__ twr,
@@ -279,13 +279,12 @@ __global__ void __launch_bounds__(512, 2) k_r2c_mixed(const float2* __restrict__
     __syncthreads();
     if (!ok) return;
     float2* dst = out + row * (uint64_t)(M + 1);
-    for (int k = t; k <= M; k += T) {
-        const float2 za = Z[k < M ? k : 0];
-        const float2 zb = Z[k > 0 ? M - k : 0];
-        const float2 e = make_float2(0.5f * (za.x + zb.x), 0.5f * (za.y - zb.y));
-        const float2 o = make_float2(0.5f * (za.y + zb.y), 0.5f * (zb.x - za.x));
-        const float2 X = cadd(e, cmul<false>(o, __ldg(twr + k)));
-        st_stream(dst + k, cscale(X, (k == 0 || k == M) ? s_edge : s_int));
+    for (int k = t; k <= M / 2; k += T) {   // bins k and M - k from one pair
+        float2 xk, xm;
+        r2c_pair(Z[k], Z[k > 0 ? M - k : 0], __ldg(twr + k), xk, xm);
+        const float sc = k == 0 ? s_edge : s_int;
+        st_stream(dst + k, cscale(xk, sc));
+        if (2 * k != M) st_stream(dst + M - k, cscale(xm, sc));
     }
 }
 
@@ -293,6 +292,19 @@ __global__ void __launch_bounds__(512, 2) k_r2c_mixed(const float2* __restrict__
 // Z[k] = (Xk + conj Xm) + i (Xk - conj Xm) W_N^-k (Xm = X[M-k], X[M] for k = 0; imaginary parts of
 // bins 0 and M ignored; s_edge / s_int per bin; out_scale) is staged unpadded in shared memory,
 // then z = IFFT_M(Z) goes to HBM as x[2m] = Re z[m], x[2m+1] = Im z[m].
+// Z of one half spectrum staged unpadded in `stage`: bins k and M - k make Z[k] and Z[M-k]
+// (c2r_pair), each bin read once.
+__device__ __forceinline__ void mixed_unsplit(const float2* __restrict__ src, float2* __restrict__ stage,
+                                              const float2* __restrict__ twr, int M, int t, int T, float s_edge,
+                                              float s_int, float out_scale) {
+    for (int k = t; k <= M / 2; k += T) {
+        float2 zk, zm;
+        c2r_pair(ld_stream(src + k), ld_stream(src + M - k), k == 0, __ldg(twr + k), s_edge, s_int, out_scale, zk, zm);
+        stage[k] = zk;
+        if (k > 0 && 2 * k != M) stage[M - k] = zm;
+    }
+}
+
 template <class ROWS>
 __global__ void __launch_bounds__(512, 2) k_c2r_mixed(const float2* __restrict__ in, float2* __restrict__ out,
                                                       const float2* __restrict__ tw, const float2* __restrict__ twr,
@@ -307,10 +319,7 @@ __global__ void __launch_bounds__(512, 2) k_c2r_mixed(const float2* __restrict__
     float2* buf0 = smem + (size_t)(rl < rows ? rl : 0) * 2 * len;
     float2* buf1 = buf0 + len;
     const float2* src = in + row * (uint64_t)(M + 1);
-    if (ok)
-        for (int k = t; k < M; k += T)
-            buf1[k] = c2r_split(ld_stream(src + k), ld_stream(src + (k == 0 ? M : M - k)), k, __ldg(twr + k), s_edge,
-                                s_int, out_scale);
+    if (ok) mixed_unsplit(src, buf1, twr, M, t, T, s_edge, s_int, out_scale);
     __syncthreads();
     ROWS::template run<true, false, true>(a, nullptr, out + row * M, buf0, buf1, tw, ok, t, T, 1.f);
 }
@@ -359,17 +368,16 @@ __global__ void __launch_bounds__(512, 2) k_stft_mixed(const float* __restrict__
     __syncthreads();
     if (!ok) return;
     float2* dst = out + row * (uint64_t)(M + 1);
-    for (int k = t; k <= M; k += T) {
-        const float2 za = Z[k < M ? k : 0];
-        const float2 zb = Z[k > 0 ? M - k : 0];
-        const float2 e = make_float2(0.5f * (za.x + zb.x), 0.5f * (za.y - zb.y));
-        const float2 o = make_float2(0.5f * (za.y + zb.y), 0.5f * (zb.x - za.x));
-        st_stream(dst + k, cadd(e, cmul<false>(o, __ldg(twr + k))));
+    for (int k = t; k <= M / 2; k += T) {
+        float2 xk, xm;
+        r2c_pair(Z[k], Z[k > 0 ? M - k : 0], __ldg(twr + k), xk, xm);
+        st_stream(dst + k, xk);
+        if (2 * k != M) st_stream(dst + M - k, xm);
     }
 }
 
 // Inverse STFT of even non-power-of-two N = 2M (M 13-smooth) in one kernel: per wave each row
-// stages its frame's un-split spectrum (c2r_split, out_scale) in buf1 and runs the M-point
+// stages its frame's un-split spectrum (c2r_pair, out_scale) in buf1 and runs the M-point
 // inverse passes into its natural-order row buffer; the segment split, carry, envelope and
 // overlap-add (window applied there) are IstftSegment (istft_ola.cuh), as in k_istft.
 template <class ROWS, int VEC>
@@ -396,9 +404,7 @@ __global__ void __launch_bounds__(512, 2) k_istft_mixed(const float2* __restrict
         __syncthreads();   // the previous wave is done with the row buffers and the carry
         // rows past R (a CTA's partial first or last wave) transform frame f0 again, unread
         const float2* src = src0 + (uint64_t)(f0 + (rl < R ? rl : 0)) * (M + 1);
-        for (int k = t; k < M; k += T)
-            buf1[k] = c2r_split(ld_stream(src + k), ld_stream(src + (k == 0 ? M : M - k)), k, __ldg(twr + k), 1.f, 1.f,
-                                out_scale);
+        mixed_unsplit(src, buf1, twr, M, t, T, 1.f, 1.f, out_scale);
         __syncthreads();
         ROWS::template run<true, false, false>(a, nullptr, nullptr, buf0, buf1, tw, true, t, T, 1.f);
         __syncthreads();
