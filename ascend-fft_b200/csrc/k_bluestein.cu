@@ -7,8 +7,13 @@
 //   0 < m < n, else 0;  conv = IFFT_M(FFT_M(a) * FFT_M(h)).
 // FFT_M(h) / M (the filter) and c are built per (plan, n) in FP64 on the device and rounded
 // to fp32.  The kernel loads x*c zero-padded, runs the forward M-point Stockham FFT in
-// registers and shared memory, multiplies by the filter, re-enters the inverse FFT through
-// shared memory, multiplies by c and stores the first n outputs.  The inverse transform uses
+// registers and shared memory, multiplies by the filter, runs the inverse FFT by the transposed
+// graph (Team::passes_transposed: it starts from the registers the forward one ends in, one
+// exchange less than re-entering through shared memory), multiplies by c and stores the first n
+// outputs.  n <= M/2, so the first DFT16 has eight zero inputs and the last one eight outputs
+// nobody reads.  What bounds it: shared memory and L1 (83 % of their wavefront rate in ncu:
+// exchanges, twiddles, filter and chirp).  n = 1003, 8192 rows: 90.2 us re-entering through
+// shared memory, 73.7 us so.  The inverse transform uses
 // conj(c) and conj(filter): h is symmetric (h[M-m] = h[m]), so the filter of conj(h) is the
 // conjugate of the filter of h.
 #include <cuda_runtime.h>
@@ -46,25 +51,32 @@ k_bluestein(const float2* __restrict__ in, float2* __restrict__ out, const float
     float2* sm = smem + rl * S;
     const int len = (int)n;
     float2 v[E];
-    TF::run(v, sm, tw, t, rl, [&](int i) {
-        return (ok && i < len) ? cmul<INV>(ld_stream(src + i), __ldg(chirp + i)) : make_float2(0.f, 0.f);
-    });
-    TF::for_each_slot(v, t, [&](int k, float2& x) { x = cmul<INV>(x, __ldg(filt + k)); });
-    TF::sync(rl);   // the last forward pass has read the exchange buffer
-    TF::for_each_out(v, t, [&](int k, float2 x) { sm[spad(k)] = x; });
+    static_assert(TF::S::radix(0) == 16 && E == 16 && TF::P >= 2, "pass 0 is one DFT16 per thread");
+#pragma unroll
+    for (int r = 0; r < E / 2; ++r) {   // n <= M/2: the upper half of the padded row is zero
+        const int i = t + r * T;
+        v[r] = (ok && i < len) ? cmul<INV>(ld_stream(src + i), __ldg(chirp + i)) : make_float2(0.f, 0.f);
+    }
+    dft16_low<false>(v);
+    TF::template put<0>(v, sm, t);
     TF::sync(rl);
+    TF::template get<1>(v, sm, t);
+    if constexpr (TF::P > 2) TF::sync(rl);
+    TF::template passes<1>(v, sm, tw, t, rl);
+    TF::for_each_slot(v, t, [&](int k, float2& x) { x = cmul<INV>(x, __ldg(filt + k)); });
     // Both transforms derive the same shared-memory and twiddle addresses from t; left alone the
     // compiler computes them once and keeps them all live through both halves (over 160
     // registers).  The inverse half takes opaque copies of t and of the buffer, recomputed here.
     const int ti = opaque(t, v[0].x);
     float2* smi = smem + opaque(rl, v[0].x) * S;
-    TI::load_first(v, ti, [&](int i) { return smi[spad(i)]; });
-    TI::sync(rl);   // the inverse passes reuse the buffer
-    TI::template passes<0>(v, smi, tw, ti, rl);
-    if (ok)
-        TI::for_each_out(v, ti, [&](int k, float2 x) {
-            if (k < len) st_stream(dst + k, cscale(cmul<INV>(x, __ldg(chirp + k)), scale));
-        });
+    TI::passes_transposed(v, smi, tw, ti, rl);
+    if (ok) {
+#pragma unroll
+        for (int r = 0; r < E / 2; ++r) {   // only the first n <= M/2 outputs exist
+            const int k = ti + r * T;
+            if (k < len) st_stream(dst + k, cscale(cmul<INV>(v[r], __ldg(chirp + k)), scale));
+        }
+    }
 }
 
 // c[j] = exp(-i*pi*(j^2 mod 2n)/n) for j < n (fp32), and the zero-padded symmetric sequence
