@@ -31,8 +31,15 @@ __host__ __device__ constexpr int min_blocks_64regs(int threads) {
     return 65536 / (threads * 64) > 0 ? 65536 / (threads * 64) : 1;
 }
 
+// Minimum resident CTAs of a kernel with E complex values per thread: 64 registers up to E = 16,
+// 128 for E = 32 (64 of them hold the values).
+template <int E>
+__host__ __device__ constexpr int min_blocks(int threads) {
+    return E <= 16 ? min_blocks_64regs(threads) : 65536 / (threads * 128) > 0 ? 65536 / (threads * 128) : 1;
+}
+
 template <int N, int E, int ROWS, bool INV>
-__global__ void __launch_bounds__((N / E) * ROWS, min_blocks_64regs((N / E) * ROWS))
+__global__ void __launch_bounds__((N / E) * ROWS, min_blocks<E>((N / E) * ROWS))
 k_c2c(const float2* __restrict__ in, float2* __restrict__ out, const float2* __restrict__ tw,
       uint64_t batch, float scale) {
     constexpr int T = N / E;
@@ -47,8 +54,11 @@ k_c2c(const float2* __restrict__ in, float2* __restrict__ out, const float2* __r
     const float2* src = in + row * N;
     float2* dst = out + row * N;
     float2 v[E];
-    TM::run(v, smem + rl * S, tw, t, rl,
-            [&](int i) { return ok ? ld_once_ca(src + i) : make_float2(0.f, 0.f); });
+    TM::load_first(v, t, [&](int i) { return ok ? ld_once_ca(src + i) : make_float2(0.f, 0.f); });
+    constexpr unsigned AHEAD = prefetch_ahead(min_blocks<E>(T * ROWS));
+    if (blockIdx.x + AHEAD < gridDim.x)
+        prefetch_span<ROWS * N * 8, T * ROWS>(in + ((uint64_t)blockIdx.x + AHEAD) * (ROWS * N), in + batch * N);
+    TM::template passes<0>(v, smem + rl * S, tw, t, rl);
     pdl_trigger();
     if (ok) TM::for_each_out(v, t, [&](int i, float2 x) { st_stream(dst + i, cscale(x, scale)); });
 }

@@ -54,8 +54,9 @@ static const Entry kTable[] = {
     E_(4096, 16, 256),
     E_(4096, 16, 512),
     E_(8192, 8, 1024),
-    E_(8192, 16, 512),
-    E_(16384, 16, 1024),
+    // served by the one-pass kernels of k_long_direct.cu; listed for the candidates' limits
+    {8192, 16, 512, 1, nullptr, 1, smem_stride<8192, 16, false>() * 8},
+    {16384, 16, 1024, 1, nullptr, 1, smem_stride<16384, 16, false>() * 8},
 };
 #undef E_
 

@@ -18,7 +18,29 @@ inline bool pdlEnabled() {
     return on;
 }
 
-// `args` must have exactly the kernel's parameter types.
+// `args` must have exactly the kernel's parameter types.  `cluster` CTAs (dividing the grid) form
+// a thread-block cluster.
+template <typename... Args>
+cudaError_t launchPdlCluster(const void* fn, unsigned grid, int block, int smem, unsigned cluster, cudaStream_t stream,
+                             Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdlEnabled() ? 2 : 1;
+    void* argv[] = {static_cast<void*>(&args)...};
+    return cudaLaunchKernelExC(&cfg, fn, argv);
+}
+
 template <typename... Args>
 cudaError_t launchPdl(const void* fn, unsigned grid, int block, int smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};

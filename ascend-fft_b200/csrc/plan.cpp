@@ -365,6 +365,7 @@ struct Plan::Impl {
         void* hi = nullptr;
     };
     std::map<uint32_t, LongTw> twLong;                 // n -> two-level W_n tables
+    std::map<uint32_t, void*> twDirect;                // n -> table of the one-pass long kernels
     void* devIn = nullptr;
     void* devOut = nullptr;
     void* devWork = nullptr;
@@ -408,6 +409,7 @@ Plan::~Plan() {
         if (kv.second.lo) backend::release(kv.second.lo);
         if (kv.second.hi) backend::release(kv.second.hi);
     }
+    for (auto& kv : impl_->twDirect) backend::release(kv.second);
     if (impl_->devIn) backend::release(impl_->devIn);
     if (impl_->devOut) backend::release(impl_->devOut);
     if (impl_->devWork) backend::release(impl_->devWork);
@@ -489,15 +491,21 @@ bool Plan::validShape(uint32_t n, uint32_t batch, int kind) const {
 }
 
 // Kernel variant for (kind, n): the candidate's radix/cta when compiled for n (one CTA per
-// transform, e = radix); otherwise, for long C2C lengths, the four-step kernels (e = 0), or one
-// thread-block cluster per row (e = -1) when the candidate is scheduled "cluster".  Measured on
-// B200 at batch*n = 2^26 the two-kernel four-step is the faster of the two at every long n
-// (the cluster kernel is bound by instruction issue at 16 resident warps per SM), so it is
-// the default.
+// transform, e = radix); otherwise, for long C2C lengths, the one-pass kernels (e = -3), the L2
+// ring (e = -2), one persistent thread-block cluster per row (e = -1) or the four-step kernels
+// (e = 0), by the candidate's schedule.  The one-pass kernels take "stockham" candidates at every
+// long length: at batch*n = 2^26 they run 1.1x (n = 8192) to 1.3x (32768) as fast as what served
+// those before, radix-16 single CTAs up to 16384 and four-step above (k_long_direct.cu).
 int Plan::resolve(int kind, uint32_t n, int* e, int* cta) const {
     const int r = cand_.p.radix, c = cand_.a.ctaThreads;
     if (kind == backend::kC2C) {
         const std::string& sched = cand_.f.schedule;
+        if (sched == "stockham" && (r == 16 || !backend::hasVariant(backend::kC2C, n, r, c)) &&
+            backend::longDirectTableBytes && backend::longDirectTableBytes(n)) {
+            *e = -3;
+            *cta = 256;
+            return 0;
+        }
         if (sched == "stockham" && n <= kMaxSinglePass && backend::hasVariant(backend::kC2C, n, r, c)) {
             *e = r;
             *cta = c;
@@ -580,6 +588,18 @@ int Plan::prepareLong(uint32_t n) {
     return 0;
 }
 
+int Plan::prepareDirect(uint32_t n) {
+    if (impl_->twDirect.count(n)) return 0;
+    void* t = nullptr;
+    if (backend::alloc(&t, backend::longDirectTableBytes(n))) return -1;
+    if (backend::buildLongDirectTable(t, n, stream_) || backend::streamSync(stream_)) {
+        backend::release(t);
+        return -1;
+    }
+    impl_->twDirect[n] = t;
+    return 0;
+}
+
 int Plan::preparePfa(uint32_t n) {
     uint32_t a = 0, b = 0;
     if (!backend::pfaSplit(n, &a, &b) || prepareC2C(b, kColsE)) return -1;
@@ -642,12 +662,13 @@ int Plan::prepare(uint32_t n, uint32_t batch) {
     if (!validShape(n, batch, kPrepare)) return -8;
     int e = 0, cta = 0;
     if (resolve(backend::kC2C, n, &e, &cta)) return -8;
-    const int rcode = e > 0 ? prepareC2C(n, e) : prepareLong(n);
+    const int rcode = e > 0 ? prepareC2C(n, e) : e == -3 ? prepareDirect(n) : prepareLong(n);
     if (rcode) return -1;
     tf_.clear();
     tf_.push_back({Transform::GenTwiddles, "FP64 twiddle tables built on the device, rounded to fp32"});
     tf_.push_back({Transform::LaunchKernel, e > 0 ? "stockham single-pass kernel on the context stream"
                                             : e == -1 ? "one thread-block cluster per row (on-chip transpose)"
+                                            : e == -3 ? "one pass, a CTA or a thread-block cluster per row"
                                             : e == -2 ? "one persistent four-step launch, intermediate in an L2 ring"
                                                       : "four-step column + row kernels on the context stream"});
     return 0;
@@ -693,6 +714,10 @@ int Plan::execC2CWith(const void* dIn, void* dOut, uint32_t n, uint64_t batch, i
         if (prepareC2C(n, e)) return -2;
         if (backend::launchC2C(dIn, dOut, n, batch, inv, scale, impl_->twC2C[{n, e}], e, cta, s)) return -5;
         return 0;
+    }
+    if (e == -3) {
+        if (prepareDirect(n)) return -2;
+        return backend::launchLongDirect(dIn, dOut, n, batch, inv, scale, impl_->twDirect[n], s) ? -5 : 0;
     }
     if (prepareLong(n)) return -2;
     uint32_t n1 = 0, n2 = 0;

@@ -121,6 +121,9 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 // Split cluster barrier: arrive (release: this thread's earlier memory accesses are ordered
 // before the barrier) ... wait (acquire).  Every thread of the cluster alternates them.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+// Arrive without ordering this thread's own memory accesses: for a thread whose earlier loads have
+// all been consumed and which has no earlier stores to publish.
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
 // Address of the same shared-memory location in CTA `rank` of this cluster.

@@ -311,6 +311,7 @@ private:
     int prepareC2C(uint32_t n, int e);
     int prepareReal(uint32_t n);
     int prepareLong(uint32_t n);
+    int prepareDirect(uint32_t n);
     int prepareBluestein(uint32_t n);
     int preparePfa(uint32_t n);
     int prepareMixed(uint32_t n);
