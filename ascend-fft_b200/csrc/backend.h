@@ -240,7 +240,8 @@ int launchIstftAdjoint(const void* gradOut, void* gradSpec, uint32_t n, uint64_t
 
 // Column FFTs: ny-point transforms down the ncols columns of `mats` row-major matrices,
 // element (m, i, col) at m*matStride + i*pitch + col (float2 units).  ny in 32..4096;
-// tw = Stockham table (ny, 16); in == out allowed.
+// tw = Stockham table (ny, colsE(ny)); in == out allowed.
+constexpr int colsE(uint32_t ny) { return ny >= 512 ? 32 : 16; }   // values per thread
 bool hasCols(uint32_t ny);
 int launchCols(const void* in, void* out, uint32_t ny, uint32_t ncols, uint64_t pitch, uint64_t matStride,
                uint64_t mats, bool inverse, float scale, const void* tw, void* stream);

@@ -236,7 +236,7 @@ k_c2r(const float2* __restrict__ in, float2* __restrict__ out, const float2* __r
 // Every load precedes the CTA's first __syncthreads and every store follows its last, so
 // in == out is allowed.
 template <int NY, int E, int C, bool INV>
-__global__ void __launch_bounds__((NY / E) * C, min_blocks_64regs((NY / E) * C))
+__global__ void __launch_bounds__((NY / E) * C, min_blocks<E>((NY / E) * C))
 k_cols(const float2* __restrict__ in, float2* __restrict__ out, const float2* __restrict__ tw,
        uint32_t ncols, uint64_t pitch, uint64_t matStride, uint32_t colBlocks, float scale) {
     constexpr int S = smem_stride<NY, E, true>();
@@ -251,9 +251,16 @@ k_cols(const float2* __restrict__ in, float2* __restrict__ out, const float2* __
     const float2* src = in + m * matStride + (live ? col : 0u);
     float2* dst = out + m * matStride + col;
     float2 v[E];
-    TM::run(v, smem + c * S, tw, t, 0, [&](int i) {
-        return live ? ld_once_ca(src + (size_t)i * pitch) : make_float2(0.f, 0.f);
-    });
+    TM::load_first(v, t, [&](int i) { return live ? ld_once_ca(src + (size_t)i * pitch) : make_float2(0.f, 0.f); });
+    constexpr unsigned AHEAD = prefetch_ahead(min_blocks<E>((NY / E) * C));
+    if (blockIdx.x + AHEAD < gridDim.x) {   // the first line of each row segment of a later strip
+        const uint32_t b = blockIdx.x + AHEAD;
+        const float2* next = in + (uint64_t)(b / colBlocks) * matStride + (b % colBlocks) * C;
+#pragma unroll
+        for (int i = 0; i < NY; i += (NY / E) * C)
+            if (i + (int)threadIdx.x < NY) prefetch_l2(next + (size_t)(i + threadIdx.x) * pitch);
+    }
+    TM::template passes<0>(v, smem + c * S, tw, t, 0);
     if (live) TM::for_each_out(v, t, [&](int k, float2 x) { st_stream(dst + (size_t)k * pitch, cscale(x, scale)); });
 }
 

@@ -810,9 +810,10 @@ int Plan::longStatus(unsigned* status) {
 int Plan::execCols(const void* dIn, void* dOut, uint32_t n, uint64_t mats, uint32_t cols,
                    uint64_t pitch, bool inverse, float scale, void* stream) {
     if (!backend::hasCols(n)) return -8;
-    if (prepareC2C(n, kColsE)) return -2;
+    const int e = backend::colsE(n);
+    if (prepareC2C(n, e)) return -2;
     if (backend::launchCols(dIn, dOut, n, cols, pitch, (uint64_t)n * pitch, mats, inverse, scale,
-                            impl_->twC2C[{n, kColsE}], stream))
+                            impl_->twC2C[{n, e}], stream))
         return -5;
     return 0;
 }
