@@ -19,5 +19,6 @@ def __getattr__(name):
     if name in ("fft", "ifft", "fft2", "ifft2", "rfft", "irfft", "rfft2", "irfft2", "stft", "istft", "c2c", "c2c_axis", "c2c_2d", "r2c", "c2r",
                 "c2c_tensor", "plan_for", "autotune"):
         from . import ops
-        return getattr(ops, name)
+        globals()[name] = getattr(ops, name)   # found without this function from now on
+        return globals()[name]
     raise AttributeError(name)

@@ -107,6 +107,24 @@ class Metric(C.Structure):
 
 
 _lib = None
+_torch_ops = None
+
+
+def load_torch_ops():
+    """The module of csrc_torch/ (transforms on torch tensors, torch imported first), loaded once."""
+    global _torch_ops
+    if _torch_ops is None:
+        import importlib.machinery
+        import importlib.util
+        load()
+        path = LIB_PATH.with_name("_torch_ops.so")
+        if not path.exists():
+            raise ImportError(f"{path} is missing: build it with `python ascend-fft_b200/build.py`")
+        loader = importlib.machinery.ExtensionFileLoader("_torch_ops", str(path))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_torch_ops", loader))
+        loader.exec_module(module)
+        _torch_ops = module
+    return _torch_ops
 
 
 def load() -> C.CDLL:

@@ -23,6 +23,13 @@ hand-written adjoints behind torch.autograd.Function:
     rfft : grad_x = C2R(g) with bins 0 and n/2 weighted 1 and the others 1/2, times s
     irfft: grad_X = R2C(g) with bins 0 and n/2 weighted c and the others 2c  (c = output scale)
 Every call enqueues on torch's current stream; nothing runs on the CPU.
+
+The functions below hand plain calls to csrc_torch/torch_ops.cpp, which launches the same kernels
+and records C++ autograd nodes without the interpreter in between, and run the autograd.Function
+classes here for what it leaves to them (it answers None): functorch, forward-mode, tracing and
+dispatch modes, tensor subclasses, gradients that take several torch operations.  A call of 16 rows
+of 256 points takes 16.1 us through the Function and 5.5 us through the module; rfft of 1024 rows of
+4096 with its gradient 93.3 and 54.3 us, 18 of them on the GPU.
 """
 from __future__ import annotations
 
@@ -31,7 +38,11 @@ import threading
 
 import torch
 
+from . import _lib
 from .core import DEFAULT_CANDIDATE, BflyError, Context
+
+_native = _lib.load_torch_ops()
+_NORM = {None: 0, "": 0, "backward": 0, "ortho": 1, "forward": 2}
 
 _lock = threading.Lock()
 _state = {}   # device index -> {"ctx": Context, "plans": {candidate id: Plan}, "tuned": {...}}
@@ -52,6 +63,9 @@ BEST_REAL = {32: "r8_cta256_shared_fp32_stockham", 64: "r8_cta256_shared_fp32_st
 
 def _device_state(device: torch.device):
     idx = device.index if device.index is not None else torch.cuda.current_device()
+    st = _state.get(idx)   # set once, complete: no lock to read it
+    if st is not None:
+        return st
     with _lock:
         if idx not in _state:
             ctx = Context()
@@ -102,11 +116,28 @@ def autotune(n: int, batch: int, device: torch.device | None = None, top_k: int 
     if plan is None:
         raise BflyError(f"select(n={n}, batch={batch})", -1)
     st["tuned"][("c2c", n)] = plan
+    _native.forget_plans()
     return log
 
 
+def _find_plan(device: int, real: int, n: int):
+    """The module's question: the plan for a length, and its handle."""
+    plan = plan_for(torch.device("cuda", device), n, "real" if real else "c2c")
+    return plan, plan._h.value
+
+
+_native.bind(_find_plan, BflyError)
+
+
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(t.get_device())   # 0.1 us; building a Stream object 2.4
+
+
+def _norm_code(norm: str | None) -> int:
+    code = _NORM.get(norm)
+    if code is None:
+        raise ValueError(f"invalid norm {norm!r}")
+    return code
 
 
 def _scale(norm: str | None, n: int, forward: bool) -> float:
@@ -293,12 +324,18 @@ def c2c_tensor(x: torch.Tensor, direction: int = -1, scale: float = 1.0, split_t
 
 
 def fft(x: torch.Tensor, norm: str | None = None, dim: int = -1) -> torch.Tensor:
+    y = _native.fft(x, dim, -1, _norm_code(norm))
+    if y is not None:
+        return y
     if dim % max(x.dim(), 1) != x.dim() - 1:
         return _FFTAxis.apply(x, dim, -1, _scale(norm, x.shape[dim], True))
     return _FFT.apply(x, -1, _scale(norm, x.shape[-1], True))
 
 
 def ifft(x: torch.Tensor, norm: str | None = None, dim: int = -1) -> torch.Tensor:
+    y = _native.fft(x, dim, 1, _norm_code(norm))
+    if y is not None:
+        return y
     if dim % max(x.dim(), 1) != x.dim() - 1:
         return _FFTAxis.apply(x, dim, 1, _scale(norm, x.shape[dim], False))
     return _FFT.apply(x, 1, _scale(norm, x.shape[-1], False))
@@ -374,9 +411,14 @@ def stft(x: torch.Tensor, n_fft: int, hop_length: int | None = None, win_length:
     window = _pad_window(window, win_length, n_fft, "stft window", x.device)
     if normalized:
         window = (window if window is not None else torch.ones(n_fft, device=x.device)) * n_fft ** -0.5
-    lead = x.shape[:-1]
-    y = _STFT.apply(x.contiguous().reshape(-1, x.shape[-1]), n_fft, hop, center, window)
-    return y.reshape(*lead, y.shape[-2], y.shape[-1]).transpose(-1, -2)
+    flat = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
+    flat = flat.contiguous()
+    y = _native.stft(flat, n_fft, hop, bool(center), window)
+    if y is None:
+        y = _STFT.apply(flat, n_fft, hop, center, window)
+    if x.dim() != 2:
+        y = y.reshape(*x.shape[:-1], y.shape[-2], y.shape[-1])
+    return y.transpose(-1, -2)
 
 
 class _ISTFT(torch.autograd.Function):
@@ -495,10 +537,12 @@ def istft(X: torch.Tensor, n_fft: int, hop_length: int | None = None, win_length
             _envelope_checked.clear()
         _envelope_checked[key] = True
     lead = X.shape[:-2]
-    spec = X.reshape(-1, X.shape[-2], frames).transpose(-1, -2).contiguous()
+    spec = (X if X.dim() == 3 else X.reshape(-1, X.shape[-2], frames)).transpose(-1, -2).contiguous()
     scale = n_fft ** 0.5 if normalized else 1.0
-    y = _ISTFT.apply(spec, n_fft, hop, center, window, out_len, scale)
-    return y.reshape(*lead, out_len)
+    y = _native.istft(spec, n_fft, hop, bool(center), window, out_len, scale)
+    if y is None:
+        y = _ISTFT.apply(spec, n_fft, hop, center, window, out_len, scale)
+    return y if X.dim() == 3 else y.reshape(*lead, out_len)
 
 
 class _RFFT2(torch.autograd.Function):
@@ -558,17 +602,26 @@ def _need_2d(x: torch.Tensor, what: str):
 
 def fft2(x: torch.Tensor, norm: str | None = None) -> torch.Tensor:
     """2-D FFT over the last two dimensions (torch.fft.fft2 with dim=(-2, -1))."""
+    y = _native.fft2(x, -1, _norm_code(norm))
+    if y is not None:
+        return y
     _need_2d(x, "fft2")
     return _FFT2.apply(x, -1, _scale(norm, x.shape[-2] * x.shape[-1], True))
 
 
 def ifft2(x: torch.Tensor, norm: str | None = None) -> torch.Tensor:
+    y = _native.fft2(x, 1, _norm_code(norm))
+    if y is not None:
+        return y
     _need_2d(x, "ifft2")
     return _FFT2.apply(x, 1, _scale(norm, x.shape[-2] * x.shape[-1], False))
 
 
 def rfft2(x: torch.Tensor, norm: str | None = None) -> torch.Tensor:
     """torch.fft.rfft2 over the last two dimensions: float32 [..., ny, nx] -> [..., ny, nx/2+1]."""
+    y = _native.rfft2(x, _norm_code(norm))
+    if y is not None:
+        return y
     _need_2d(x, "rfft2")
     return _RFFT2.apply(x, _scale(norm, x.shape[-2] * x.shape[-1], True))
 
@@ -581,14 +634,19 @@ def irfft2(X: torch.Tensor, s: tuple | None = None, norm: str | None = None) -> 
     nx = s[-1] if s is not None else 2 * (X.shape[-1] - 1)
     if s is not None and s[-2] != ny:
         raise ValueError("irfft2: s[-2] must equal X.shape[-2] (no cropping or padding)")
+    y = _native.irfft2(X, nx, _norm_code(norm))
+    if y is not None:
+        return y
     return _IRFFT2.apply(X, nx, _scale(norm, ny * nx, False))
 
 
 def rfft(x: torch.Tensor, norm: str | None = None) -> torch.Tensor:
-    return _RFFT.apply(x, _scale(norm, x.shape[-1], True))
+    y = _native.rfft(x, _norm_code(norm))
+    return y if y is not None else _RFFT.apply(x, _scale(norm, x.shape[-1], True))
 
 
 def irfft(X: torch.Tensor, n: int | None = None, norm: str | None = None) -> torch.Tensor:
     if n is None:
         n = 2 * (X.shape[-1] - 1)
-    return _IRFFT.apply(X, n, _scale(norm, n, False))
+    y = _native.irfft(X, n, _norm_code(norm))
+    return y if y is not None else _IRFFT.apply(X, n, _scale(norm, n, False))

@@ -2,7 +2,8 @@
 
 CUDA translation units are compiled by nvcc with `-gencode arch=compute_100a,code=sm_100a`,
 host units by g++, and everything is linked into bfly/_lib/libbfly_b200.so next to the Python
-package (the CUDA runtime is linked statically).  Objects go to _build/; a unit is rebuilt only
+package (the CUDA runtime is linked statically); csrc_torch/ becomes the Python module
+bfly/_lib/_torch_ops.so on top of it.  Objects go to _build/; a unit is rebuilt only
 when it or a header is newer than its object.
 
     python ascend-fft_b200/build.py [--force] [--jobs N]
@@ -23,6 +24,8 @@ CSRC = PKG / "csrc"
 BUILD = PKG / "_build"
 LIBDIR = PKG / "bfly" / "_lib"
 LIB = LIBDIR / "libbfly_b200.so"
+TORCH_SRC = PKG / "csrc_torch" / "torch_ops.cpp"
+TORCH_LIB = LIBDIR / "_torch_ops.so"   # the Python module bfly/ops.py calls
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 INCLUDES = ["-I", str(ROOT / "include"), "-I", str(CSRC)]
@@ -60,6 +63,22 @@ def compile_one(cmd):
     return r.stderr
 
 
+def torch_cmd(obj: Path):
+    """Compile and link commands of the torch module (C++ against the installed torch)."""
+    import sysconfig
+
+    from torch.utils import cpp_extension
+    includes = [*INCLUDES, "-I", sysconfig.get_paths()["include"], "-I", str(Path(nvcc()).parents[1] / "include")]
+    for d in cpp_extension.include_paths():
+        includes += ["-isystem", d]
+    dirs = cpp_extension.library_paths()
+    return (["g++", "-std=c++17", "-O2", "-fPIC", "-Wall", "-Wextra", f"-DTORCH_EXTENSION_NAME={TORCH_LIB.stem}",
+             *includes, "-c", str(TORCH_SRC), "-o", str(obj)],
+            ["g++", "-shared", "-o", str(TORCH_LIB.with_suffix(".so.tmp")), str(obj), *[f"-L{d}" for d in dirs],
+             f"-L{LIBDIR}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", f"-l:{LIB.name}",
+             "-Wl,-rpath,$ORIGIN"])
+
+
 def build(force: bool = False, jobs: int | None = None, verbose: bool = False) -> Path:
     BUILD.mkdir(parents=True, exist_ok=True)
     LIBDIR.mkdir(parents=True, exist_ok=True)
@@ -78,6 +97,10 @@ def build(force: bool = False, jobs: int | None = None, verbose: bool = False) -
         if force or stale(src, obj, deps):
             cmds.append(["g++", "-std=c++17", "-O2", "-fPIC", "-Wall", "-Wextra", *INCLUDES,
                          "-c", str(src), "-o", str(obj)])
+    torch_obj = BUILD / (TORCH_SRC.stem + ".torch.o")
+    torch_compile, torch_link = torch_cmd(torch_obj)
+    if force or stale(TORCH_SRC, torch_obj, [ROOT / "include" / "bfly_b200.h"]):
+        cmds.append(torch_compile)
     if cmds:
         with cf.ThreadPoolExecutor(max_workers=jobs or min(len(cmds), os.cpu_count() or 4)) as ex:
             for out in ex.map(compile_one, cmds):
@@ -88,6 +111,9 @@ def build(force: bool = False, jobs: int | None = None, verbose: bool = False) -
         compile_one([nvcc(), "-shared", *ARCH, "-cudart", "static", "-o", str(tmp),
                      *[str(o) for o in objs], "-lpthread", "-ldl", "-lrt"])
         os.replace(tmp, LIB)
+    if not TORCH_LIB.exists() or torch_obj.stat().st_mtime > TORCH_LIB.stat().st_mtime:
+        compile_one(torch_link)
+        os.replace(torch_link[3], TORCH_LIB)
     return LIB
 
 
