@@ -14,6 +14,7 @@
 // constant offsets and strides fold into the loads and stores (37 % fewer instructions at
 // n = 1000).
 // This unit: the twiddle kernel and the launchers; the kernels are in mixed.cuh.
+#include "launch.cuh"
 #include "mixed.cuh"
 
 namespace bfly {
@@ -72,25 +73,22 @@ struct MixedShape {
     int cls = 0;   // radix class of the kernel instance (mixed_pass_r)
 };
 constexpr int kMixedMaxSmem = 227 * 1024;
-static_assert(2 * (dev::spad((int)kMixedMaxN - 1) + 1) * 8 <= kMixedMaxSmem, "two rows of the longest length fit in shared memory");
+static_assert(2 * (int)kMixedMaxN * 8 <= kMixedMaxSmem, "two rows of the longest length fit in shared memory");
 
 MixedShape mixedShape(const MixedRadix& plan) {
     MixedShape m;
     m.args = mixedArgs(plan);
-    // one butterfly of the largest radix per thread and pass (more of the smaller radices);
-    // measured on B200 over n = 12..12000: ceil(n / R_max) threads per row with ~200-300
-    // threads per CTA beat n/8 threads per row, larger CTAs, and an 80-register budget
-    int rmax = 2;
-    for (int p = 0; p < plan.passes; ++p) {
-        rmax = std::max(rmax, plan.radix[p]);
+    // about one butterfly of the largest radix per thread and pass (more of the smaller radices);
+    // measured on B200 over n = 12..12000: n / R_max threads per row with ~200-300 threads per CTA
+    // beat n/8 threads per row, larger CTAs, and an 80-register budget
+    for (int p = 0; p < plan.passes; ++p)
         m.cls = std::max(m.cls, plan.radix[p] == 11 || plan.radix[p] == 13 ? 2 : plan.radix[p] > 10 ? 1 : 0);
-    }
-    m.T = std::min(512, (plan.n + rmax - 1) / rmax);
-    m.rows = std::max(1, 224 / m.T);
+    m.T = dev::mixedThreads(plan.n, plan.radix, plan.passes);
+    m.rows = dev::mixedRows(m.T);
     // pass 0 stores at stride R_0: pad its buffer every R_0 slots when R_0 is even (odd strides
     // are conflict-free already), unless that no longer fits (then it stays unpadded)
     const int r0 = plan.radix[0];
-    m.len = dev::spad(plan.n - 1) + 1;
+    m.len = plan.n;
     m.args.pad0 = (r0 % 2 == 0 && plan.passes > 1) ? r0 : 0;
     if (m.args.pad0) {
         const int len0 = std::max(m.len, plan.n + (plan.n - 1) / m.args.pad0 + 1);
@@ -100,6 +98,8 @@ MixedShape mixedShape(const MixedRadix& plan) {
     m.args.magic0 =
         m.args.pad0 ? (unsigned)((0x100000000ull + m.args.pad0 - 1) / (unsigned long long)m.args.pad0) : 0u;
     m.smem = m.rows * 2 * m.len * 8;
+    const int warps = (m.rows * m.T + 31) / 32;   // 64 registers a thread: 32 warps per SM
+    m.args.ahead = dev::prefetch_ahead(std::max(1, std::min(32 / warps, kMixedMaxSmem / m.smem)));
     return m;
 }
 
@@ -129,10 +129,10 @@ int launchMixed(const void* in, void* out, const MixedRadix& plan, uint64_t batc
     if (int e = optInSharedMemory((const void*)fn, kMixedMaxSmem)) return e;
     const uint64_t groups = (batch + m.rows - 1) / m.rows;
     if (groups > 0x7fffffffull) return (int)cudaErrorInvalidValue;
-    fn<<<(unsigned)groups, m.T * m.rows, m.smem, reinterpret_cast<cudaStream_t>(stream)>>>(
+    return (int)launchPdlKernel(
+        fn, groups, m.T * m.rows, m.smem, stream,
         static_cast<const float2*>(in), static_cast<float2*>(out), static_cast<const float2*>(tw), m.args, batch, m.T,
         m.rows, m.len, scale);
-    return (int)cudaGetLastError();
 }
 
 int launchR2CMixed(const void* in, void* out, const MixedRadix& half, uint64_t batch, const void* tw, const void* twr,
@@ -144,10 +144,10 @@ int launchR2CMixed(const void* in, void* out, const MixedRadix& half, uint64_t b
     if (int e = optInSharedMemory((const void*)fn, kMixedMaxSmem)) return e;
     const uint64_t groups = (batch + m.rows - 1) / m.rows;
     if (groups > 0x7fffffffull) return (int)cudaErrorInvalidValue;
-    fn<<<(unsigned)groups, m.T * m.rows, m.smem, reinterpret_cast<cudaStream_t>(stream)>>>(
+    return (int)launchPdlKernel(
+        fn, groups, m.T * m.rows, m.smem, stream,
         static_cast<const float2*>(in), static_cast<float2*>(out), static_cast<const float2*>(tw),
         static_cast<const float2*>(twr), m.args, batch, m.T, m.rows, m.len, sEdge, sInt);
-    return (int)cudaGetLastError();
 }
 
 int launchC2RMixed(const void* in, void* out, const MixedRadix& half, uint64_t batch, const void* tw, const void* twr,
@@ -159,10 +159,10 @@ int launchC2RMixed(const void* in, void* out, const MixedRadix& half, uint64_t b
     if (int e = optInSharedMemory((const void*)fn, kMixedMaxSmem)) return e;
     const uint64_t groups = (batch + m.rows - 1) / m.rows;
     if (groups > 0x7fffffffull) return (int)cudaErrorInvalidValue;
-    fn<<<(unsigned)groups, m.T * m.rows, m.smem, reinterpret_cast<cudaStream_t>(stream)>>>(
+    return (int)launchPdlKernel(
+        fn, groups, m.T * m.rows, m.smem, stream,
         static_cast<const float2*>(in), static_cast<float2*>(out), static_cast<const float2*>(tw),
         static_cast<const float2*>(twr), m.args, batch, m.T, m.rows, m.len, sEdge, sInt, outScale);
-    return (int)cudaGetLastError();
 }
 
 int launchStftMixed(const void* sig, void* out, const MixedRadix& half, uint64_t signals, uint32_t framesPerSignal,
@@ -176,11 +176,11 @@ int launchStftMixed(const void* sig, void* out, const MixedRadix& half, uint64_t
     const uint64_t frames = signals * framesPerSignal;
     const uint64_t groups = (frames + m.rows - 1) / m.rows;
     if (groups > 0x7fffffffull) return (int)cudaErrorInvalidValue;
-    fn<<<(unsigned)groups, m.T * m.rows, m.smem, reinterpret_cast<cudaStream_t>(stream)>>>(
+    return (int)launchPdlKernel(
+        fn, groups, m.T * m.rows, m.smem, stream,
         static_cast<const float*>(sig), static_cast<float2*>(out), static_cast<const float2*>(tw),
         static_cast<const float2*>(twr), static_cast<const float*>(window), m.args, frames, framesPerSignal,
         (int64_t)sigLen, sigStride, hop, center ? 1 : 0, m.T, m.rows, m.len);
-    return (int)cudaGetLastError();
 }
 
 int launchIstftMixed(const void* spec, void* out, const MixedRadix& half, uint64_t signals, uint32_t frames,
@@ -212,11 +212,11 @@ int launchIstftMixed(const void* spec, void* out, const MixedRadix& half, uint64
     istftSegments((uint32_t)N, m.rows, frames, hop, signals, (uint64_t)sms * perSm, &q, &segs);
     const uint64_t grid = signals * segs;
     if (grid > 0x7fffffffull) return (int)cudaErrorInvalidValue;
-    fn<<<(unsigned)grid, m.T * m.rows, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
+    return (int)launchPdlKernel(
+        fn, grid, m.T * m.rows, smem, stream,
         static_cast<const float2*>(spec), static_cast<float*>(out), static_cast<const float2*>(tw),
         static_cast<const float2*>(twr), static_cast<const float*>(window), m.args, frames, hop, q, segs, start,
         outLen, scale / N, m.T, m.rows, m.len);
-    return (int)cudaGetLastError();
 }
 
 }  // namespace backend

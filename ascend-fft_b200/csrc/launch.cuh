@@ -4,6 +4,7 @@
 // BFLY_PDL=0 in the environment launches them plainly instead (read once per process).
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 #include <cstdlib>
 
@@ -55,6 +56,17 @@ cudaError_t launchPdl(const void* fn, unsigned grid, int block, int smem, cudaSt
     cfg.numAttrs = pdlEnabled() ? 1 : 0;
     void* argv[] = {static_cast<void*>(&args)...};
     return cudaLaunchKernelExC(&cfg, fn, argv);
+}
+
+// The same for a typed kernel: the arguments convert to its parameters.
+template <typename T>
+struct SameType {
+    using type = T;
+};
+template <typename... P>
+cudaError_t launchPdlKernel(void (*fn)(P...), uint64_t grid, int block, int smem, void* stream,
+                            typename SameType<P>::type... args) {
+    return launchPdl((const void*)fn, (unsigned)grid, block, smem, reinterpret_cast<cudaStream_t>(stream), args...);
 }
 
 }  // namespace backend

@@ -10,8 +10,8 @@
 // R-point DFT in registers (radix 2..16, odd and Good-Thomas composite radices included) and
 // outputs at (j - k) R + k + r Ns.  A row of n values lives in two shared buffers (ping-pong);
 // the first pass reads HBM directly (coalesced over j), the last writes HBM directly (Ns = n/R
-// there, so the store index is j + r n/R, coalesced too).  T = min(512, ceil(n / R_max)) threads
-// per row, each taking butterflies j = t, t + T, ...; max(1, 224 / T) rows per CTA.  k = j mod Ns
+// there, so the store index is j + r n/R, coalesced too).  T threads per row (mixedThreads), each
+// taking butterflies j = t, t + T, ...; max(1, 224 / T) rows per CTA.  k = j mod Ns
 // uses a multiply-high by ceil(2^32 / Ns) (exact for j, Ns < 2^14).  The pass list is a kernel
 // argument, so one kernel (per radix class) serves every such length; the plans of common
 // lengths also have kernels with the pass list fixed at compile time (FixedRows), whose
@@ -39,11 +39,53 @@ struct MixedArgs {
     int twoff[backend::kMixedMaxPasses];
     unsigned magic[backend::kMixedMaxPasses];   // ceil(2^32 / ns), pass p >= 1
     // the buffer pass 0 writes: element i at i + i / pad0, pad0 = R_0 when R_0 is even (its
-    // stride-R_0 stores then hit distinct banks), else 0 (element i at i); the other buffers
-    // hold element i at spad(i)
+    // stride-R_0 stores then hit distinct banks), else 0 (element i at i).  The other buffers are
+    // unpadded: later passes load and store runs of consecutive elements (only pass 1's runs, of
+    // R_0 < 16, meet a second one in a half-warp), and a pad would cost two instructions an access
     int pad0;
     unsigned magic0;   // ceil(2^32 / pad0), 0 when pad0 = 0
+    unsigned ahead;    // CTAs between a CTA and the one whose input it asks for (prefetch_l2)
 };
+
+// Threads per row: T butterflies at a time, so a pass of n/R takes ceil(n / (R T)) rounds of which
+// the last may be nearly empty (n = 1200 = 16 15 5 on 75 threads: five of the 80 radix-15
+// butterflies in a round of their own).  Of the divisions of every pass's butterflies into equal
+// rounds between n / R_max (one largest butterfly a thread) and twice that, at most 512, the one
+// with the least T * sum(rounds * R), whole warps of a CTA counted.
+constexpr int mixedRows(int T) { return 224 / T > 1 ? 224 / T : 1; }
+constexpr int mixedThreads(int n, const int* radix, int passes) {
+    int rmax = 2;
+    for (int p = 0; p < passes; ++p) rmax = radix[p] > rmax ? radix[p] : rmax;
+    const int least = (n + rmax - 1) / rmax;
+    const int lo = least < 512 ? least : 257, hi = 2 * least < 512 ? 2 * least : 512;
+    int best = least < 512 ? least : 512;
+    long long bestCost = -1;
+    for (int p = -1; p < passes; ++p)
+        for (int rounds = 1; rounds <= 48; ++rounds) {
+            const int nb = p < 0 ? 0 : n / radix[p];
+            const int T = p < 0 ? best : (nb + rounds - 1) / rounds;
+            if (p < 0 ? rounds > 1 : (T < lo || T > hi)) continue;
+            long long slots = 0;
+            for (int q = 0; q < passes; ++q) slots += (long long)((n / radix[q] + T - 1) / T) * radix[q];
+            const int cta = mixedRows(T) * T;
+            const long long cost = slots * T * ((cta + 31) / 32 * 32) / cta;
+            if (bestCost < 0 || cost < bestCost || (cost == bestCost && T < best)) {
+                bestCost = cost;
+                best = T;
+            }
+        }
+    return best;
+}
+
+// A CTA's share of a later CTA's input: `rows` rows of `bytes` bytes, the array ending at `end`.
+__device__ __forceinline__ void mixed_load_ahead(const void* in, const MixedArgs& a, int rows, size_t bytes,
+                                                 uint64_t batch) {
+    if (blockIdx.x + a.ahead >= gridDim.x) return;
+    const char* base = static_cast<const char*>(in);
+    const char* p = base + ((uint64_t)blockIdx.x + a.ahead) * rows * bytes;
+    const char* last = p + rows * bytes < base + batch * bytes ? p + rows * bytes : base + batch * bytes;
+    for (p += threadIdx.x * 128; p < last; p += blockDim.x * 128) prefetch_l2(p);
+}
 
 // KIND bit 0: source is the row in HBM (pass 0, which writes the pass-0 buffer); bit 1:
 // destination is the row in HBM (scaled); bit 2: source is the pass-0 buffer (pass 1); bit 3:
@@ -69,7 +111,7 @@ __device__ __forceinline__ void mixed_pass(const float2* __restrict__ src, float
             v[r] = (KIND & 1)   ? ld_stream(src + j + r * nb)
                    : (KIND & 8) ? src[j + r * nb]
                    : (KIND & 4) ? src[js + r * nbs]
-                                : src[spad(j + r * nb)];
+                                : src[j + r * nb];
         if (!PASS0) {
 #pragma unroll
             for (int r = 1; r < R; ++r) v[r] = cmul<INV>(v[r], __ldg(twp + (r - 1) * Ns + k));
@@ -81,7 +123,7 @@ __device__ __forceinline__ void mixed_pass(const float2* __restrict__ src, float
             if (KIND & 2) st_stream(dst + base + r * Ns, cscale(v[r], scale));
             else if (KIND & 16) dst[base + r * Ns] = v[r];
             else if (PASS0) dst[j * stride0 + r] = v[r];
-            else dst[spad(base + r * Ns)] = v[r];
+            else dst[base + r * Ns] = v[r];
         }
     }
 }
@@ -155,9 +197,9 @@ __device__ __forceinline__ float2* mixed_row(const MixedArgs& a, const float2* s
 
 // The same passes for a plan fixed at compile time (its radices R0, R1, ...): n, Ns, the
 // butterfly counts, threads per row and the pass-0 pad are constants, so the element offsets
-// of every load and store fold into the instructions and the radix needs no dispatch.  T =
-// min(512, ceil(n / R_max)) threads per row and pad0 = R_0 (even R_0) or 0, as mixedShape
-// sets them; twiddles at the plan's offsets.
+// of every load and store fold into the instructions and the radix needs no dispatch.
+// mixedThreads threads per row and pad0 = R_0 (even R_0) or 0, as mixedShape sets them; twiddles at
+// the plan's offsets.
 template <int R, bool INV, int KIND, int N, int NS, int T, int PAD0>
 __device__ __forceinline__ void fixed_pass(const float2* __restrict__ src, float2* __restrict__ dst,
                                            const float2* __restrict__ twp, int t, float scale) {
@@ -177,7 +219,7 @@ __device__ __forceinline__ void fixed_pass(const float2* __restrict__ src, float
             v[r] = (KIND & 1)   ? ld_stream(src + j + r * nb)
                    : (KIND & 8) ? src[j + r * nb]
                    : (KIND & 4) ? src[js + r * nbs]
-                                : src[spad(j + r * nb)];
+                                : src[j + r * nb];
         if (!PASS0) {
 #pragma unroll
             for (int r = 1; r < R; ++r) v[r] = cmul<INV>(v[r], __ldg(twp + (r - 1) * NS + k));
@@ -189,7 +231,7 @@ __device__ __forceinline__ void fixed_pass(const float2* __restrict__ src, float
             if (KIND & 2) st_stream(dst + base + r * NS, cscale(v[r], scale));
             else if (KIND & 16) dst[base + r * NS] = v[r];
             else if (PASS0) dst[j * stride0 + r] = v[r];
-            else dst[spad(base + r * NS)] = v[r];
+            else dst[base + r * NS] = v[r];
         }
     }
 }
@@ -197,8 +239,8 @@ __device__ __forceinline__ void fixed_pass(const float2* __restrict__ src, float
 template <int... Rs>
 struct FixedPlan {
     static constexpr int N = (Rs * ...);
-    static constexpr int RMAX = std::max({Rs...});
-    static constexpr int T = (N + RMAX - 1) / RMAX < 512 ? (N + RMAX - 1) / RMAX : 512;
+    static constexpr int radix[] = {Rs...};
+    static constexpr int T = mixedThreads(N, radix, sizeof...(Rs));
     static constexpr int R0 = std::get<0>(std::make_tuple(Rs...));
     static constexpr int PAD0 = (R0 % 2 == 0 && sizeof...(Rs) > 1) ? R0 : 0;
 };
@@ -249,11 +291,13 @@ __global__ void __launch_bounds__(512, 2) k_mixed(const float2* __restrict__ in,
                                                   const float2* __restrict__ tw, MixedArgs a, uint64_t batch, int T,
                                                   int rows, int len, float scale) {
     extern __shared__ float2 smem[];
+    pdl_wait();
     const int rl = threadIdx.x / T;
     const int t = threadIdx.x - rl * T;
     const uint64_t row = (uint64_t)blockIdx.x * rows + rl;
     const bool ok = rl < rows && row < batch;
     float2* buf0 = smem + (size_t)(rl < rows ? rl : 0) * 2 * len;
+    mixed_load_ahead(in, a, rows, (size_t)a.n * 8, batch);
     ROWS::template run<INV, true, true>(a, in + row * a.n, out + row * a.n, buf0, buf0 + len, tw, ok, t, T, scale);
 }
 
@@ -268,15 +312,18 @@ __global__ void __launch_bounds__(512, 2) k_r2c_mixed(const float2* __restrict__
                                                       MixedArgs a, uint64_t batch, int T, int rows, int len,
                                                       float s_edge, float s_int) {
     extern __shared__ float2 smem[];
+    pdl_wait();
     const int rl = threadIdx.x / T;
     const int t = threadIdx.x - rl * T;
     const uint64_t row = (uint64_t)blockIdx.x * rows + rl;
     const bool ok = rl < rows && row < batch;
     const int M = a.n;
     float2* buf0 = smem + (size_t)(rl < rows ? rl : 0) * 2 * len;
+    mixed_load_ahead(in, a, rows, (size_t)M * 8, batch);
     const float2* Z = ROWS::template run<false, true, false>(a, in + row * M, nullptr, buf0, buf0 + len, tw, ok, t, T,
                                                            1.f);
     __syncthreads();
+    pdl_trigger();
     if (!ok) return;
     float2* dst = out + row * (uint64_t)(M + 1);
     for (int k = t; k <= M / 2; k += T) {   // bins k and M - k from one pair
@@ -311,6 +358,7 @@ __global__ void __launch_bounds__(512, 2) k_c2r_mixed(const float2* __restrict__
                                                       MixedArgs a, uint64_t batch, int T, int rows, int len,
                                                       float s_edge, float s_int, float out_scale) {
     extern __shared__ float2 smem[];
+    pdl_wait();
     const int rl = threadIdx.x / T;
     const int t = threadIdx.x - rl * T;
     const uint64_t row = (uint64_t)blockIdx.x * rows + rl;
@@ -319,6 +367,7 @@ __global__ void __launch_bounds__(512, 2) k_c2r_mixed(const float2* __restrict__
     float2* buf0 = smem + (size_t)(rl < rows ? rl : 0) * 2 * len;
     float2* buf1 = buf0 + len;
     const float2* src = in + row * (uint64_t)(M + 1);
+    mixed_load_ahead(in, a, rows, (size_t)(M + 1) * 8, batch);
     if (ok) mixed_unsplit(src, buf1, twr, M, t, T, s_edge, s_int, out_scale);
     __syncthreads();
     ROWS::template run<true, false, true>(a, nullptr, out + row * M, buf0, buf1, tw, ok, t, T, 1.f);
@@ -333,6 +382,7 @@ __global__ void __launch_bounds__(512, 2) k_stft_mixed(const float* __restrict__
                                                        uint32_t framesPerSignal, int64_t sigLen, uint64_t sigStride,
                                                        uint32_t hop, int center, int T, int rows, int len) {
     extern __shared__ float2 smem[];
+    pdl_wait();
     const int rl = threadIdx.x / T;
     const int t = threadIdx.x - rl * T;
     const uint64_t row = (uint64_t)blockIdx.x * rows + rl;
@@ -366,6 +416,7 @@ __global__ void __launch_bounds__(512, 2) k_stft_mixed(const float* __restrict__
     __syncthreads();
     const float2* Z = ROWS::template run<false, false, false>(a, nullptr, nullptr, buf0, buf1, tw, ok, t, T, 1.f);
     __syncthreads();
+    pdl_trigger();
     if (!ok) return;
     float2* dst = out + row * (uint64_t)(M + 1);
     for (int k = t; k <= M / 2; k += T) {
@@ -387,6 +438,7 @@ __global__ void __launch_bounds__(512, 2) k_istft_mixed(const float2* __restrict
                                                         uint32_t hop, uint32_t Q, uint32_t segs, int64_t start,
                                                         uint64_t outLen, float out_scale, int T, int rows, int len) {
     extern __shared__ float2 smem[];
+    pdl_wait();
     const int rl = threadIdx.x / T;
     const int t = threadIdx.x - rl * T;
     const int M = a.n;
@@ -416,6 +468,7 @@ __global__ void __launch_bounds__(512, 2) k_istft_mixed(const float2* __restrict
                 return make_float4(w.x * x.x, w.y * x.y, w.z * x.z, w.w * x.w);
             });
     }
+    pdl_trigger();
     seg.zeroTail(segs);
 }
 
