@@ -246,10 +246,9 @@ int launchCols(const void* in, void* out, uint32_t ny, uint32_t ncols, uint64_t 
     if (grid > 0x7fffffffull) return (int)cudaErrorInvalidValue;
     if (int err = prepareEntry(x)) return err;
     auto fn = reinterpret_cast<dev::KCols>(const_cast<void*>(x->fn));
-    fn<<<(unsigned)grid, x->cta, x->smem, S(stream)>>>(static_cast<const float2*>(in), static_cast<float2*>(out),
-                                                      static_cast<const float2*>(tw), ncols, pitch, matStride,
-                                                      colBlocks, scale);
-    return rc(cudaGetLastError());
+    return rc(launchPdlKernel(fn, grid, x->cta, x->smem, stream, static_cast<const float2*>(in),
+                              static_cast<float2*>(out), static_cast<const float2*>(tw), ncols, pitch, matStride,
+                              colBlocks, scale));
 }
 
 int launchLongB(const void* in, void* out, uint32_t n1, uint32_t n2, uint64_t batch,

@@ -123,7 +123,7 @@ struct RealSplit {
 #pragma unroll
         for (int j = 0; j < H; ++j) {
             const int k = t + j * T;
-            const float2 b = k == 0 ? lo[0] : sm[spad(M / 2 - k)];
+            const float2 b = j == 0 && t == 0 ? lo[0] : sm[spad(M / 2 - k)];
             float2 xk, xm;
             r2c_pair(lo[j], b, w[j], xk, xm);
             emit(k, xk);
@@ -154,8 +154,8 @@ struct RealSplit {
         for (int j = 0; j < H; ++j) {
             const int k = t + j * T;
             float2 zm;
-            c2r_pair(x.lo[j], x.hi[j], k == 0, __ldg(twr + k), s_edge, s_int, out_scale, v[j], zm);
-            if (k > 0) sm[spad(M / 2 - k)] = zm;
+            c2r_pair(x.lo[j], x.hi[j], j == 0 && t == 0, __ldg(twr + k), s_edge, s_int, out_scale, v[j], zm);
+            if (j > 0 || t > 0) sm[spad(M / 2 - k)] = zm;
         }
         if (t == 0) {   // bin M/2 pairs with itself
             const float c = 2.f * s_int * out_scale;
@@ -189,7 +189,11 @@ k_r2c(const float2* __restrict__ in, float2* __restrict__ out, const float2* __r
     float2* dst = out + row * (M + 1);
     float2* sm = smem + rl * S;
     float2 v[E];
-    TM::run(v, sm, tw, t, rl, [&](int i) { return ok ? ld_stream(src + i) : make_float2(0.f, 0.f); });
+    TM::load_first(v, t, [&](int i) { return ok ? ld_stream(src + i) : make_float2(0.f, 0.f); });
+    constexpr unsigned AHEAD = prefetch_ahead(min_blocks_64regs(T * ROWS));
+    if (blockIdx.x + AHEAD < gridDim.x)
+        prefetch_span<ROWS * M * 8, T * ROWS>(in + ((uint64_t)blockIdx.x + AHEAD) * (ROWS * M), in + batch * M);
+    TM::template passes<0>(v, sm, tw, t, rl);
     pdl_trigger();
     RealSplit<TM, M, E>::store(v, sm, twr, t, rl, [&](int k, float2 X) {
         if constexpr (WEIGHTED) X = cscale(X, (k == 0 || k == M) ? s_edge : s_int);
@@ -219,6 +223,10 @@ k_c2r(const float2* __restrict__ in, float2* __restrict__ out, const float2* __r
     float2* sm = smem + rl * S;
     using RS = RealSplit<TM, M, E>;
     const auto x = RS::bins(t, [&](int k) { return ok ? ld_stream(src + k) : make_float2(0.f, 0.f); });
+    constexpr unsigned AHEAD = prefetch_ahead(min_blocks_64regs(T * ROWS));
+    if (blockIdx.x + AHEAD < gridDim.x)
+        prefetch_span<ROWS * (M + 1) * 8, T * ROWS>(in + ((uint64_t)blockIdx.x + AHEAD) * (ROWS * (M + 1)),
+                                                    in + batch * (M + 1));
     float2 v[E];
     RS::load(v, sm, twr, t, rl, x, s_edge, s_int, out_scale);
     TM::template passes<0>(v, sm, tw, t, rl);
@@ -233,6 +241,8 @@ k_c2r(const float2* __restrict__ in, float2* __restrict__ out, const float2* __r
 // and transforms along a middle axis of a contiguous [outer][n][inner] array (pitch = inner).
 // C consecutive columns per CTA with the column index fastest across threads, so every row
 // access is one C*8-byte segment; columns at or past ncols compute on zeros and store nothing.
+// (Numbering the columns of all matrices through, so that only the last CTA has idle columns, gave
+// nothing at 129 columns of 256 and cost 7 % at 1024 of 1024: the division delays the loads.)
 // Every load precedes the CTA's first __syncthreads and every store follows its last, so
 // in == out is allowed.
 template <int NY, int E, int C, bool INV>
@@ -243,6 +253,7 @@ k_cols(const float2* __restrict__ in, float2* __restrict__ out, const float2* __
     using TM = Team<NY, E, INV, kSyncBlock>;
     static_assert(TM::P >= 2, "in-place safety needs a barrier between loads and stores");
     extern __shared__ float2 smem[];
+    pdl_wait();
     const int c = threadIdx.x % C;
     const int t = threadIdx.x / C;
     const uint64_t m = blockIdx.x / colBlocks;
@@ -261,6 +272,7 @@ k_cols(const float2* __restrict__ in, float2* __restrict__ out, const float2* __
             if (i + (int)threadIdx.x < NY) prefetch_l2(next + (size_t)(i + threadIdx.x) * pitch);
     }
     TM::template passes<0>(v, smem + c * S, tw, t, 0);
+    pdl_trigger();
     if (live) TM::for_each_out(v, t, [&](int k, float2 x) { st_stream(dst + (size_t)k * pitch, cscale(x, scale)); });
 }
 

@@ -20,6 +20,7 @@
 
 #include "backend.h"
 #include "fft_kernels.cuh"
+#include "launch.cuh"
 
 namespace bfly {
 namespace dev {
@@ -42,6 +43,7 @@ k_bluestein(const float2* __restrict__ in, float2* __restrict__ out, const float
     using TF = Team<M, E, false, SYNC>;
     using TI = Team<M, E, true, SYNC>;
     extern __shared__ float2 smem[];
+    pdl_wait();
     const int rl = threadIdx.x / T;
     const int t = threadIdx.x - rl * T;
     const uint64_t row = (uint64_t)blockIdx.x * ROWS + rl;
@@ -70,6 +72,7 @@ k_bluestein(const float2* __restrict__ in, float2* __restrict__ out, const float
     const int ti = opaque(t, v[0].x);
     float2* smi = smem + opaque(rl, v[0].x) * S;
     TI::passes_transposed(v, smi, tw, ti, rl);
+    pdl_trigger();
     if (ok) {
 #pragma unroll
         for (int r = 0; r < E / 2; ++r) {   // only the first n <= M/2 outputs exist
@@ -132,10 +135,9 @@ int launchBluesteinM(const void* in, void* out, uint32_t n, uint64_t batch, floa
     if (int e = optInSharedMemory((const void*)fn, SMEM)) return e;
     const uint64_t grid = (batch + ROWS - 1) / ROWS;
     if (grid > 0x7fffffffull) return (int)cudaErrorInvalidValue;
-    fn<<<(unsigned)grid, CTA, SMEM, reinterpret_cast<cudaStream_t>(stream)>>>(
-        static_cast<const float2*>(in), static_cast<float2*>(out), static_cast<const float2*>(tw),
-        static_cast<const float2*>(chirp), static_cast<const float2*>(filt), n, batch, scale);
-    return (int)cudaGetLastError();
+    return (int)launchPdlKernel(fn, grid, CTA, SMEM, stream, static_cast<const float2*>(in), static_cast<float2*>(out),
+                                static_cast<const float2*>(tw), static_cast<const float2*>(chirp),
+                                static_cast<const float2*>(filt), n, batch, scale);
 }
 
 }  // namespace

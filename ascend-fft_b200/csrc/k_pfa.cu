@@ -12,6 +12,7 @@
 
 #include "backend.h"
 #include "fft_kernels.cuh"
+#include "launch.cuh"
 #include "fft_odd.cuh"
 
 namespace bfly {
@@ -100,6 +101,7 @@ k_pfa(const float2* __restrict__ in, float2* __restrict__ out, const float2* __r
     using TB = Team<B, E, INV, kSyncBlock>;   // every sync below is block-wide: all rows of the
                                              // CTA run the same number of barriers
     extern __shared__ float2 smem[];
+    pdl_wait();
     const int rl = threadIdx.x / T;
     const int tid = threadIdx.x - rl * T;
     const uint64_t row = (uint64_t)blockIdx.x * P::ROWS + rl;
@@ -118,6 +120,9 @@ k_pfa(const float2* __restrict__ in, float2* __restrict__ out, const float2* __r
             const int j = tid + i * T;
             rowA[spad(j & (B - 1))] = ok ? ld_stream(src + j) : make_float2(0.f, 0.f);
         }
+        constexpr unsigned AHEAD = prefetch_ahead(min_blocks_64regs(P::CTA));
+        if (blockIdx.x + AHEAD < gridDim.x)
+            prefetch_span<P::ROWS * N * 8, P::CTA>(in + ((uint64_t)blockIdx.x + AHEAD) * (P::ROWS * N), in + batch * N);
     }
     __syncthreads();
     // 2. B-point FFT of sub-row j1 by sub-team j1, results back in natural order k2
@@ -155,6 +160,7 @@ k_pfa(const float2* __restrict__ in, float2* __restrict__ out, const float2* __r
         }
     }
     __syncthreads();
+    pdl_trigger();
     // 4. coalesced stores of X[k] = Y[k1][k2]; across lanes k2 steps by the odd A^-1 mod B,
     //    a permutation of the banks
     if (ok) {
@@ -185,10 +191,9 @@ int launchPfaAB(const void* in, void* out, uint64_t batch, float scale, const vo
     if (int e = optInSharedMemory((const void*)fn, SMEM)) return e;
     const uint64_t grid = (batch + P::ROWS - 1) / P::ROWS;
     if (grid > 0x7fffffffull) return (int)cudaErrorInvalidValue;
-    fn<<<(unsigned)grid, P::CTA, SMEM, reinterpret_cast<cudaStream_t>(stream)>>>(
-        static_cast<const float2*>(in), static_cast<float2*>(out), static_cast<const float2*>(twB),
-        static_cast<const float2*>(wA), batch, scale);
-    return (int)cudaGetLastError();
+    return (int)launchPdlKernel(fn, grid, P::CTA, SMEM, stream, static_cast<const float2*>(in),
+                                static_cast<float2*>(out), static_cast<const float2*>(twB),
+                                static_cast<const float2*>(wA), batch, scale);
 }
 
 template <int A, bool INV>
