@@ -371,6 +371,16 @@ struct Team {
             for (int r = 0; r < R; ++r) v[s * R + r] = load(t + s * T + r * (N / R));
     }
 
+    // Apply f(index, value&) to every input element as load_first holds them.
+    template <class F>
+    static __device__ __forceinline__ void for_each_in(float2 (&v)[E], int t, F&& f) {
+        constexpr int R = S::radix(0);
+#pragma unroll
+        for (int s = 0; s < E / R; ++s)
+#pragma unroll
+            for (int r = 0; r < R; ++r) f(t + s * T + r * (N / R), v[s * R + r]);
+    }
+
     // The steps of pass p: twiddles and DFTs in registers, the results to the exchange buffer, the
     // next pass's inputs back from it.  A kernel may take them apart to hold another t after an
     // exchange than before it.

@@ -103,8 +103,8 @@ __device__ __forceinline__ void c2r_pair(float2 xk, float2 xm, bool edge, float2
 template <class TM, int M, int E>
 struct RealSplit {
     static constexpr int T = M / E, H = E / 2;
-    // v: a finished transform, as Team leaves it; emit(k, X[k]) for every bin k <= M of the team's
-    // row.  `sm` must be free once the team has synchronised.
+    // v: a finished transform, as Team leaves it; emit(k, X[k], k is 0 or M) for every bin
+    // k <= M of the team's row.  `sm` must be free once the team has synchronised.
     template <class Emit>
     static __device__ __forceinline__ void store(float2 (&v)[E], float2* sm, const float2* __restrict__ twr, int t,
                                                  int row, Emit&& emit) {
@@ -119,15 +119,15 @@ struct RealSplit {
         for (int j = 0; j < H; ++j) lo[j] = v[TM::slot(j)];
         mid = v[TM::slot(H)];
         TM::sync(row);
-        if (t == 0) emit(M / 2, cconj(mid));   // bin M/2 pairs with itself
+        if (t == 0) emit(M / 2, cconj(mid), false);   // bin M/2 pairs with itself
 #pragma unroll
         for (int j = 0; j < H; ++j) {
             const int k = t + j * T;
             const float2 b = j == 0 && t == 0 ? lo[0] : sm[spad(M / 2 - k)];
             float2 xk, xm;
             r2c_pair(lo[j], b, w[j], xk, xm);
-            emit(k, xk);
-            emit(M - k, xm);
+            emit(k, xk, j == 0 && t == 0);
+            emit(M - k, xm, j == 0 && t == 0);
         }
     }
 
@@ -195,8 +195,8 @@ k_r2c(const float2* __restrict__ in, float2* __restrict__ out, const float2* __r
         prefetch_span<ROWS * M * 8, T * ROWS>(in + ((uint64_t)blockIdx.x + AHEAD) * (ROWS * M), in + batch * M);
     TM::template passes<0>(v, sm, tw, t, rl);
     pdl_trigger();
-    RealSplit<TM, M, E>::store(v, sm, twr, t, rl, [&](int k, float2 X) {
-        if constexpr (WEIGHTED) X = cscale(X, (k == 0 || k == M) ? s_edge : s_int);
+    RealSplit<TM, M, E>::store(v, sm, twr, t, rl, [&](int k, float2 X, bool edge) {
+        if constexpr (WEIGHTED) X = cscale(X, edge ? s_edge : s_int);
         if (ok) st_stream(dst + k, X);
     });
 }

@@ -24,6 +24,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fft_core.cuh"
+
 namespace bfly {
 namespace dev {
 
@@ -35,12 +37,14 @@ struct IstftSegment {
     const float* window;
     float* dst;
     float *cur, *nxt, *rinv;
+    float scale;                                  // of the sums, folded into the envelope (ADJ: none)
     int pad = 0;                                  // ADJ: fold width (0: no reflect padding)
     float *foldL = nullptr, *foldR = nullptr;     // ADJ: outputs [0, pad] and [L-1-pad, L-1)
 
     // `scratch`: 2 (N - hop) + hop floats of shared memory (carry pair, then the envelope table).
     __device__ __forceinline__ void init(int n, uint32_t hop_, uint32_t frames_, uint32_t Q, uint32_t segs, int64_t start_,
-                                         uint64_t outLen_, const float* window_, float* out, float* scratch) {
+                                         uint64_t outLen_, const float* window_, float* out, float* scratch,
+                                         float scale_) {
         N = n;
         hop = hop_;
         frames = frames_;
@@ -60,12 +64,13 @@ struct IstftSegment {
         if (c + 1 == segs) fB = frames;   // a last segment may be longer than Q (ADJ launches)
         P1 = c + 1 == segs ? (padded > end ? padded : end) : (int64_t)fB * hop;
         window = window_;
+        scale = scale_;
         dst = out + (uint64_t)s * outLen;
         cur = scratch;
         nxt = cur + CARRY;
         rinv = nxt + CARRY;
         for (int q = threadIdx.x; q < CARRY; q += CTA) cur[q] = 0.f;
-        // 1 / (overlap-added squared window) of samples every frame slot of which exists
+        // scale / (overlap-added squared window) of samples every frame slot of which exists
         // (N-1 <= p < frames*hop): periodic in p with period hop
         for (int r = threadIdx.x; r < (int)hop; r += CTA) {
             float e = 0.f;
@@ -73,7 +78,7 @@ struct IstftSegment {
                 const float w = window ? __ldg(window + j) : 1.f;
                 e += w * w;
             }
-            rinv[r] = e > 0.f ? 1.f / e : 0.f;
+            rinv[r] = e > 0.f ? scale / e : 0.f;
         }
     }
 
@@ -134,15 +139,17 @@ struct IstftSegment {
                 e += w * w;
             }
         }
-        return e > 0.f ? 1.f / e : 0.f;
+        return e > 0.f ? scale / e : 0.f;
     }
 
-    // Overlap-add of the wave of frames f0 .. f0+R-1 held in shared memory: ld1(r, j) returns
-    // w[j] x_(f0+r)[j], ld4(r, j) the float4 of samples j .. j+3 (j a multiple of 4).  Called by
-    // every thread after a barrier that follows the frames' writes; swaps the carry halves.
+    // Overlap-add of the wave of frames f0 .. f0+R-1 held in shared memory, frame r at frames0 +
+    // r * stride: ld1(p, j) returns w[j] times the sample at p (sample j of its frame), ld4(p, j)
+    // the float4 of samples j .. j+3 (j a multiple of 4).  Called by every thread after a barrier
+    // that follows the frames' writes; swaps the carry halves.  The frames that cover a sample lie
+    // at one distance, stride - hop, from the oldest on, and only the oldest may end before it.
     // CTA_C: the block size when known at compile time (0: blockDim.x).
     template <int VEC, int CTA_C, bool ADJ = false, class Ld1, class Ld4>
-    __device__ __forceinline__ void wave(uint32_t f0, int R, Ld1&& ld1, Ld4&& ld4) {
+    __device__ __forceinline__ void wave(uint32_t f0, int R, const float* frames0, int stride, Ld1&& ld1, Ld4&& ld4) {
         const int cta = CTA_C > 0 ? CTA_C : CTA;
         auto clampq = [](int64_t v, int hi) { return (int)(v < 0 ? 0 : (v > hi ? hi : v)); };
         const bool tail = f0 + R == frames;   // no later frame: every sample of the span is complete
@@ -160,15 +167,20 @@ struct IstftSegment {
         const int stepH = VEC * cta / (int)hop, stepR = VEC * cta - stepH * (int)hop;
         int qh = VEC * (int)threadIdx.x / (int)hop;
         int qr = VEC * (int)threadIdx.x - qh * (int)hop;
+        const int next = stride - (int)hop;   // the same padded sample in the following frame
         for (int q = VEC * threadIdx.x; q < span; q += VEC * cta) {
-            const int rlo = qh - K + 1 > 0 ? qh - K + 1 : 0;
+            int r = qh - K + 1 > 0 ? qh - K + 1 : 0;
             const int rhi = qh < R - 1 ? qh : R - 1;
+            int j = qr + (qh - r) * (int)hop;
+            const float* p = frames0 + r * stride + j;
+            if (j >= N) {   // hop does not divide N: the oldest frame has ended
+                ++r;
+                j -= (int)hop;
+                p += next;
+            }
             if constexpr (VEC == 1) {
                 float val = q < CARRY ? cur[q] : 0.f;
-                for (int r = rlo; r <= rhi; ++r) {
-                    const int j = qr + (qh - r) * (int)hop;
-                    if (j < N) val += ld1(r, j);
-                }
+                for (; r <= rhi; ++r, j -= (int)hop, p += next) val += ld1(p, j);
                 if (q >= done) {
                     nxt[q - done] = val;
                 } else if (q >= wlo && q < whi) {
@@ -177,15 +189,12 @@ struct IstftSegment {
                 }
             } else {
                 float4 val = q < CARRY ? *reinterpret_cast<const float4*>(cur + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int r = rlo; r <= rhi; ++r) {
-                    const int j = qr + (qh - r) * (int)hop;
-                    if (j < N) {
-                        const float4 x = ld4(r, j);
-                        val.x += x.x;
-                        val.y += x.y;
-                        val.z += x.z;
-                        val.w += x.w;
-                    }
+#pragma unroll 4
+                for (; r <= rhi; ++r, j -= (int)hop, p += next) {
+                    const float4 x = ld4(p, j);
+                    const float2 lo = cadd(make_float2(val.x, val.y), make_float2(x.x, x.y));
+                    const float2 hi = cadd(make_float2(val.z, val.w), make_float2(x.z, x.w));
+                    val = make_float4(lo.x, lo.y, hi.x, hi.y);
                 }
                 if (q >= done) {
                     *reinterpret_cast<float4*>(nxt + q - done) = val;

@@ -444,26 +444,26 @@ __global__ void __launch_bounds__(512, 2) k_istft_mixed(const float2* __restrict
     const int M = a.n;
     IstftSegment seg;
     seg.init(2 * M, hop, frames, Q, segs, start, outLen, window, out,
-             reinterpret_cast<float*>(smem + (size_t)rows * 2 * len));
+             reinterpret_cast<float*>(smem + (size_t)rows * 2 * len), out_scale);
     const float2* src0 = spec + (uint64_t)(blockIdx.x / segs) * frames * (M + 1);
     float2* buf0 = smem + (size_t)rl * 2 * len;
     float2* buf1 = buf0 + len;
     const int finOff = ((a.passes - 1) & 1) ? len : 0;   // buffer the last pass writes
-    auto frameOf = [&](int r) { return reinterpret_cast<const float*>(smem + (size_t)r * 2 * len + finOff); };
 
     for (uint32_t f0 = seg.fA; f0 < seg.fB; f0 += rows) {
         const int R = (int)min((uint32_t)rows, seg.fB - f0);
         __syncthreads();   // the previous wave is done with the row buffers and the carry
         // rows past R (a CTA's partial first or last wave) transform frame f0 again, unread
         const float2* src = src0 + (uint64_t)(f0 + (rl < R ? rl : 0)) * (M + 1);
-        mixed_unsplit(src, buf1, twr, M, t, T, 1.f, 1.f, out_scale);
+        mixed_unsplit(src, buf1, twr, M, t, T, 1.f, 1.f, 1.f);
         __syncthreads();
         ROWS::template run<true, false, false>(a, nullptr, nullptr, buf0, buf1, tw, true, t, T, 1.f);
         __syncthreads();
         seg.wave<VEC, 0>(
-            f0, R, [&](int r, int j) { return (window ? __ldg(window + j) : 1.f) * frameOf(r)[j]; },
-            [&](int r, int j) {
-                const float4 x = *reinterpret_cast<const float4*>(frameOf(r) + j);
+            f0, R, reinterpret_cast<const float*>(smem) + finOff * 2, 4 * len,
+            [&](const float* p, int j) { return (window ? __ldg(window + j) : 1.f) * *p; },
+            [&](const float* p, int j) {
+                const float4 x = *reinterpret_cast<const float4*>(p);
                 const float4 w = window ? __ldg(reinterpret_cast<const float4*>(window + j)) : make_float4(1.f, 1.f, 1.f, 1.f);
                 return make_float4(w.x * x.x, w.y * x.y, w.z * x.z, w.w * x.w);
             });
