@@ -241,6 +241,8 @@ int launchCols(const void* in, void* out, uint32_t ny, uint32_t ncols, uint64_t 
                uint64_t mats, bool inverse, float scale, const void* tw, void* stream) {
     const Entry* x = dev::findCols(ny, inverse);
     if (!x || ncols == 0 || mats == 0) return (int)cudaErrorInvalidValue;
+    int staged = 0;
+    if (launchColsStaged(in, out, ny, ncols, pitch, matStride, mats, inverse, scale, tw, stream, &staged)) return staged;
     const uint32_t colBlocks = (ncols + (uint32_t)x->rows - 1) / (uint32_t)x->rows;
     const uint64_t grid = mats * colBlocks;
     if (grid > 0x7fffffffull) return (int)cudaErrorInvalidValue;

@@ -40,6 +40,11 @@ const Entry* findCols(uint32_t ny, bool inverse);   // rows = columns per CTA
 bool findTw(uint32_t n, int e, KTw* fn, int* count);
 
 }  // namespace dev
+namespace backend {
+// launchCols by k_staged (k_staged.cu) where that takes the call; *rc is its status.
+bool launchColsStaged(const void* in, void* out, uint32_t ny, uint32_t ncols, uint64_t pitch, uint64_t matStride,
+                      uint64_t mats, bool inverse, float scale, const void* tw, void* stream, int* rc);
+}  // namespace backend
 }  // namespace bfly
 
 // Geometry helpers for the instantiation macros.
