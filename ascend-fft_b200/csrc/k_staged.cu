@@ -94,16 +94,17 @@ k_staged(const float2* in, float2* out, const float2* __restrict__ tw, uint64_t 
 #pragma unroll
         for (int i = 0; i < N; i += G::NT / (C / 2)) cp_async16(dst + i * C, src + (uint64_t)(row + i) * pitch, live);
     };
-    uint64_t b = blockIdx.x;
-    if (b < strips) issue(b);
+    uint64_t left = blockIdx.x;   // strip strips - 1 - left: the last matrix first, as k_cols
+    if (left < strips) issue(strips - 1 - left);
     cp_async_commit();
-    for (; b < strips; b += gridDim.x) {
+    for (; left < strips; left += gridDim.x) {
+        const uint64_t b = strips - 1 - left;
         cp_async_wait_all();
         __syncthreads();   // the strip is staged, and the last one's exchanges are over
         float2 v[E];
         TM::load_first(v, t, [&](int i) { return stage[i * C + c]; });
         __syncthreads();   // the stage is free
-        if (b + gridDim.x < strips) issue(b + gridDim.x);
+        if (left + gridDim.x < strips) issue(b - gridDim.x);
         cp_async_commit();
         staged_passes<TM, E, 0>(v, plane + c * G::PLANE, tw, t);
         const uint32_t col = (uint32_t)(b % colBlocks) * C + c;
