@@ -46,14 +46,13 @@ __device__ __forceinline__ void ragged_tile(const RaggedEntry& r, uint64_t tileI
     const float sgn = r.direction > 0 ? -1.f : 1.f;   // conjugation for the inverse
     const float sc = r.scale;
     float2 v[E];
-    TM::run(v, smem + rl * S, static_cast<const float2*>(r.tw), t, rl, [&](int i) {
-        if (!ok) return make_float2(0.f, 0.f);
-        const float2 x = ld_stream(src + i);
-        return make_float2(x.x, sgn * x.y);
-    });
+    TM::load_first(v, t, [&](int i) { return ok ? ld_stream(src + i) : make_float2(0.f, 0.f); });
+    const float2 conj = make_float2(1.f, sgn), out = make_float2(sc, sgn * sc);
+#pragma unroll
+    for (int i = 0; i < E; ++i) v[i] = __fmul2_rn(v[i], conj);
+    TM::template passes<0>(v, smem + rl * S, static_cast<const float2*>(r.tw), t, rl);
     pdl_trigger();
-    if (ok)
-        TM::for_each_out(v, t, [&](int i, float2 x) { st_stream(dst + i, make_float2(x.x * sc, sgn * sc * x.y)); });
+    if (ok) TM::for_each_out(v, t, [&](int i, float2 x) { st_stream(dst + i, __fmul2_rn(x, out)); });
 }
 
 __device__ __forceinline__ int find_request_plain(const RaggedEntry* __restrict__ reqs, int nreq, uint64_t tile) {
