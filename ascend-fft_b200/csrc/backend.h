@@ -119,8 +119,13 @@ int launchPfa(const void* in, void* out, uint32_t n, uint64_t batch, bool invers
 
 // Any-length C2C (Bluestein), n in [2, kBluesteinMaxN], in one kernel per padded length M =
 // bluesteinM(n) (power of two >= 2n-1, >= 64).  Tables per n: chirp (n float2), filter (M
-// float2), built in FP64 on the device with an M-double2 scratch; tw = Stockham table (M, 16).
+// float2), built in FP64 on the device with an M-double2 scratch; tw = Stockham table (M, bluesteinE(M)).
 constexpr uint32_t kBluesteinMaxN = 8192;
+// Values per thread of the padded transforms: 32 where that takes a pass and an exchange off each
+// (us, 16 and 32: n = 151 x 32768 rows 54.0 / 46.3, 503 x 16384 64.4 / 51.5, 4093 x 2048 101.0 / 85.2,
+// 7001 x 1024 121.0 / 98.4); at M = 2048, three passes either way, 16 keeps more warps (n = 1003 x 8192
+// 65.2 / 76.1).
+constexpr int bluesteinE(uint32_t M) { return M == 512 || M == 1024 || M >= 8192 ? 32 : 16; }
 uint32_t bluesteinM(uint32_t n);   // 0 when n is outside [2, kBluesteinMaxN]
 int buildBluesteinTables(void* chirp, void* filt, void* scratch, uint32_t n, void* stream);
 int launchBluestein(const void* in, void* out, uint32_t n, uint64_t batch, bool inverse, float scale,

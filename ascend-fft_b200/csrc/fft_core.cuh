@@ -187,20 +187,6 @@ template <bool INV> struct DFT<16, INV> {
     }
 };
 
-// DFT16 of eight values and eight zeros: v[8..15] are zero whatever they hold.
-template <bool INV>
-__device__ __forceinline__ void dft16_low(float2* v) {
-    float2 y[4][4];
-#pragma unroll
-    for (int n2 = 0; n2 < 4; ++n2) {
-        const float2 a = v[n2], b = v[4 + n2];
-        y[0][n2] = cadd(a, b);
-        y[2][n2] = csub(a, b);
-        add_sub_i<INV>(a, b, y[1][n2], y[3][n2]);
-    }
-    dft16_rows<INV>(y, v);
-}
-
 // a * exp(-+2*pi*i*Q/32), Q compile-time.
 template <int Q, bool INV>
 __device__ __forceinline__ float2 rot32(float2 a) {
@@ -226,6 +212,18 @@ __device__ __forceinline__ void twiddle32(float2* v) {   // v[n2] *= W_32^(K1 n2
     }
 }
 // 32 = 4 x 8.
+template <bool INV>
+__device__ __forceinline__ void dft32_rows(float2 (&y)[4][8], float2* v) {   // y[k1][n2]
+    twiddle32<1, INV>(y[1]);
+    twiddle32<2, INV>(y[2]);
+    twiddle32<3, INV>(y[3]);
+#pragma unroll
+    for (int k1 = 0; k1 < 4; ++k1) {
+        DFT<8, INV>::run(y[k1]);
+#pragma unroll
+        for (int k2 = 0; k2 < 8; ++k2) v[k1 + 4 * k2] = y[k1][k2];
+    }
+}
 template <bool INV> struct DFT<32, INV> {
     static __device__ __forceinline__ void run(float2* v) {
         float2 y[4][8];
@@ -236,17 +234,25 @@ template <bool INV> struct DFT<32, INV> {
 #pragma unroll
             for (int k1 = 0; k1 < 4; ++k1) y[k1][n2] = c[k1];
         }
-        twiddle32<1, INV>(y[1]);
-        twiddle32<2, INV>(y[2]);
-        twiddle32<3, INV>(y[3]);
-#pragma unroll
-        for (int k1 = 0; k1 < 4; ++k1) {
-            DFT<8, INV>::run(y[k1]);
-#pragma unroll
-            for (int k2 = 0; k2 < 8; ++k2) v[k1 + 4 * k2] = y[k1][k2];
-        }
+        dft32_rows<INV>(y, v);
     }
 };
+
+// DFT of R = 16 or 32 values whose upper half is zero, whatever v holds there.
+template <int R, bool INV>
+__device__ __forceinline__ void dft_low(float2* v) {
+    constexpr int B = R / 4;
+    float2 y[4][B];
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) {
+        const float2 a = v[n2], b = v[B + n2];
+        y[0][n2] = cadd(a, b);
+        y[2][n2] = csub(a, b);
+        add_sub_i<INV>(a, b, y[1][n2], y[3][n2]);
+    }
+    if constexpr (R == 16) dft16_rows<INV>(y, v);
+    else dft32_rows<INV>(y, v);
+}
 
 // ------------------------------------------------------------------ pass schedule
 // Greedy radix schedule: radix E while it divides the remaining length, remainder last.

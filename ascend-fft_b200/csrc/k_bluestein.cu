@@ -10,10 +10,11 @@
 // registers and shared memory, multiplies by the filter, runs the inverse FFT by the transposed
 // graph (Team::passes_transposed: it starts from the registers the forward one ends in, one
 // exchange less than re-entering through shared memory), multiplies by c and stores the first n
-// outputs.  n <= M/2, so the first DFT16 has eight zero inputs and the last one eight outputs
-// nobody reads.  What bounds it: shared memory and L1 (83 % of their wavefront rate in ncu:
+// outputs.  n <= M/2, so half the inputs of the first butterfly are zero and half the outputs of
+// the last are not read.  What bounds it: shared memory and L1 (83 % of their wavefront rate in ncu:
 // exchanges, twiddles, filter and chirp).  n = 1003, 8192 rows: 90.2 us re-entering through
-// shared memory, 73.7 us so.  The inverse transform uses
+// shared memory, 70.0 us so, 65.2 us with the chirp loaded beside the row instead of behind each
+// element's bounds check.  The inverse transform uses
 // conj(c) and conj(filter): h is symmetric (h[M-m] = h[m]), so the filter of conj(h) is the
 // conjugate of the filter of h.
 #include <cuda_runtime.h>
@@ -33,7 +34,7 @@ __device__ __forceinline__ int opaque(int x, float dep) {
 }
 
 template <int M, int E, int ROWS, bool INV>
-__global__ void __launch_bounds__((M / E) * ROWS, min_blocks_64regs((M / E) * ROWS))
+__global__ void __launch_bounds__((M / E) * ROWS, min_blocks<E>((M / E) * ROWS))
 k_bluestein(const float2* __restrict__ in, float2* __restrict__ out, const float2* __restrict__ tw,
             const float2* __restrict__ chirp, const float2* __restrict__ filt, uint32_t n, uint64_t batch,
             float scale) {
@@ -53,13 +54,18 @@ k_bluestein(const float2* __restrict__ in, float2* __restrict__ out, const float
     float2* sm = smem + rl * S;
     const int len = (int)n;
     float2 v[E];
-    static_assert(TF::S::radix(0) == 16 && E == 16 && TF::P >= 2, "pass 0 is one DFT16 per thread");
+    static_assert(TF::S::radix(0) == E && E >= 16 && TF::P >= 2, "pass 0 is one butterfly per thread");
+    float2 c[E / 2];
 #pragma unroll
     for (int r = 0; r < E / 2; ++r) {   // n <= M/2: the upper half of the padded row is zero
         const int i = t + r * T;
-        v[r] = (ok && i < len) ? cmul<INV>(ld_stream(src + i), __ldg(chirp + i)) : make_float2(0.f, 0.f);
+        v[r] = ok && i < len ? ld_stream(src + i) : make_float2(0.f, 0.f);
     }
-    dft16_low<false>(v);
+#pragma unroll
+    for (int r = 0; r < E / 2; ++r) c[r] = __ldg(chirp + min(t + r * T, len - 1));
+#pragma unroll
+    for (int r = 0; r < E / 2; ++r) v[r] = cmul<INV>(v[r], c[r]);   // all loads in flight before the first product
+    dft_low<E, false>(v);
     TF::template put<0>(v, sm, t);
     TF::sync(rl);
     TF::template get<1>(v, sm, t);
@@ -73,11 +79,14 @@ k_bluestein(const float2* __restrict__ in, float2* __restrict__ out, const float
     float2* smi = smem + opaque(rl, v[0].x) * S;
     TI::passes_transposed(v, smi, tw, ti, rl);
     pdl_trigger();
-    if (ok) {
+    if (ok) {   // only the first n <= M/2 outputs exist
 #pragma unroll
-        for (int r = 0; r < E / 2; ++r) {   // only the first n <= M/2 outputs exist
+        for (int r = 0; r < E / 2; ++r) c[r] = __ldg(chirp + min(ti + r * T, len - 1));
+#pragma unroll
+        for (int r = 0; r < E / 2; ++r) {
             const int k = ti + r * T;
-            if (k < len) st_stream(dst + k, cscale(cmul<INV>(v[r], __ldg(chirp + k)), scale));
+            const float2 x = cscale(cmul<INV>(v[r], c[r]), scale);
+            if (k < len) st_stream(dst + k, x);
         }
     }
 }
@@ -127,8 +136,8 @@ namespace {
 template <int M, bool INV>
 int launchBluesteinM(const void* in, void* out, uint32_t n, uint64_t batch, float scale, const void* tw,
                      const void* chirp, const void* filt, void* stream) {
-    constexpr int E = 16, T = M / E;
-    constexpr int CTA = T < 256 ? 256 : T;
+    constexpr int E = bluesteinE(M), T = M / E;
+    constexpr int CTA = T < 4096 / E ? 4096 / E : T;   // at least 4096 values
     constexpr int ROWS = CTA / T;
     constexpr int SMEM = ROWS * dev::smem_stride<M, E, false>() * 8;
     auto* fn = dev::k_bluestein<M, E, ROWS, INV>;

@@ -45,7 +45,7 @@ static const TwEntry kTw[] = {
     TW_(256, 8), TW_(256, 16), TW_(512, 8), TW_(512, 16), TW_(1024, 8), TW_(1024, 16),
     TW_(2048, 8), TW_(2048, 16), TW_(4096, 8), TW_(4096, 16), TW_(8192, 8), TW_(8192, 16),
     TW_(16384, 8), TW_(16384, 16),
-    TW_(512, 32), TW_(1024, 32), TW_(2048, 32), TW_(4096, 32),   // columns
+    TW_(512, 32), TW_(1024, 32), TW_(2048, 32), TW_(4096, 32), TW_(8192, 32), TW_(16384, 32),
 };
 #undef TW_
 

@@ -636,7 +636,7 @@ int Plan::prepareAnyLength(uint32_t n) {
 
 int Plan::prepareBluestein(uint32_t n) {
     const uint32_t M = backend::bluesteinM(n);
-    if (!M || prepareC2C(M, kColsE)) return -1;
+    if (!M || prepareC2C(M, backend::bluesteinE(M))) return -1;
     if (impl_->bluestein.count(n)) return 0;
     Impl::Chirp t;
     void* scratch = nullptr;
@@ -703,8 +703,9 @@ int Plan::execC2CWith(const void* dIn, void* dOut, uint32_t n, uint64_t batch, i
     if (!pow2(n) || n < kMinN) {   // Bluestein: one kernel on the padded power-of-two length
         if (prepareBluestein(n)) return -2;
         const auto& t = impl_->bluestein[n];
-        if (backend::launchBluestein(dIn, dOut, n, batch, inv, scale,
-                                     impl_->twC2C[{backend::bluesteinM(n), kColsE}], t.chirp, t.filt, s))
+        const uint32_t M = backend::bluesteinM(n);
+        if (backend::launchBluestein(dIn, dOut, n, batch, inv, scale, impl_->twC2C[{M, backend::bluesteinE(M)}],
+                                     t.chirp, t.filt, s))
             return -5;
         return 0;
     }
