@@ -98,7 +98,7 @@ MixedShape mixedShape(const MixedRadix& plan) {
     m.args.magic0 =
         m.args.pad0 ? (unsigned)((0x100000000ull + m.args.pad0 - 1) / (unsigned long long)m.args.pad0) : 0u;
     m.smem = m.rows * 2 * m.len * 8;
-    const int warps = (m.rows * m.T + 31) / 32;   // 64 registers a thread: 32 warps per SM
+    const int warps = (m.rows * m.T + 31) / 32;   // at 64 registers a thread 32 warps per SM
     m.args.ahead = dev::prefetch_ahead(std::max(1, std::min(32 / warps, kMixedMaxSmem / m.smem)));
     return m;
 }

@@ -196,28 +196,38 @@ int launchPfaAB(const void* in, void* out, uint64_t batch, float scale, const vo
                                 static_cast<const float2*>(wA), batch, scale);
 }
 
+// Whether n = A*B runs here rather than on the mixed-radix kernel.  The five trips through shared
+// memory pay where B is long enough for its passes, or so short (16) that it has one; at 32 and 64,
+// and for A = 15 up to 128, the two or three plain passes are ahead (us at 2^24 points, here and
+// there: n = 96 97.0 / 62.4, 192 88.1 / 55.2, 288 81.0 / 74.4, 240 98.8 / 45.6, 960 77.9 / 64.1; n = 768 55.7 /
+// 64.7, 144 61.3 / 65.5, 3840 60.1 / 67.1).
+constexpr bool pfaTaken(uint32_t a, uint32_t b) {
+    return a * b <= kPfaMaxN && b != 32 && b != 64 && !(a == 15 && b <= 128);
+}
+
+template <int A, int B, bool INV>
+int launchPfaIf(const void* in, void* out, uint64_t batch, float scale, const void* twB, const void* wA,
+                void* stream) {
+    if constexpr (pfaTaken(A, B)) return launchPfaAB<A, B, INV>(in, out, batch, scale, twB, wA, stream);
+    return (int)cudaErrorInvalidValue;
+}
+
 template <int A, bool INV>
 int launchPfaA(const void* in, void* out, uint32_t b, uint64_t batch, float scale, const void* twB,
                const void* wA, void* stream) {
+#define BFLY_PB(B) \
+    case B: return launchPfaIf<A, B, INV>(in, out, batch, scale, twB, wA, stream)
     switch (b) {
-        case 16: return launchPfaAB<A, 16, INV>(in, out, batch, scale, twB, wA, stream);
-        case 32: return launchPfaAB<A, 32, INV>(in, out, batch, scale, twB, wA, stream);
-        case 64: return launchPfaAB<A, 64, INV>(in, out, batch, scale, twB, wA, stream);
-        case 128: return launchPfaAB<A, 128, INV>(in, out, batch, scale, twB, wA, stream);
-        case 256: return launchPfaAB<A, 256, INV>(in, out, batch, scale, twB, wA, stream);
-        case 512: return launchPfaAB<A, 512, INV>(in, out, batch, scale, twB, wA, stream);
-        case 1024:
-            if constexpr (A * 1024 <= kPfaMaxN) return launchPfaAB<A, 1024, INV>(in, out, batch, scale, twB, wA, stream);
-            break;
-        case 2048:
-            if constexpr (A * 2048 <= kPfaMaxN) return launchPfaAB<A, 2048, INV>(in, out, batch, scale, twB, wA, stream);
-            break;
-        case 4096:
-            if constexpr (A * 4096 <= kPfaMaxN) return launchPfaAB<A, 4096, INV>(in, out, batch, scale, twB, wA, stream);
-            break;
-        default: break;
+        BFLY_PB(16);
+        BFLY_PB(128);
+        BFLY_PB(256);
+        BFLY_PB(512);
+        BFLY_PB(1024);
+        BFLY_PB(2048);
+        BFLY_PB(4096);
+        default: return (int)cudaErrorInvalidValue;
     }
-    return (int)cudaErrorInvalidValue;
+#undef BFLY_PB
 }
 
 }  // namespace
@@ -227,7 +237,7 @@ bool pfaSplit(uint32_t n, uint32_t* a, uint32_t* b) {
     for (uint32_t A : {3u, 5u, 9u, 15u}) {
         if (n % A) continue;
         const uint32_t B = n / A;
-        if (B >= 16 && !(B & (B - 1)) && n <= kPfaMaxN) {
+        if (B >= 16 && !(B & (B - 1)) && pfaTaken(A, B)) {
             *a = A;
             *b = B;
         }

@@ -266,8 +266,12 @@ __device__ __forceinline__ float2* fixed_row(const float2* src, float2* dst, flo
 
 // Row policies of the kernels below: the runtime pass list (radix class CLS) or a plan fixed at
 // compile time (Rs; launched with its T and pad0 only).
+// kRegs: 64 leave room for 32 warps per SM.  Shared memory holds most plans of class 1 to 25 warps,
+// which 80 registers allow too, and at 64 its butterflies spill (n = 1536: 130.3 us at 64, 116.2 at
+// 80, 124.8 at 96); classes 0 and 2 lose by it (n = 1000: 137.4, 154.0; 1001: 161.5, 169.8).
 template <int CLS>
 struct GenericRows {
+    static constexpr int kRegs = CLS == 1 ? 80 : 64;
     template <bool INV, bool SRC_HBM, bool DST_HBM>
     static __device__ __forceinline__ float2* run(const MixedArgs& a, const float2* src, float2* dst, float2* buf0,
                                                   float2* buf1, const float2* __restrict__ tw, bool ok, int t, int T,
@@ -277,6 +281,7 @@ struct GenericRows {
 };
 template <int... Rs>
 struct FixedRows {
+    static constexpr int kRegs = 64;
     template <bool INV, bool SRC_HBM, bool DST_HBM>
     static __device__ __forceinline__ float2* run(const MixedArgs& a, const float2* src, float2* dst, float2* buf0,
                                                   float2* buf1, const float2* __restrict__ tw, bool ok, int t, int,
@@ -287,7 +292,7 @@ struct FixedRows {
 };
 
 template <bool INV, class ROWS>
-__global__ void __launch_bounds__(512, 2) k_mixed(const float2* __restrict__ in, float2* __restrict__ out,
+__global__ void __maxnreg__(ROWS::kRegs) k_mixed(const float2* __restrict__ in, float2* __restrict__ out,
                                                   const float2* __restrict__ tw, MixedArgs a, uint64_t batch, int T,
                                                   int rows, int len, float scale) {
     extern __shared__ float2 smem[];
@@ -307,7 +312,7 @@ __global__ void __launch_bounds__(512, 2) k_mixed(const float2* __restrict__ in,
 // shared memory, then bins k and M - k by pairs (r2c_pair), times s_edge at bins 0 and M and s_int
 // elsewhere.
 template <class ROWS>
-__global__ void __launch_bounds__(512, 2) k_r2c_mixed(const float2* __restrict__ in, float2* __restrict__ out,
+__global__ void __maxnreg__(ROWS::kRegs) k_r2c_mixed(const float2* __restrict__ in, float2* __restrict__ out,
                                                       const float2* __restrict__ tw, const float2* __restrict__ twr,
                                                       MixedArgs a, uint64_t batch, int T, int rows, int len,
                                                       float s_edge, float s_int) {
@@ -353,7 +358,7 @@ __device__ __forceinline__ void mixed_unsplit(const float2* __restrict__ src, fl
 }
 
 template <class ROWS>
-__global__ void __launch_bounds__(512, 2) k_c2r_mixed(const float2* __restrict__ in, float2* __restrict__ out,
+__global__ void __maxnreg__(ROWS::kRegs) k_c2r_mixed(const float2* __restrict__ in, float2* __restrict__ out,
                                                       const float2* __restrict__ tw, const float2* __restrict__ twr,
                                                       MixedArgs a, uint64_t batch, int T, int rows, int len,
                                                       float s_edge, float s_int, float out_scale) {
@@ -376,7 +381,7 @@ __global__ void __launch_bounds__(512, 2) k_c2r_mixed(const float2* __restrict__
 // STFT: frame f of signal s, y[j] = w[j] x_s[f hop + j - (center ? N/2 : 0)] (reflect padding,
 // as k_stft), packed as z[m] = y[2m] + i y[2m+1] and staged unpadded; then the R2C of k_r2c_mixed.
 template <class ROWS>
-__global__ void __launch_bounds__(512, 2) k_stft_mixed(const float* __restrict__ sig, float2* __restrict__ out,
+__global__ void __maxnreg__(ROWS::kRegs) k_stft_mixed(const float* __restrict__ sig, float2* __restrict__ out,
                                                        const float2* __restrict__ tw, const float2* __restrict__ twr,
                                                        const float* __restrict__ window, MixedArgs a, uint64_t frames,
                                                        uint32_t framesPerSignal, int64_t sigLen, uint64_t sigStride,
@@ -432,7 +437,7 @@ __global__ void __launch_bounds__(512, 2) k_stft_mixed(const float* __restrict__
 // inverse passes into its natural-order row buffer; the segment split, carry, envelope and
 // overlap-add (window applied there) are IstftSegment (istft_ola.cuh), as in k_istft.
 template <class ROWS, int VEC>
-__global__ void __launch_bounds__(512, 2) k_istft_mixed(const float2* __restrict__ spec, float* __restrict__ out,
+__global__ void __maxnreg__(ROWS::kRegs) k_istft_mixed(const float2* __restrict__ spec, float* __restrict__ out,
                                                         const float2* __restrict__ tw, const float2* __restrict__ twr,
                                                         const float* __restrict__ window, MixedArgs a, uint32_t frames,
                                                         uint32_t hop, uint32_t Q, uint32_t segs, int64_t start,
