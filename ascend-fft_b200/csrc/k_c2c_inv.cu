@@ -8,6 +8,8 @@ namespace dev {
 
 #define E_(N, E, CTA) {N, E, CTA, 1, (const void*)&k_c2c<N, E, BFLY_ROWS(N, E, CTA), true>, \
     BFLY_ROWS(N, E, CTA), BFLY_ROWS(N, E, CTA) * smem_stride<N, E, false>() * 8}
+// Radix 16 served by k_long_direct.cu; listed for the candidates' limits.
+#define D_(N, CTA) {N, 16, CTA, 1, nullptr, BFLY_ROWS(N, 16, CTA), BFLY_ROWS(N, 16, CTA) * smem_stride<N, 16, false>() * 8}
 static const Entry kTable[] = {
     E_(32, 8, 128),
     E_(32, 8, 256),
@@ -42,9 +44,9 @@ static const Entry kTable[] = {
     E_(1024, 8, 128),
     E_(1024, 8, 256),
     E_(1024, 8, 512),
-    E_(1024, 16, 128),
-    E_(1024, 16, 256),
-    E_(1024, 16, 512),
+    D_(1024, 128),
+    D_(1024, 256),
+    D_(1024, 512),
     E_(2048, 8, 256),
     E_(2048, 8, 512),
     E_(2048, 16, 128),
@@ -54,10 +56,10 @@ static const Entry kTable[] = {
     E_(4096, 16, 256),
     E_(4096, 16, 512),
     E_(8192, 8, 1024),
-    // served by the one-pass kernels of k_long_direct.cu; listed for the candidates' limits
-    {8192, 16, 512, 1, nullptr, 1, smem_stride<8192, 16, false>() * 8},
-    {16384, 16, 1024, 1, nullptr, 1, smem_stride<16384, 16, false>() * 8},
+    D_(8192, 512),
+    D_(16384, 1024),
 };
+#undef D_
 #undef E_
 
 const Entry* findC2CInv(uint32_t n, int e, int cta) {

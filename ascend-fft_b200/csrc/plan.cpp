@@ -493,15 +493,15 @@ bool Plan::validShape(uint32_t n, uint32_t batch, int kind) const {
 // Kernel variant for (kind, n): the candidate's radix/cta when compiled for n (one CTA per
 // transform, e = radix); otherwise, for long C2C lengths, the one-pass kernels (e = -3), the L2
 // ring (e = -2), one persistent thread-block cluster per row (e = -1) or the four-step kernels
-// (e = 0), by the candidate's schedule.  The one-pass kernels take "stockham" candidates at every
-// long length: at batch*n = 2^26 they run 1.1x (n = 8192) to 1.3x (32768) as fast as what served
+// (e = 0), by the candidate's schedule.  The one-pass kernels take "stockham" candidates of radix 16
+// at 1024 and at every long length: they run 1.1x (1024) to 1.3x (8192, 32768) as fast as what served
 // those before, radix-16 single CTAs up to 16384 and four-step above (k_long_direct.cu).
 int Plan::resolve(int kind, uint32_t n, int* e, int* cta) const {
     const int r = cand_.p.radix, c = cand_.a.ctaThreads;
     if (kind == backend::kC2C) {
         const std::string& sched = cand_.f.schedule;
         if (sched == "stockham" && (r == 16 || !backend::hasVariant(backend::kC2C, n, r, c)) &&
-            backend::longDirectTableBytes && backend::longDirectTableBytes(n)) {
+            backend::directTableBytes && backend::directTableBytes(n)) {
             *e = -3;
             *cta = 256;
             return 0;
@@ -591,8 +591,8 @@ int Plan::prepareLong(uint32_t n) {
 int Plan::prepareDirect(uint32_t n) {
     if (impl_->twDirect.count(n)) return 0;
     void* t = nullptr;
-    if (backend::alloc(&t, backend::longDirectTableBytes(n))) return -1;
-    if (backend::buildLongDirectTable(t, n, stream_) || backend::streamSync(stream_)) {
+    if (backend::alloc(&t, backend::directTableBytes(n))) return -1;
+    if (backend::buildDirectTable(t, n, stream_) || backend::streamSync(stream_)) {
         backend::release(t);
         return -1;
     }
@@ -718,7 +718,7 @@ int Plan::execC2CWith(const void* dIn, void* dOut, uint32_t n, uint64_t batch, i
     }
     if (e == -3) {
         if (prepareDirect(n)) return -2;
-        return backend::launchLongDirect(dIn, dOut, n, batch, inv, scale, impl_->twDirect[n], s) ? -5 : 0;
+        return backend::launchDirect(dIn, dOut, n, batch, inv, scale, impl_->twDirect[n], s) ? -5 : 0;
     }
     if (prepareLong(n)) return -2;
     uint32_t n1 = 0, n2 = 0;
