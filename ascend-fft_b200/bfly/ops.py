@@ -1,8 +1,7 @@
 """torch.fft-style functions on CUDA tensors backed by the hand-written sm_100a kernels, with
 hand-written adjoints behind torch.autograd.Function:
 
-    fft(x, dim) / ifft(x, dim)  complex64, n in 32..65536 along the last dim (four-step above
-                            16384 points per row), 32..4096 along any other dim (column kernel
+    fft(x, dim) / ifft(x, dim)  complex64, n in 32..65536 along the last dim, 32..4096 along any other dim (column kernel
                             over the contiguous [outer][n][inner] view)
     fft2(x) / ifft2(x)      complex64 [..., ny, nx]: row pass (nx as fft) + column pass
                             (ny in 32..4096)

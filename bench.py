@@ -618,7 +618,7 @@ class Subs:
         emit({"sub": "long_fwd_bwd", "unit": UNIT,
               "cols": ["fwd_gbs", "bwd_gbs", "fwd_rel_l2", "bwd_rel_l2", "ring_fwd_gbs", "ring_rel_l2",
                        "cufft_fwd_gbs", "cufft_inv_gbs"],
-              "schedule": "single pass n <= 16384, two-kernel four-step above; ring = one-launch four-step",
+              "schedule": "one pass: a CTA per row n <= 16384, a cluster per row above; ring = one-launch four-step",
               "rows": {f"n{n}_b{(1 << 26) // n}": v for n, v in res.items()}})
         self.summary["long_fwd_bwd_frac"] = {str(n): [round(v[0] / peak, 3), round(v[1] / peak, 3)] for n, v in res.items()}
 

@@ -218,7 +218,8 @@ public:
     // the CUDA default stream, stream() the context stream) and return; no host
     // synchronisation, no host<->device copies.
     //   direction -1 forward, +1 inverse; scale multiplies the output.
-    //   n in [32, 16384] single pass, [8192, 65536] four-step (workspace grown on demand);
+    //   n in [32, 65536] in a single pass, or n in [8192, 65536] by the candidate's schedule
+    //   (four_step and ring grow a workspace on demand);
     //   n = A * 2^k (A in {3, 5, 9, 15}, 2^k >= 16, n <= 12288) by the prime-factor mapping in
     //   one kernel; other n = 2^a 3^b 5^c 7^d 11^e 13^f <= 12288 (2..16 included) by mixed-radix Stockham
     //   passes in one kernel; any other n in [2, 8192] by Bluestein's algorithm in one kernel
