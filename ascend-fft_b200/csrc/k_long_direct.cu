@@ -18,7 +18,7 @@
 // (32-byte runs through a layout that saves an exchange measured 2545 GB/s against 3374): the
 // row FFTs load with 16 threads along a row and change to 16 rows across lanes at their one
 // exchange, so that the stride-N1 stores are 128-byte runs too.
-// 2^26 points, one launch, GB/s at n = 32768 / 65536: 3828 / 3379 before the loads ahead, against
+// 2^26 points, one launch, GB/s at n = 32768 / 65536: 3828 / 3379 (loads ahead into L2 add nothing), against
 // 2980 / 2925 for the two four-step kernels, each of which crosses HBM; exchanging through
 // distributed shared memory instead of L2 3009 / 2565, 8192 points per CTA (512 threads) 3318 /
 // 3104.  What bounds it: the wait for the matrix writes to reach L2 at the first cluster barrier,
@@ -45,7 +45,6 @@ struct LongDirect {
     static constexpr int S2 = (spad(N2 - 1) + 1) | 1;   // odd: rows across lanes hit distinct banks
     static constexpr int SMEM = (COLS * S1 > ROWS2 * S2 ? COLS * S1 : ROWS2 * S2) * 8;
     static_assert(COLS * T1 == NT && ROWS2 * (N2 / E) == NT, "inconsistent cluster shape");
-    static_assert(COLS % 16 == 0, "column slices are whole lines");
     // one table: Stockham twiddles of N1 and of 256, then rows of 256 values W_n^(n2 T1 j), j < 16,
     // and W_n^(n2 t), t < T1
     static constexpr int TW2 = Sched<N1, E>::TWSIZE, WT = TW2 + Sched<N2, E>::TWSIZE, TABLE = WT + (E + T1) * N2;
@@ -70,11 +69,6 @@ k_long_direct(const float2* in, float2* out, const float2* __restrict__ table, f
         const uint32_t n2 = rank * L::COLS + c;
         const float2* src = in + row * L::N + n2;
         TA::load_first(v, t1, [&](int i) { return ld_once_ca(src + i * L::N2); });
-        constexpr unsigned AHEAD = prefetch_ahead(min_blocks_64regs(L::NT)) / L::C * L::C;
-        if (blockIdx.x + AHEAD < gridDim.x) {   // this rank's columns of a later row, one line a thread
-            constexpr int LINES = L::COLS * 8 / 128;
-            prefetch_l2(in + (row + AHEAD / L::C) * L::N + (tid / LINES) * L::N2 + rank * L::COLS + tid % LINES * 16);
-        }
         TA::template passes<0>(v, smem + c * L::S1, table, t1, 0);
         const float2* wt = table + L::WT + n2;
         const float2 w0 = __ldg(wt + (E + t1) * L::N2);
