@@ -89,9 +89,10 @@ __device__ __forceinline__ void c2r_pair(float2 xk, float2 xm, bool edge, float2
         xm = cscale(xm, s_int);
     }
     const float2 ev = make_float2(xk.x + xm.x, xk.y - xm.y);
-    const float2 od = cmul<true>(make_float2(xk.x - xm.x, xk.y + xm.y), w);
-    zk = cscale(make_float2(ev.x - od.y, ev.y + od.x), out_scale);
-    zm = cscale(make_float2(ev.x + od.y, od.x - ev.y), out_scale);
+    // the scale rides on the twiddle and on the sums' multiply-adds
+    const float2 od = cmul<true>(make_float2(xk.x - xm.x, xk.y + xm.y), cscale(w, out_scale));
+    zk = make_float2(fmaf(ev.x, out_scale, -od.y), fmaf(ev.y, out_scale, od.x));
+    zm = make_float2(fmaf(ev.x, out_scale, od.y), fmaf(-ev.y, out_scale, od.x));
 }
 
 // The split of one row held by a team (TM = Team<M, E, ...>), pairs (k, M-k) with k = t + j T,

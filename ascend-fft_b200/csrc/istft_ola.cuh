@@ -37,14 +37,12 @@ struct IstftSegment {
     const float* window;
     float* dst;
     float *cur, *nxt, *rinv;
-    float scale;                                  // of the sums, folded into the envelope (ADJ: none)
     int pad = 0;                                  // ADJ: fold width (0: no reflect padding)
     float *foldL = nullptr, *foldR = nullptr;     // ADJ: outputs [0, pad] and [L-1-pad, L-1)
 
     // `scratch`: 2 (N - hop) + hop floats of shared memory (carry pair, then the envelope table).
     __device__ __forceinline__ void init(int n, uint32_t hop_, uint32_t frames_, uint32_t Q, uint32_t segs, int64_t start_,
-                                         uint64_t outLen_, const float* window_, float* out, float* scratch,
-                                         float scale_) {
+                                         uint64_t outLen_, const float* window_, float* out, float* scratch) {
         N = n;
         hop = hop_;
         frames = frames_;
@@ -64,13 +62,12 @@ struct IstftSegment {
         if (c + 1 == segs) fB = frames;   // a last segment may be longer than Q (ADJ launches)
         P1 = c + 1 == segs ? (padded > end ? padded : end) : (int64_t)fB * hop;
         window = window_;
-        scale = scale_;
         dst = out + (uint64_t)s * outLen;
         cur = scratch;
         nxt = cur + CARRY;
         rinv = nxt + CARRY;
         for (int q = threadIdx.x; q < CARRY; q += CTA) cur[q] = 0.f;
-        // scale / (overlap-added squared window) of samples every frame slot of which exists
+        // 1 / (overlap-added squared window) of samples every frame slot of which exists
         // (N-1 <= p < frames*hop): periodic in p with period hop
         for (int r = threadIdx.x; r < (int)hop; r += CTA) {
             float e = 0.f;
@@ -78,7 +75,7 @@ struct IstftSegment {
                 const float w = window ? __ldg(window + j) : 1.f;
                 e += w * w;
             }
-            rinv[r] = e > 0.f ? scale / e : 0.f;
+            rinv[r] = e > 0.f ? 1.f / e : 0.f;
         }
     }
 
@@ -139,7 +136,7 @@ struct IstftSegment {
                 e += w * w;
             }
         }
-        return e > 0.f ? scale / e : 0.f;
+        return e > 0.f ? 1.f / e : 0.f;
     }
 
     // Overlap-add of the wave of frames f0 .. f0+R-1 held in shared memory, frame r at frames0 +

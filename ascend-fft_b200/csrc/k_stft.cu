@@ -155,7 +155,7 @@ k_istft(const float2* __restrict__ spec, float* __restrict__ out, const float2* 
     const int t = threadIdx.x - rl * T;
     IstftSegment seg;
     float* scratch = reinterpret_cast<float*>(smem + ROWS * S);
-    seg.init(N, hop, frames, Q, segs, start, outLen, window, out, scratch, out_scale);
+    seg.init(N, hop, frames, Q, segs, start, outLen, window, out, scratch);
     if constexpr (ADJ) seg.initFold(pad, scratch + 2 * (N - (int)hop) + (int)hop);
     const float2* src0 = spec + (uint64_t)(blockIdx.x / segs) * frames * (M + 1);
     float2* sm = smem + rl * S;
@@ -168,7 +168,7 @@ k_istft(const float2* __restrict__ spec, float* __restrict__ out, const float2* 
         const auto x = RS::bins(t, [&](int k) { return ld_stream(src + k); });
         __syncthreads();   // the previous wave is done with the row buffers and the carry
         float2 v[E];
-        RS::load(v, sm, twr, t, rl, x, ADJ ? s_edge : 1.f, ADJ ? s_int : 1.f, 1.f);
+        RS::load(v, sm, twr, t, rl, x, ADJ ? s_edge : 1.f, ADJ ? s_int : 1.f, ADJ ? 1.f : out_scale);
         TM::template passes<0>(v, sm, tw, t, rl);
         TM::sync(rl);
         TM::for_each_out(v, t, [&](int i, float2 z) {   // windowed frame: samples 2i, 2i+1 at sm[i]
