@@ -58,22 +58,26 @@ constexpr int mixedThreads(int n, const int* radix, int passes) {
     for (int p = 0; p < passes; ++p) rmax = radix[p] > rmax ? radix[p] : rmax;
     const int least = (n + rmax - 1) / rmax;
     const int lo = least < 512 ? least : 257, hi = 2 * least < 512 ? 2 * least : 512;
-    int best = least < 512 ? least : 512;
-    long long bestCost = -1;
-    for (int p = -1; p < passes; ++p)
-        for (int rounds = 1; rounds <= 48; ++rounds) {
-            const int nb = p < 0 ? 0 : n / radix[p];
-            const int T = p < 0 ? best : (nb + rounds - 1) / rounds;
-            if (p < 0 ? rounds > 1 : (T < lo || T > hi)) continue;
-            long long slots = 0;
-            for (int q = 0; q < passes; ++q) slots += (long long)((n / radix[q] + T - 1) / T) * radix[q];
-            const int cta = mixedRows(T) * T;
-            const long long cost = slots * T * ((cta + 31) / 32 * 32) / cta;
-            if (bestCost < 0 || cost < bestCost || (cost == bestCost && T < best)) {
-                bestCost = cost;
-                best = T;
-            }
+    int best = 0;
+    long long bestCost = 0;
+    auto consider = [&](int T) {
+        long long slots = 0;
+        for (int q = 0; q < passes; ++q) slots += (long long)((n / radix[q] + T - 1) / T) * radix[q];
+        const int cta = mixedRows(T) * T;
+        const long long cost = slots * T * ((cta + 31) / 32 * 32) / cta;
+        if (!best || cost < bestCost || (cost == bestCost && T < best)) {
+            bestCost = cost;
+            best = T;
         }
+    };
+    consider(least < 512 ? least : 512);
+    for (int p = 0; p < passes; ++p) {
+        const int nb = n / radix[p];
+        for (int rounds = (nb + hi - 1) / hi; rounds <= (nb + lo - 1) / lo; ++rounds) {
+            const int T = (nb + rounds - 1) / rounds;
+            if (T >= lo && T <= hi) consider(T);
+        }
+    }
     return best;
 }
 
@@ -449,7 +453,7 @@ __global__ void __maxnreg__(ROWS::kRegs) k_istft_mixed(const float2* __restrict_
     const int M = a.n;
     IstftSegment seg;
     seg.init(2 * M, hop, frames, Q, segs, start, outLen, window, out,
-             reinterpret_cast<float*>(smem + (size_t)rows * 2 * len), out_scale);
+             reinterpret_cast<float*>(smem + (size_t)rows * 2 * len));
     const float2* src0 = spec + (uint64_t)(blockIdx.x / segs) * frames * (M + 1);
     float2* buf0 = smem + (size_t)rl * 2 * len;
     float2* buf1 = buf0 + len;
@@ -460,7 +464,7 @@ __global__ void __maxnreg__(ROWS::kRegs) k_istft_mixed(const float2* __restrict_
         __syncthreads();   // the previous wave is done with the row buffers and the carry
         // rows past R (a CTA's partial first or last wave) transform frame f0 again, unread
         const float2* src = src0 + (uint64_t)(f0 + (rl < R ? rl : 0)) * (M + 1);
-        mixed_unsplit(src, buf1, twr, M, t, T, 1.f, 1.f, 1.f);
+        mixed_unsplit(src, buf1, twr, M, t, T, 1.f, 1.f, out_scale);
         __syncthreads();
         ROWS::template run<true, false, false>(a, nullptr, nullptr, buf0, buf1, tw, true, t, T, 1.f);
         __syncthreads();
