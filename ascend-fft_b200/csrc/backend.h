@@ -216,13 +216,11 @@ int launchIstftMixed(const void* spec, void* out, const MixedRadix& half, uint64
 // or null for none), R2C of each frame into out[s][f][n/2+1].  n a power of two in
 // [kStftMinN, kStftMaxN]; twr = W_n^k, k <= n/2.
 constexpr uint32_t kStftMinN = 64, kStftMaxN = 8192;
-// Values a thread holds of a frame's n/2-point transform; tw below is the Stockham table of
-// (n/2, that).  Inverse frames (launchIstft, launchStftAdjoint) take 32 at 512 and 1024 points: two
-// passes and one exchange instead of three and two (60008 frames of 1024: 70.2 -> 59.1 us).
-// Forward frames (launchStft, launchIstftAdjoint) wait for their samples more than for their
-// passes and keep the higher occupancy.
-constexpr int kStftE = 16;
-constexpr int istftE(uint32_t half) { return half == 512 || half == 1024 ? 32 : 16; }
+// Values a thread holds of a frame's n/2-point transform: 32 at 512 and 1024 points, which then take
+// two passes and one exchange instead of three and two (us, 16 and 32: launchStft, 65540 frames of
+// 1024 90.9 / 82.7, 32772 of 2048 97.7 / 84.0; launchIstft, 60008 frames of 1024 70.2 / 59.1).  tw below is
+// the Stockham table (n/2, stftE(n/2)) in all four.
+constexpr int stftE(uint32_t half) { return half == 512 || half == 1024 ? 32 : 16; }
 bool hasStft(uint32_t n);
 int launchStft(const void* sig, void* out, uint32_t n, uint64_t signals, uint32_t framesPerSignal,
                uint64_t sigLen, uint64_t sigStride, uint32_t hop, bool center, const void* window,

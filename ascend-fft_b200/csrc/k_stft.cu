@@ -196,8 +196,8 @@ template <int N, bool ADJ = false>
 int launchStftN(const float* sig, void* out, uint64_t rows, uint32_t framesPerSignal, uint64_t sigLen,
                 uint64_t sigStride, uint32_t hop, bool center, const float* window, const void* tw,
                 const void* twr, void* stream, int64_t gStart = 0, float sEdge = 1.f, float sInt = 1.f) {
-    constexpr int M = N / 2, E = kStftE, T = M / E;
-    constexpr int CTA = T < 256 ? 256 : T;
+    constexpr int M = N / 2, E = stftE(M), T = M / E;
+    constexpr int CTA = T < 4096 / E ? 4096 / E : T;   // at least 4096 values
     constexpr int ROWS = CTA / T;
     constexpr int SMEM = ROWS * dev::smem_stride<M, E, false>() * 8;
     auto* fn = dev::k_stft<N, E, ROWS, ADJ>;
@@ -214,7 +214,7 @@ int launchStftN(const float* sig, void* out, uint64_t rows, uint32_t framesPerSi
 template <int N, bool ADJ = false>
 int launchIstftN(const float2* spec, float* out, uint64_t signals, uint32_t frames, uint32_t hop, int64_t start,
                  uint64_t outLen, const float* window, const void* tw, const void* twr, float scale, void* stream) {
-    constexpr int M = N / 2, E = istftE(M), T = M / E;
+    constexpr int M = N / 2, E = stftE(M), T = M / E;
     constexpr int CTA = T < 4096 / E ? 4096 / E : T;   // at least 4096 values
     constexpr int ROWS = CTA / T;
     constexpr int ROWBYTES = ROWS * dev::istft_row_stride<M, E>() * 8;

@@ -854,9 +854,9 @@ int Plan::execStft(const void* dSig, void* dOut, uint32_t n, uint64_t signals, u
             return -5;
         return 0;
     }
-    if (prepareC2C(n / 2, backend::kStftE) || prepareReal(n)) return -2;
+    if (prepareC2C(n / 2, backend::stftE(n / 2)) || prepareReal(n)) return -2;
     if (backend::launchStft(dSig, dOut, n, signals, (uint32_t)frames, sigLen, sigLen, hop, center, dWindow,
-                            impl_->twC2C[{n / 2, backend::kStftE}], impl_->twReal[n], stream))
+                            impl_->twC2C[{n / 2, backend::stftE(n / 2)}], impl_->twReal[n], stream))
         return -5;
     return 0;
 }
@@ -868,9 +868,9 @@ int Plan::execStftBackward(const void* dGradSpec, void* dGradSig, uint32_t n, ui
     if (center ? sigLen < (uint64_t)n + 2 : sigLen < n) return -8;
     const uint64_t frames = center ? 1 + sigLen / hop : 1 + (sigLen - n) / hop;
     if (frames > 0xFFFFFFFFull || signals > 0xFFFFFFFFull / frames) return -8;
-    if (prepareC2C(n / 2, backend::istftE(n / 2)) || prepareReal(n)) return -2;
+    if (prepareC2C(n / 2, backend::stftE(n / 2)) || prepareReal(n)) return -2;
     if (backend::launchStftAdjoint(dGradSpec, dGradSig, n, signals, (uint32_t)frames, hop, center, sigLen, dWindow,
-                                   impl_->twC2C[{n / 2, backend::istftE(n / 2)}], impl_->twReal[n], stream))
+                                   impl_->twC2C[{n / 2, backend::stftE(n / 2)}], impl_->twReal[n], stream))
         return -5;
     return 0;
 }
@@ -883,9 +883,9 @@ int Plan::execIstftBackward(const void* dGradOut, void* dGradSpec, uint32_t n, u
         return -8;
     if (signals > 0xFFFFFFFFull / frames || outLen == 0 || outLen > (1ull << 62)) return -8;
     if (reinterpret_cast<uintptr_t>(dWindow) & 7u) return -8;
-    if (prepareC2C(n / 2, backend::kStftE) || prepareReal(n)) return -2;
+    if (prepareC2C(n / 2, backend::stftE(n / 2)) || prepareReal(n)) return -2;
     if (backend::launchIstftAdjoint(dGradOut, dGradSpec, n, signals, frames, hop, center ? (int64_t)(n / 2) : 0,
-                                    outLen, dWindow, impl_->twC2C[{n / 2, backend::kStftE}], impl_->twReal[n], scale, stream))
+                                    outLen, dWindow, impl_->twC2C[{n / 2, backend::stftE(n / 2)}], impl_->twReal[n], scale, stream))
         return -5;
     return 0;
 }
@@ -906,9 +906,9 @@ int Plan::execIstft(const void* dSpec, void* dOut, uint32_t n, uint64_t signals,
             return -5;
         return 0;
     }
-    if (prepareC2C(n / 2, backend::istftE(n / 2)) || prepareReal(n)) return -2;
+    if (prepareC2C(n / 2, backend::stftE(n / 2)) || prepareReal(n)) return -2;
     if (backend::launchIstft(dSpec, dOut, n, signals, frames, hop, center ? (int64_t)(n / 2) : 0, outLen, dWindow,
-                             impl_->twC2C[{n / 2, backend::istftE(n / 2)}], impl_->twReal[n], scale, stream))
+                             impl_->twC2C[{n / 2, backend::stftE(n / 2)}], impl_->twReal[n], scale, stream))
         return -5;
     return 0;
 }
