@@ -3,8 +3,8 @@
 //   frame f of signal s:  y[j] = w[j] * x_s[f*hop + j - (center ? N/2 : 0)],  j < N,
 //   positions outside [0, L) reflected (x[-i] = x[i], x[L-1+i] = x[L-1-i]) as torch.stft's
 //   default pad_mode="reflect";  out[s][f][k] = sum_j y[j] exp(-2*pi*i*j*k/N), k <= N/2.
-// Frames overlap, so samples are read through the read-only cache (L1/L2 reuse across the
-// N/hop frames that cover them) instead of the streaming path of the batched transforms.
+// Frames overlap, so samples are read through L1 (ld_reused: reuse across the N/hop frames that
+// cover them) instead of the streaming path of the batched transforms.
 // The reference runs its STFT cases as a dense-frame R2C proxy (docs/testing.md:118,
 // config/test_matrix.json "stft": R2C with batch = frames); framing, windowing and overlap
 // are done here inside the transform.
@@ -53,7 +53,7 @@ k_stft(const float* __restrict__ sig, float2* __restrict__ out, const float2* __
         for (int r = threadIdx.x; r < (int)hop; r += blockDim.x) {
             float e = 0.f;
             for (int j = r; j < N; j += (int)hop) {
-                const float w = window ? __ldg(window + j) : 1.f;
+                const float w = window ? ld_reused(window + j) : 1.f;
                 e += w * w;
             }
             rinv[r] = e > 0.f ? 1.f / e : 0.f;
@@ -67,7 +67,7 @@ k_stft(const float* __restrict__ sig, float2* __restrict__ out, const float2* __
         for (int64_t g = fh - K + 1 > 0 ? fh - K + 1 : 0; g <= fh && g < (int64_t)framesPerSignal; ++g) {
             const int64_t j = p - g * hop;
             if (j < N) {
-                const float w = window ? __ldg(window + j) : 1.f;
+                const float w = window ? ld_reused(window + j) : 1.f;
                 e += w * w;
             }
         }
@@ -76,11 +76,11 @@ k_stft(const float* __restrict__ sig, float2* __restrict__ out, const float2* __
     auto sample = [&](int64_t i) {
         if constexpr (ADJ) {
             const int64_t k = i - gStart;
-            return k >= 0 && k < sigLen ? __ldg(x + k) * inv(i) : 0.f;
+            return k >= 0 && k < sigLen ? ld_reused(x + k) * inv(i) : 0.f;
         } else {
             i = i < 0 ? -i : i;
             i = i >= sigLen ? 2 * (sigLen - 1) - i : i;
-            return __ldg(x + i);
+            return ld_reused(x + i);
         }
     };
     // Interior frames starting on an 8-byte boundary (every frame of an even hop away from the
@@ -95,7 +95,7 @@ k_stft(const float* __restrict__ sig, float2* __restrict__ out, const float2* __
     // on memory per issue).
     float2 v[E];
     if (direct) {
-        TM::load_first(v, t, [&](int m) { return __ldg(xv + m); });
+        TM::load_first(v, t, [&](int m) { return ld_reused(xv + m); });
         if constexpr (ADJ) {   // start even, hop even: i mod hop and i mod hop + 1 are one pair
             const uint32_t i0 = (uint32_t)(start % hop);
             TM::for_each_in(v, t, [&](int m, float2& z) {
@@ -109,7 +109,7 @@ k_stft(const float* __restrict__ sig, float2* __restrict__ out, const float2* __
     }
     if (window) {
         float2 w[E];
-        TM::load_first(w, t, [&](int m) { return __ldg(reinterpret_cast<const float2*>(window) + m); });
+        TM::load_first(w, t, [&](int m) { return ld_reused(reinterpret_cast<const float2*>(window) + m); });
 #pragma unroll
         for (int i = 0; i < E; ++i) v[i] = __fmul2_rn(v[i], w[i]);
     }
@@ -172,7 +172,7 @@ k_istft(const float2* __restrict__ spec, float* __restrict__ out, const float2* 
         TM::template passes<0>(v, sm, tw, t, rl);
         TM::sync(rl);
         TM::for_each_out(v, t, [&](int i, float2 z) {   // windowed frame: samples 2i, 2i+1 at sm[i]
-            const float2 w = window ? __ldg(reinterpret_cast<const float2*>(window) + i) : make_float2(1.f, 1.f);
+            const float2 w = window ? ld_reused(reinterpret_cast<const float2*>(window) + i) : make_float2(1.f, 1.f);
             sm[i] = make_float2(z.x * w.x, z.y * w.y);
         });
         __syncthreads();

@@ -406,7 +406,7 @@ __global__ void __maxnreg__(ROWS::kRegs) k_stft_mixed(const float* __restrict__ 
         auto sample = [&](int64_t i) {
             i = i < 0 ? -i : i;
             i = i >= sigLen ? 2 * (sigLen - 1) - i : i;
-            return __ldg(x + i);
+            return ld_reused(x + i);
         };
         // interior frames starting on an 8-byte boundary read one float2 per complex value; the
         // others sample with reflection
@@ -414,9 +414,9 @@ __global__ void __maxnreg__(ROWS::kRegs) k_stft_mixed(const float* __restrict__ 
         const float2* xv = reinterpret_cast<const float2*>(x + (direct ? start : 0));
         const float2* wv = reinterpret_cast<const float2*>(window);
         for (int m = t; m < M; m += T) {
-            float2 z = direct ? __ldg(xv + m) : make_float2(sample(start + 2 * m), sample(start + 2 * m + 1));
+            float2 z = direct ? ld_reused(xv + m) : make_float2(sample(start + 2 * m), sample(start + 2 * m + 1));
             if (window) {
-                const float2 w = __ldg(wv + m);
+                const float2 w = ld_reused(wv + m);
                 z = make_float2(z.x * w.x, z.y * w.y);
             }
             buf1[m] = z;
@@ -470,10 +470,10 @@ __global__ void __maxnreg__(ROWS::kRegs) k_istft_mixed(const float2* __restrict_
         __syncthreads();
         seg.wave<VEC, 0>(
             f0, R, reinterpret_cast<const float*>(smem) + finOff * 2, 4 * len,
-            [&](const float* p, int j) { return (window ? __ldg(window + j) : 1.f) * *p; },
+            [&](const float* p, int j) { return (window ? ld_reused(window + j) : 1.f) * *p; },
             [&](const float* p, int j) {
                 const float4 x = *reinterpret_cast<const float4*>(p);
-                const float4 w = window ? __ldg(reinterpret_cast<const float4*>(window + j)) : make_float4(1.f, 1.f, 1.f, 1.f);
+                const float4 w = window ? ld_reused(reinterpret_cast<const float4*>(window + j)) : make_float4(1.f, 1.f, 1.f, 1.f);
                 return make_float4(w.x * x.x, w.y * x.y, w.z * x.z, w.w * x.w);
             });
     }
