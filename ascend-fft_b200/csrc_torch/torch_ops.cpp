@@ -345,9 +345,10 @@ struct C2R2DNode : Function<C2R2DNode> {
     }
 };
 
+// `w` is optional: apply() asks every plain Tensor argument for its device, an undefined one included.
 struct StftNode : Function<StftNode> {
-    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& window, int64_t n, int64_t hop,
-                          bool center) {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Maybe& w, int64_t n, int64_t hop, bool center) {
+        const Tensor window = w.value_or(Tensor());
         ctx->saved_data["n"] = n;
         ctx->saved_data["hop"] = hop;
         ctx->saved_data["center"] = center;
@@ -370,8 +371,9 @@ struct StftNode : Function<StftNode> {
 };
 
 struct IstftNode : Function<IstftNode> {
-    static Tensor forward(AutogradContext* ctx, const Tensor& spec, const Tensor& window, int64_t n, int64_t hop,
-                          bool center, int64_t outLen, double scale) {
+    static Tensor forward(AutogradContext* ctx, const Tensor& spec, const Maybe& w, int64_t n, int64_t hop, bool center,
+                          int64_t outLen, double scale) {
+        const Tensor window = w.value_or(Tensor());
         ctx->saved_data["n"] = n;
         ctx->saved_data["hop"] = hop;
         ctx->saved_data["center"] = center;
@@ -448,7 +450,7 @@ Maybe stft(const Tensor& x, int64_t n, int64_t hop, bool center, const Maybe& w)
         !oneKernelFrames(n) || x.size(1) < (center ? n + 2 : n) || x.size(0) < 1 ||
         (window.defined() && !takes(window, at::kFloat)))
         return std::nullopt;
-    return wantsGrad(x) || (window.defined() && wantsGrad(window)) ? StftNode::apply(x, window, n, hop, center)
+    return wantsGrad(x) || (window.defined() && wantsGrad(window)) ? StftNode::apply(x, w, n, hop, center)
                                                                    : execStft(x, n, hop, center, window);
 }
 
@@ -459,7 +461,7 @@ Maybe istft(const Tensor& spec, int64_t n, int64_t hop, bool center, const Maybe
         !oneKernelFrames(n) || (window.defined() && !takes(window, at::kFloat)))
         return std::nullopt;
     return wantsGrad(spec) || (window.defined() && wantsGrad(window))
-               ? IstftNode::apply(spec, window, n, hop, center, outLen, scale)
+               ? IstftNode::apply(spec, w, n, hop, center, outLen, scale)
                : execIstft(spec, n, hop, center, window, outLen, scale);
 }
 
