@@ -157,9 +157,15 @@ def _need_cuda(t: torch.Tensor, dtype: torch.dtype, what: str):
         raise TypeError(f"{what}: expected {dtype}, got {t.dtype}")
 
 
+def _dense(t: torch.Tensor) -> torch.Tensor:
+    """`t` in contiguous memory that holds the values themselves: contiguous() alone returns a
+    conjugate or negative view as it is, with the memory of the tensor it is a view of."""
+    return t.resolve_conj().resolve_neg().contiguous()
+
+
 def c2c(x: torch.Tensor, direction: int, scale: float, out: torch.Tensor | None = None) -> torch.Tensor:
     _need_cuda(x, torch.complex64, "c2c")
-    x = x.contiguous()
+    x = _dense(x)
     n = x.shape[-1]
     batch = x.numel() // n if n else 0
     y = out if out is not None else torch.empty_like(x)
@@ -173,7 +179,7 @@ def c2c(x: torch.Tensor, direction: int, scale: float, out: torch.Tensor | None 
 
 def r2c(x: torch.Tensor, s_edge: float = 1.0, s_int: float = 1.0) -> torch.Tensor:
     _need_cuda(x, torch.float32, "r2c")
-    x = x.contiguous()
+    x = _dense(x)
     n = x.shape[-1]
     batch = x.numel() // n if n else 0
     y = torch.empty(*x.shape[:-1], n // 2 + 1, dtype=torch.complex64, device=x.device)
@@ -188,7 +194,7 @@ def r2c(x: torch.Tensor, s_edge: float = 1.0, s_int: float = 1.0) -> torch.Tenso
 def c2r(X: torch.Tensor, n: int, s_edge: float = 1.0, s_int: float = 1.0,
         out_scale: float | None = None) -> torch.Tensor:
     _need_cuda(X, torch.complex64, "c2r")
-    X = X.contiguous()
+    X = _dense(X)
     if X.shape[-1] != n // 2 + 1:
         raise ValueError(f"c2r: last dimension {X.shape[-1]} != n/2+1 = {n // 2 + 1}")
     batch = X.numel() // X.shape[-1] if X.shape[-1] else 0
@@ -220,7 +226,7 @@ def c2c_axis(x: torch.Tensor, dim: int, direction: int, scale: float) -> torch.T
     dim = dim % x.dim()
     if dim == x.dim() - 1:
         return c2c(x, direction, scale)
-    x = x.contiguous()
+    x = _dense(x)
     n = x.shape[dim]
     outer, inner = _outer_inner(x.shape, dim)
     y = torch.empty_like(x)
@@ -237,7 +243,7 @@ def c2c_2d(x: torch.Tensor, direction: int, scale: float) -> torch.Tensor:
     """2-D C2C over the last two dimensions of a complex64 CUDA tensor."""
     _need_cuda(x, torch.complex64, "c2c_2d")
     _need_2d(x, "c2c_2d")
-    x = x.contiguous()
+    x = _dense(x)
     ny, nx = x.shape[-2], x.shape[-1]
     batch = x.numel() // (ny * nx) if ny * nx else 0
     y = torch.empty_like(x)
@@ -280,7 +286,7 @@ class _FFT(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        return c2c(g.contiguous(), -ctx.direction, ctx.scale), None, None
+        return c2c(g, -ctx.direction, ctx.scale), None, None
 
 
 class _RFFT(torch.autograd.Function):
@@ -291,7 +297,7 @@ class _RFFT(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        return c2r(g.contiguous(), ctx.n, 1.0, 0.5, ctx.scale), None
+        return c2r(g, ctx.n, 1.0, 0.5, ctx.scale), None
 
 
 class _IRFFT(torch.autograd.Function):
@@ -303,13 +309,13 @@ class _IRFFT(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         c = ctx.scale
-        return r2c(g.contiguous(), c, 2.0 * c), None, None
+        return r2c(g, c, 2.0 * c), None, None
 
 
 def c2c_tensor(x: torch.Tensor, direction: int = -1, scale: float = 1.0, split_terms: int = 3) -> torch.Tensor:
     """Split-BF16 tensor-core C2C (n a power of two in 64..4096) on torch's current stream."""
     _need_cuda(x, torch.complex64, "c2c_tensor")
-    x = x.contiguous()
+    x = _dense(x)
     n = x.shape[-1]
     batch = x.numel() // n if n else 0
     y = torch.empty_like(x)
@@ -349,6 +355,7 @@ class _STFT(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, n, hop, center, window):
+        x = _dense(x)
         signals, length = x.shape
         frames = (1 + length // hop) if center else (1 + (length - n) // hop)
         y = torch.empty(signals, frames, n // 2 + 1, dtype=torch.complex64, device=x.device)
@@ -370,16 +377,17 @@ class _STFT(torch.autograd.Function):
         if _pow2(n) and (length >= n + 2 if ctx.center else length >= n):
             # one kernel: each frame's weighted C2R, the window, the overlap-add and the fold of
             # the reflect padding
+            g = _dense(g)
             gx = torch.empty(signals, length, dtype=torch.float32, device=g.device)
             rc = plan_for(g.device, n, "real").exec_stft_backward(
-                g.contiguous().data_ptr(), gx.data_ptr(), n, signals, length, hop, ctx.center,
+                g.data_ptr(), gx.data_ptr(), n, signals, length, hop, ctx.center,
                 window.data_ptr() if window is not None else 0, _stream(g))
             if rc:
                 raise BflyError(f"exec_stft_backward(n={n}, signals={signals}, length={length}, hop={hop})", rc)
             return gx, None, None, None, None
         # other lengths: the adjoint of each frame's one-sided transform (the weighted C2R of
         # rfft's backward), then the window, overlap-add and reflect fold
-        fr = c2r(g.contiguous().reshape(signals * frames, n // 2 + 1), n, 1.0, 0.5, 1.0)
+        fr = c2r(g.reshape(signals * frames, n // 2 + 1), n, 1.0, 0.5, 1.0)
         fr = fr.reshape(signals, frames, n)
         if window is not None:
             fr = fr * window
@@ -411,7 +419,7 @@ def stft(x: torch.Tensor, n_fft: int, hop_length: int | None = None, win_length:
     if normalized:
         window = (window if window is not None else torch.ones(n_fft, device=x.device)) * n_fft ** -0.5
     flat = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
-    flat = flat.contiguous()
+    flat = _dense(flat)
     y = _native.stft(flat, n_fft, hop, bool(center), window)
     if y is None:
         y = _STFT.apply(flat, n_fft, hop, center, window)
@@ -428,6 +436,7 @@ class _ISTFT(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, spec, n, hop, center, window, out_len, scale):
+        spec = _dense(spec)
         signals, frames = spec.shape[0], spec.shape[1]
         y = torch.empty(signals, out_len, dtype=torch.float32, device=spec.device)
         rc = plan_for(spec.device, n, "real").exec_istft(
@@ -445,9 +454,10 @@ class _ISTFT(torch.autograd.Function):
         n, hop, frames = ctx.n, ctx.hop, ctx.frames
         if _pow2(n):
             # one kernel: the frames of g / envelope, windowed, transformed and weighted
+            g = _dense(g)
             gs = torch.empty(g.shape[0], frames, n // 2 + 1, dtype=torch.complex64, device=g.device)
             rc = plan_for(g.device, n, "real").exec_istft_backward(
-                g.contiguous().data_ptr(), gs.data_ptr(), n, g.shape[0], frames, hop, ctx.center,
+                g.data_ptr(), gs.data_ptr(), n, g.shape[0], frames, hop, ctx.center,
                 window.data_ptr() if window is not None else 0, g.shape[1], ctx.scale, _stream(g))
             if rc:
                 raise BflyError(f"exec_istft_backward(n={n}, frames={frames}, hop={hop})", rc)
@@ -496,7 +506,7 @@ def _pad_window(window, win_length, n_fft, what, device):
     if wl < n_fft:
         left = (n_fft - wl) // 2
         window = torch.nn.functional.pad(window, (left, n_fft - wl - left))
-    return window.contiguous()
+    return _dense(window)
 
 
 def istft(X: torch.Tensor, n_fft: int, hop_length: int | None = None, win_length: int | None = None,
@@ -536,7 +546,7 @@ def istft(X: torch.Tensor, n_fft: int, hop_length: int | None = None, win_length
             _envelope_checked.clear()
         _envelope_checked[key] = True
     lead = X.shape[:-2]
-    spec = (X if X.dim() == 3 else X.reshape(-1, X.shape[-2], frames)).transpose(-1, -2).contiguous()
+    spec = _dense((X if X.dim() == 3 else X.reshape(-1, X.shape[-2], frames)).transpose(-1, -2))
     scale = n_fft ** 0.5 if normalized else 1.0
     y = _native.istft(spec, n_fft, hop, bool(center), window, out_len, scale)
     if y is None:
@@ -550,7 +560,7 @@ class _RFFT2(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, scale):
         _need_cuda(x, torch.float32, "rfft2")
-        x = x.contiguous()
+        x = _dense(x)
         ny, nx = x.shape[-2], x.shape[-1]
         batch = x.numel() // (ny * nx) if ny * nx else 0
         y = torch.empty(*x.shape[:-1], nx // 2 + 1, dtype=torch.complex64, device=x.device)
@@ -564,7 +574,7 @@ class _RFFT2(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        gc = c2c_axis(g.contiguous(), -2, 1, 1.0)
+        gc = c2c_axis(g, -2, 1, 1.0)
         return c2r(gc, ctx.nx, 1.0, 0.5, ctx.scale), None
 
 
@@ -574,7 +584,7 @@ class _IRFFT2(torch.autograd.Function):
     @staticmethod
     def forward(ctx, X, nx, scale):
         _need_cuda(X, torch.complex64, "irfft2")
-        X = X.contiguous()
+        X = _dense(X)
         ny = X.shape[-2]
         if X.shape[-1] != nx // 2 + 1:
             raise ValueError(f"irfft2: last dimension {X.shape[-1]} != nx/2+1 = {nx // 2 + 1}")
@@ -591,7 +601,7 @@ class _IRFFT2(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         c = ctx.scale
-        return c2c_axis(r2c(g.contiguous(), c, 2.0 * c), -2, -1, 1.0), None, None
+        return c2c_axis(r2c(g, c, 2.0 * c), -2, -1, 1.0), None, None
 
 
 def _need_2d(x: torch.Tensor, what: str):
