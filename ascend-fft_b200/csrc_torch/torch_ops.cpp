@@ -10,7 +10,7 @@
 // at kMaxPlans entries.  Nodes hold no plan: a backward pass looks its own up.
 #include <torch/extension.h>
 
-#include <ATen/FuncTorchTLS.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -131,9 +131,11 @@ bool takes(const Tensor& x, at::ScalarType type) {
 }
 // Contiguous memory that holds the values themselves (a conjugate view's does not).
 Tensor dense(const Tensor& x) { return x.resolve_conj().resolve_neg().contiguous(); }
+// No functorch transform around the call (its front key is included while one is active; the
+// thread's functorch state itself outlives the first of them), no tracing, no dispatch mode.
 bool plainMode() {
-    const auto& functorch = at::functorch::functorchTLSAccessor();
-    return !functorch && !torch::jit::tracer::isTracing() && !c10::impl::dispatch_mode_enabled();
+    return !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) &&
+           !torch::jit::tracer::isTracing() && !c10::impl::dispatch_mode_enabled();
 }
 bool wantsGrad(const Tensor& x) { return at::GradMode::is_enabled() && x.requires_grad(); }
 void* streamOf(const Tensor& x) { return c10::cuda::getCurrentCUDAStream(x.get_device()).stream(); }
