@@ -127,6 +127,10 @@ def _find_plan(device: int, real: int, n: int):
 
 _native.bind(_find_plan, BflyError)
 
+# The module returns plain tensors and runs no torch operation that __torch_function__ could see, so
+# subclasses go to the Functions.
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
 
 def _stream(t: torch.Tensor) -> int:
     return torch._C._cuda_getCurrentRawStream(t.get_device())   # 0.1 us; building a Stream object 2.4
@@ -329,7 +333,7 @@ def c2c_tensor(x: torch.Tensor, direction: int = -1, scale: float = 1.0, split_t
 
 
 def fft(x: torch.Tensor, norm: str | None = None, dim: int = -1) -> torch.Tensor:
-    y = _native.fft(x, dim, -1, _norm_code(norm))
+    y = _native.fft(x, dim, -1, _norm_code(norm)) if type(x) in _PLAIN else None
     if y is not None:
         return y
     if dim % max(x.dim(), 1) != x.dim() - 1:
@@ -338,7 +342,7 @@ def fft(x: torch.Tensor, norm: str | None = None, dim: int = -1) -> torch.Tensor
 
 
 def ifft(x: torch.Tensor, norm: str | None = None, dim: int = -1) -> torch.Tensor:
-    y = _native.fft(x, dim, 1, _norm_code(norm))
+    y = _native.fft(x, dim, 1, _norm_code(norm)) if type(x) in _PLAIN else None
     if y is not None:
         return y
     if dim % max(x.dim(), 1) != x.dim() - 1:
@@ -420,7 +424,8 @@ def stft(x: torch.Tensor, n_fft: int, hop_length: int | None = None, win_length:
         window = (window if window is not None else torch.ones(n_fft, device=x.device)) * n_fft ** -0.5
     flat = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
     flat = _dense(flat)
-    y = _native.stft(flat, n_fft, hop, bool(center), window)
+    plain = type(flat) in _PLAIN and (window is None or type(window) in _PLAIN)
+    y = _native.stft(flat, n_fft, hop, bool(center), window) if plain else None
     if y is None:
         y = _STFT.apply(flat, n_fft, hop, center, window)
     if x.dim() != 2:
@@ -548,7 +553,8 @@ def istft(X: torch.Tensor, n_fft: int, hop_length: int | None = None, win_length
     lead = X.shape[:-2]
     spec = _dense((X if X.dim() == 3 else X.reshape(-1, X.shape[-2], frames)).transpose(-1, -2))
     scale = n_fft ** 0.5 if normalized else 1.0
-    y = _native.istft(spec, n_fft, hop, bool(center), window, out_len, scale)
+    plain = type(spec) in _PLAIN and (window is None or type(window) in _PLAIN)
+    y = _native.istft(spec, n_fft, hop, bool(center), window, out_len, scale) if plain else None
     if y is None:
         y = _ISTFT.apply(spec, n_fft, hop, center, window, out_len, scale)
     return y if X.dim() == 3 else y.reshape(*lead, out_len)
@@ -611,7 +617,7 @@ def _need_2d(x: torch.Tensor, what: str):
 
 def fft2(x: torch.Tensor, norm: str | None = None) -> torch.Tensor:
     """2-D FFT over the last two dimensions (torch.fft.fft2 with dim=(-2, -1))."""
-    y = _native.fft2(x, -1, _norm_code(norm))
+    y = _native.fft2(x, -1, _norm_code(norm)) if type(x) in _PLAIN else None
     if y is not None:
         return y
     _need_2d(x, "fft2")
@@ -619,7 +625,7 @@ def fft2(x: torch.Tensor, norm: str | None = None) -> torch.Tensor:
 
 
 def ifft2(x: torch.Tensor, norm: str | None = None) -> torch.Tensor:
-    y = _native.fft2(x, 1, _norm_code(norm))
+    y = _native.fft2(x, 1, _norm_code(norm)) if type(x) in _PLAIN else None
     if y is not None:
         return y
     _need_2d(x, "ifft2")
@@ -628,7 +634,7 @@ def ifft2(x: torch.Tensor, norm: str | None = None) -> torch.Tensor:
 
 def rfft2(x: torch.Tensor, norm: str | None = None) -> torch.Tensor:
     """torch.fft.rfft2 over the last two dimensions: float32 [..., ny, nx] -> [..., ny, nx/2+1]."""
-    y = _native.rfft2(x, _norm_code(norm))
+    y = _native.rfft2(x, _norm_code(norm)) if type(x) in _PLAIN else None
     if y is not None:
         return y
     _need_2d(x, "rfft2")
@@ -643,19 +649,19 @@ def irfft2(X: torch.Tensor, s: tuple | None = None, norm: str | None = None) -> 
     nx = s[-1] if s is not None else 2 * (X.shape[-1] - 1)
     if s is not None and s[-2] != ny:
         raise ValueError("irfft2: s[-2] must equal X.shape[-2] (no cropping or padding)")
-    y = _native.irfft2(X, nx, _norm_code(norm))
+    y = _native.irfft2(X, nx, _norm_code(norm)) if type(X) in _PLAIN else None
     if y is not None:
         return y
     return _IRFFT2.apply(X, nx, _scale(norm, ny * nx, False))
 
 
 def rfft(x: torch.Tensor, norm: str | None = None) -> torch.Tensor:
-    y = _native.rfft(x, _norm_code(norm))
+    y = _native.rfft(x, _norm_code(norm)) if type(x) in _PLAIN else None
     return y if y is not None else _RFFT.apply(x, _scale(norm, x.shape[-1], True))
 
 
 def irfft(X: torch.Tensor, n: int | None = None, norm: str | None = None) -> torch.Tensor:
     if n is None:
         n = 2 * (X.shape[-1] - 1)
-    y = _native.irfft(X, n, _norm_code(norm))
+    y = _native.irfft(X, n, _norm_code(norm)) if type(X) in _PLAIN else None
     return y if y is not None else _IRFFT.apply(X, n, _scale(norm, n, False))
