@@ -41,7 +41,7 @@ from . import _lib
 from .core import DEFAULT_CANDIDATE, BflyError, Context
 
 _native = _lib.load_torch_ops()
-_NORM = {None: 0, "": 0, "backward": 0, "ortho": 1, "forward": 2}
+_NORM = {"backward": 0, "ortho": 1, "forward": 2}
 
 _lock = threading.Lock()
 _state = {}   # device index -> {"ctx": Context, "plans": {candidate id: Plan}, "tuned": {...}}
@@ -137,7 +137,8 @@ def _stream(t: torch.Tensor) -> int:
 
 
 def _norm_code(norm: str | None) -> int:
-    code = _NORM.get(norm)
+    norm = norm or "backward"
+    code = _NORM.get(norm) if isinstance(norm, str) else None
     if code is None:
         raise ValueError(f"invalid norm {norm!r}")
     return code

@@ -120,10 +120,11 @@ void check(int rc, const std::string& what) {
 }
 
 // ------------------------------------------------------------------ what is taken here
-// A plain CUDA tensor of `type` outside every transform that has to see the call itself.
+// A plain CUDA tensor of `type` outside every transform that has to see the call itself.  Empty ones
+// stay with Python, whose scales divide by the length.
 bool takes(const Tensor& x, at::ScalarType type) {
     if (!x.defined() || !x.is_cuda() || x.scalar_type() != type || x.layout() != at::kStrided ||
-        x.unsafeGetTensorImpl()->key_set().has_any(c10::python_ks) || x._fw_grad(0).defined())
+        x.unsafeGetTensorImpl()->key_set().has_any(c10::python_ks) || !x.numel() || x._fw_grad(0).defined())
         return false;
     for (const int64_t d : x.sizes())
         if (d > INT32_MAX) return false;
