@@ -50,6 +50,7 @@ constexpr size_t kMaxPlans = 4096;
 struct Table {
     std::mutex mu;
     std::unordered_map<uint64_t, Plan> plans;
+    uint64_t forgotten = 0;      // times forgetPlans has emptied it
     PyObject* find = nullptr;    // find(device, real, n) -> (plan object, handle)
     PyObject* error = nullptr;   // bfly.BflyError
 };
@@ -66,11 +67,13 @@ Table& table() {
 
 Plan planFor(int device, bool real, int64_t n) {
     Table& t = table();
+    uint64_t forgotten;
     const uint64_t key = ((uint64_t)device << 33) | ((uint64_t)real << 32) | (uint32_t)n;
     {
         std::lock_guard<std::mutex> lock(t.mu);
         const auto it = t.plans.find(key);
         if (it != t.plans.end()) return it->second;
+        forgotten = t.forgotten;
     }
     Plan p;
     {
@@ -91,6 +94,7 @@ Plan planFor(int device, bool real, int64_t n) {
     std::unordered_map<uint64_t, Plan> old;   // released after the lock: a Held takes the interpreter's
     {
         std::lock_guard<std::mutex> lock(t.mu);
+        if (t.forgotten != forgotten) return p;   // asked for before the table was emptied: not kept
         if (t.plans.size() >= kMaxPlans) old.swap(t.plans);
         t.plans[key] = p;
     }
@@ -101,6 +105,7 @@ void forgetPlans() {
     std::unordered_map<uint64_t, Plan> old;
     std::lock_guard<std::mutex> lock(table().mu);
     old.swap(table().plans);
+    ++table().forgotten;
 }
 
 void bind(py::object find, py::object error) {
