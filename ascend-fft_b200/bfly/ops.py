@@ -21,6 +21,7 @@ hand-written adjoints behind torch.autograd.Function:
     ifft : grad_x = s * FFT(g)
     rfft : grad_x = C2R(g) with bins 0 and n/2 weighted 1 and the others 1/2, times s
     irfft: grad_X = R2C(g) with bins 0 and n/2 weighted c and the others 2c  (c = output scale)
+Gradients can be differentiated in turn (create_graph=True); windows are constants.
 Every call enqueues on torch's current stream; nothing runs on the CPU.
 
 The functions below hand plain calls to csrc_torch/torch_ops.cpp, which launches the same kernels
@@ -261,6 +262,8 @@ def c2c_2d(x: torch.Tensor, direction: int, scale: float) -> torch.Tensor:
     return y
 
 
+# Every transform is linear, so the adjoint of an adjoint is the transform: backward() calls the
+# classes themselves, and a gradient that needs a gradient of its own has one.
 class _FFTAxis(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, dim, direction, scale):
@@ -269,7 +272,7 @@ class _FFTAxis(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        return c2c_axis(g, ctx.dim, -ctx.direction, ctx.scale), None, None, None
+        return _FFTAxis.apply(g, ctx.dim, -ctx.direction, ctx.scale), None, None, None
 
 
 class _FFT2(torch.autograd.Function):
@@ -280,7 +283,7 @@ class _FFT2(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        return c2c_2d(g, -ctx.direction, ctx.scale), None, None
+        return _FFT2.apply(g, -ctx.direction, ctx.scale), None, None
 
 
 class _FFT(torch.autograd.Function):
@@ -291,30 +294,34 @@ class _FFT(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        return c2c(g, -ctx.direction, ctx.scale), None, None
+        return _FFT.apply(g, -ctx.direction, ctx.scale), None, None
 
 
 class _RFFT(torch.autograd.Function):
+    """Bins 0 and n/2 times scale * edge, the others times scale * inside."""
+
     @staticmethod
-    def forward(ctx, x, scale):
-        ctx.scale, ctx.n = scale, x.shape[-1]
-        return r2c(x, scale, scale)   # the scale rides on the kernel's per-bin weights
+    def forward(ctx, x, scale, edge=1.0, inside=1.0):
+        ctx.args = scale, edge, inside
+        ctx.n = x.shape[-1]
+        return r2c(x, scale * edge, scale * inside)   # the scale rides on the kernel's per-bin weights
 
     @staticmethod
     def backward(ctx, g):
-        return c2r(g, ctx.n, 1.0, 0.5, ctx.scale), None
+        scale, edge, inside = ctx.args
+        return _IRFFT.apply(g, ctx.n, scale, edge, 0.5 * inside), None, None, None
 
 
 class _IRFFT(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, X, n, scale):
-        ctx.scale = scale
-        return c2r(X, n, 1.0, 1.0, scale)
+    def forward(ctx, X, n, scale, edge=1.0, inside=1.0):
+        ctx.args = scale, edge, inside
+        return c2r(X, n, edge, inside, scale)
 
     @staticmethod
     def backward(ctx, g):
-        c = ctx.scale
-        return r2c(g, c, 2.0 * c), None, None
+        scale, edge, inside = ctx.args
+        return _RFFT.apply(g, scale, edge, 2.0 * inside), None, None, None, None
 
 
 def c2c_tensor(x: torch.Tensor, direction: int = -1, scale: float = 1.0, split_terms: int = 3) -> torch.Tensor:
@@ -380,22 +387,13 @@ class _STFT(torch.autograd.Function):
         n, hop, length = ctx.n, ctx.hop, ctx.length
         signals, frames = g.shape[0], g.shape[1]
         if _pow2(n) and (length >= n + 2 if ctx.center else length >= n):
-            # one kernel: each frame's weighted C2R, the window, the overlap-add and the fold of
-            # the reflect padding
-            g = _dense(g)
-            gx = torch.empty(signals, length, dtype=torch.float32, device=g.device)
-            rc = plan_for(g.device, n, "real").exec_stft_backward(
-                g.data_ptr(), gx.data_ptr(), n, signals, length, hop, ctx.center,
-                window.data_ptr() if window is not None else 0, _stream(g))
-            if rc:
-                raise BflyError(f"exec_stft_backward(n={n}, signals={signals}, length={length}, hop={hop})", rc)
-            return gx, None, None, None, None
+            return _STFTAdjoint.apply(g, n, hop, ctx.center, window, length), None, None, None, None
         # other lengths: the adjoint of each frame's one-sided transform (the weighted C2R of
         # rfft's backward), then the window, overlap-add and reflect fold
-        fr = c2r(g.reshape(signals * frames, n // 2 + 1), n, 1.0, 0.5, 1.0)
+        fr = _IRFFT.apply(g.reshape(signals * frames, n // 2 + 1), n, 1.0, 1.0, 0.5)
         fr = fr.reshape(signals, frames, n)
         if window is not None:
-            fr = fr * window
+            fr = fr * window.detach()
         pad = n // 2 if ctx.center else 0
         padded = length + 2 * pad
         gp = torch.nn.functional.fold(fr.transpose(1, 2), output_size=(1, padded), kernel_size=(1, n),
@@ -405,6 +403,30 @@ class _STFT(torch.autograd.Function):
             gx[:, 1:pad + 1] += gp[:, :pad].flip(-1)
             gx[:, length - 1 - pad:length - 1] += gp[:, pad + length:].flip(-1)
         return gx, None, None, None, None
+
+
+class _STFTAdjoint(torch.autograd.Function):
+    """_STFT's gradient in one kernel: each frame's weighted C2R, the window, the overlap-add and the
+    fold of the reflect padding."""
+
+    @staticmethod
+    def forward(ctx, g, n, hop, center, window, length):
+        g = _dense(g)
+        signals = g.shape[0]
+        gx = torch.empty(signals, length, dtype=torch.float32, device=g.device)
+        rc = plan_for(g.device, n, "real").exec_stft_backward(
+            g.data_ptr(), gx.data_ptr(), n, signals, length, hop, center,
+            window.data_ptr() if window is not None else 0, _stream(g))
+        if rc:
+            raise BflyError(f"exec_stft_backward(n={n}, signals={signals}, length={length}, hop={hop})", rc)
+        ctx.n, ctx.hop, ctx.center = n, hop, center
+        ctx.save_for_backward(window)
+        return gx
+
+    @staticmethod
+    def backward(ctx, h):
+        (window,) = ctx.saved_tensors
+        return _STFT.apply(h, ctx.n, ctx.hop, ctx.center, window), None, None, None, None, None
 
 
 def stft(x: torch.Tensor, n_fft: int, hop_length: int | None = None, win_length: int | None = None,
@@ -459,15 +481,8 @@ class _ISTFT(torch.autograd.Function):
         (window,) = ctx.saved_tensors
         n, hop, frames = ctx.n, ctx.hop, ctx.frames
         if _pow2(n):
-            # one kernel: the frames of g / envelope, windowed, transformed and weighted
-            g = _dense(g)
-            gs = torch.empty(g.shape[0], frames, n // 2 + 1, dtype=torch.complex64, device=g.device)
-            rc = plan_for(g.device, n, "real").exec_istft_backward(
-                g.data_ptr(), gs.data_ptr(), n, g.shape[0], frames, hop, ctx.center,
-                window.data_ptr() if window is not None else 0, g.shape[1], ctx.scale, _stream(g))
-            if rc:
-                raise BflyError(f"exec_istft_backward(n={n}, frames={frames}, hop={hop})", rc)
-            return gs, None, None, None, None, None, None
+            return _ISTFTAdjoint.apply(g, n, hop, ctx.center, window, frames, ctx.scale), None, None, None, None, None, None
+        window = window.detach() if window is not None else None
         padded = n + hop * (frames - 1)
         start = n // 2 if ctx.center else 0
         env = _envelope(window, n, hop, frames, g.device)
@@ -475,16 +490,34 @@ class _ISTFT(torch.autograd.Function):
         h = torch.zeros(g.shape[0], padded, dtype=torch.float32, device=g.device)
         e = env[start:start + keep]
         h[:, start:start + keep] = torch.where(e > 0, g[:, :keep] / torch.where(e > 0, e, 1.0), 0.0)
-        gs = torch.empty(g.shape[0], frames, n // 2 + 1, dtype=torch.complex64, device=g.device)
-        rc, got = plan_for(g.device, n, "real").exec_stft(
-            h.data_ptr(), gs.data_ptr(), n, g.shape[0], padded, hop, False,
-            window.data_ptr() if window is not None else 0, _stream(g))
-        if rc or got != frames:
-            raise BflyError(f"exec_stft (istft adjoint, n={n}, frames={frames})", rc or -1)
+        gs = _STFT.apply(h, n, hop, False, window)
         c = ctx.scale / n
         wt = torch.full((n // 2 + 1,), 2.0 * c, dtype=torch.float32, device=g.device)
         wt[0] = wt[-1] = c
         return gs * wt, None, None, None, None, None, None
+
+
+class _ISTFTAdjoint(torch.autograd.Function):
+    """_ISTFT's gradient in one kernel: the frames of g / envelope, windowed, transformed and weighted."""
+
+    @staticmethod
+    def forward(ctx, g, n, hop, center, window, frames, scale):
+        g = _dense(g)
+        gs = torch.empty(g.shape[0], frames, n // 2 + 1, dtype=torch.complex64, device=g.device)
+        rc = plan_for(g.device, n, "real").exec_istft_backward(
+            g.data_ptr(), gs.data_ptr(), n, g.shape[0], frames, hop, center,
+            window.data_ptr() if window is not None else 0, g.shape[1], scale, _stream(g))
+        if rc:
+            raise BflyError(f"exec_istft_backward(n={n}, frames={frames}, hop={hop})", rc)
+        ctx.n, ctx.hop, ctx.center, ctx.out_len, ctx.scale = n, hop, center, g.shape[1], scale
+        ctx.save_for_backward(window)
+        return gs
+
+    @staticmethod
+    def backward(ctx, h):
+        (window,) = ctx.saved_tensors
+        return (_ISTFT.apply(h, ctx.n, ctx.hop, ctx.center, window, ctx.out_len, ctx.scale), None, None, None, None, None,
+                None)
 
 
 def _envelope(window, n: int, hop: int, frames: int, device) -> torch.Tensor:
@@ -581,8 +614,7 @@ class _RFFT2(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        gc = c2c_axis(g, -2, 1, 1.0)
-        return c2r(gc, ctx.nx, 1.0, 0.5, ctx.scale), None
+        return _IRFFT.apply(_FFTAxis.apply(g, -2, 1, 1.0), ctx.nx, ctx.scale, 1.0, 0.5), None
 
 
 class _IRFFT2(torch.autograd.Function):
@@ -607,8 +639,7 @@ class _IRFFT2(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
-        c = ctx.scale
-        return c2c_axis(r2c(g, c, 2.0 * c), -2, -1, 1.0), None, None
+        return _FFTAxis.apply(_RFFT.apply(g, ctx.scale, 1.0, 2.0), -2, -1, 1.0), None, None
 
 
 def _need_2d(x: torch.Tensor, what: str):

@@ -281,9 +281,61 @@ Tensor execIstft(const Tensor& spec, int64_t n, int64_t hop, bool center, const 
     return y;
 }
 
+// The gradients of a short-time transform's input: one kernel each.
+Tensor execStftAdjoint(const Tensor& grad, int64_t n, int64_t hop, bool center, const Tensor& window, int64_t length) {
+    const Tensor g = dense(grad);
+    const int64_t signals = g.size(0);
+    Tensor gx = at::empty({signals, length}, g.options().dtype(at::kFloat));
+    const Plan p = planFor(g.get_device(), true, n);
+    check(bfly_plan_exec_stft_backward_async(p->plan, g.data_ptr(), gx.data_ptr(), (uint32_t)n, (uint64_t)signals,
+                                             (uint64_t)length, (uint32_t)hop, center, windowPtr(window), streamOf(g)),
+          frameText("exec_stft_backward", n, "signals", signals, "length", length, hop));
+    return gx;
+}
+
+Tensor execIstftAdjoint(const Tensor& grad, int64_t n, int64_t hop, bool center, const Tensor& window, int64_t frames,
+                        double scale) {
+    const Tensor g = dense(grad);
+    Tensor gs = at::empty({g.size(0), frames, n / 2 + 1}, g.options().dtype(at::kComplexFloat));
+    const Plan p = planFor(g.get_device(), true, n);
+    check(bfly_plan_exec_istft_backward_async(p->plan, g.data_ptr(), gs.data_ptr(), (uint32_t)n, (uint64_t)g.size(0),
+                                              (uint32_t)frames, (uint32_t)hop, center, windowPtr(window),
+                                              (uint64_t)g.size(1), (float)scale, streamOf(g)),
+          "exec_istft_backward(n=" + std::to_string(n) + ", frames=" + std::to_string(frames) + ", hop=" +
+              std::to_string(hop) + ")");
+    return gs;
+}
+
 // ------------------------------------------------------------------ autograd nodes (adjoints as in ops.py)
+// Every transform here is linear, so the adjoint of an adjoint is the transform: a backward pass runs
+// its launches through the same functions as a forward one, and those record a node of their own
+// where the gradient itself needs a gradient.  Windows are constants.
+bool wantsFrames(const Tensor& x, const Maybe& w) { return wantsGrad(x) || (w && wantsGrad(*w)); }
+Tensor c2cAxis(const Tensor& x, int64_t dim, int64_t direction, double scale);
+Tensor c2c2D(const Tensor& x, int64_t direction, double scale);
+// Bins 0 and n/2 times scale * edge, the others times scale * inside.
+Tensor r2c(const Tensor& x, double scale, double edge = 1.0, double inside = 1.0);
+Tensor c2r(const Tensor& x, int64_t n, double scale, double edge = 1.0, double inside = 1.0);
+Tensor stftOf(const Tensor& x, int64_t n, int64_t hop, bool center, const Maybe& w);
+Tensor istftOf(const Tensor& spec, int64_t n, int64_t hop, bool center, const Maybe& w, int64_t outLen, double scale);
+Tensor stftAdjoint(const Tensor& g, int64_t n, int64_t hop, bool center, const Maybe& w, int64_t length);
+Tensor istftAdjoint(const Tensor& g, int64_t n, int64_t hop, bool center, const Maybe& w, int64_t frames, double scale);
+
 int64_t savedInt(AutogradContext* c, const char* k) { return c->saved_data[k].toInt(); }
 double savedDouble(AutogradContext* c, const char* k) { return c->saved_data[k].toDouble(); }
+// What the four nodes of the short-time transforms keep; `size`: the signal's length or the frames.
+void saveFrames(AutogradContext* ctx, const Maybe& w, int64_t n, int64_t hop, bool center, int64_t size, double scale) {
+    ctx->saved_data["n"] = n;
+    ctx->saved_data["hop"] = hop;
+    ctx->saved_data["center"] = center;
+    ctx->saved_data["size"] = size;
+    ctx->saved_data["scale"] = scale;
+    ctx->save_for_backward({w.value_or(Tensor())});
+}
+Maybe savedWindow(AutogradContext* ctx) {
+    const Tensor w = ctx->get_saved_variables()[0];
+    return w.defined() ? Maybe(w) : std::nullopt;
+}
 
 struct C2CNode : Function<C2CNode> {   // dim: the transformed dimension
     static Tensor forward(AutogradContext* ctx, const Tensor& x, int64_t dim, int64_t direction, double scale) {
@@ -293,7 +345,7 @@ struct C2CNode : Function<C2CNode> {   // dim: the transformed dimension
         return execAxis(x, dim, direction, scale);
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-        return {execAxis(g[0], savedInt(ctx, "dim"), -savedInt(ctx, "direction"), savedDouble(ctx, "scale")), Tensor(),
+        return {c2cAxis(g[0], savedInt(ctx, "dim"), -savedInt(ctx, "direction"), savedDouble(ctx, "scale")), Tensor(),
                 Tensor(), Tensor()};
     }
 };
@@ -305,29 +357,35 @@ struct C2C2DNode : Function<C2C2DNode> {
         return exec2D(x, direction, scale);
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-        return {exec2D(g[0], -savedInt(ctx, "direction"), savedDouble(ctx, "scale")), Tensor(), Tensor()};
+        return {c2c2D(g[0], -savedInt(ctx, "direction"), savedDouble(ctx, "scale")), Tensor(), Tensor()};
     }
 };
 
 struct R2CNode : Function<R2CNode> {
-    static Tensor forward(AutogradContext* ctx, const Tensor& x, double scale) {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, double scale, double edge, double inside) {
         ctx->saved_data["scale"] = scale;
+        ctx->saved_data["edge"] = edge;
+        ctx->saved_data["inside"] = inside;
         ctx->saved_data["n"] = x.size(-1);
-        return execR2C(x, scale, scale);
+        return execR2C(x, scale * edge, scale * inside);
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-        return {execC2R(g[0], savedInt(ctx, "n"), 1.0, 0.5, savedDouble(ctx, "scale")), Tensor()};
+        return {c2r(g[0], savedInt(ctx, "n"), savedDouble(ctx, "scale"), savedDouble(ctx, "edge"),
+                    0.5 * savedDouble(ctx, "inside")),
+                Tensor(), Tensor(), Tensor()};
     }
 };
 
 struct C2RNode : Function<C2RNode> {
-    static Tensor forward(AutogradContext* ctx, const Tensor& x, int64_t n, double scale) {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, int64_t n, double scale, double edge, double inside) {
         ctx->saved_data["scale"] = scale;
-        return execC2R(x, n, 1.0, 1.0, scale);
+        ctx->saved_data["edge"] = edge;
+        ctx->saved_data["inside"] = inside;
+        return execC2R(x, n, edge, inside, scale);
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-        const double c = savedDouble(ctx, "scale");
-        return {execR2C(g[0], c, 2.0 * c), Tensor(), Tensor()};
+        return {r2c(g[0], savedDouble(ctx, "scale"), savedDouble(ctx, "edge"), 2.0 * savedDouble(ctx, "inside")),
+                Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
 
@@ -338,7 +396,7 @@ struct R2C2DNode : Function<R2C2DNode> {
         return execR2C2D(x, scale);
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-        return {execC2R(execAxis(g[0], -2, 1, 1.0), savedInt(ctx, "nx"), 1.0, 0.5, savedDouble(ctx, "scale")), Tensor()};
+        return {c2r(c2cAxis(g[0], -2, 1, 1.0), savedInt(ctx, "nx"), savedDouble(ctx, "scale"), 1.0, 0.5), Tensor()};
     }
 };
 
@@ -348,62 +406,89 @@ struct C2R2DNode : Function<C2R2DNode> {
         return execC2R2D(x, nx, scale);
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-        const double c = savedDouble(ctx, "scale");
-        return {execAxis(execR2C(g[0], c, 2.0 * c), -2, -1, 1.0), Tensor(), Tensor()};
+        return {c2cAxis(r2c(g[0], savedDouble(ctx, "scale"), 1.0, 2.0), -2, -1, 1.0), Tensor(), Tensor()};
     }
 };
 
 // `w` is optional: apply() asks every plain Tensor argument for its device, an undefined one included.
 struct StftNode : Function<StftNode> {
     static Tensor forward(AutogradContext* ctx, const Tensor& x, const Maybe& w, int64_t n, int64_t hop, bool center) {
-        const Tensor window = w.value_or(Tensor());
-        ctx->saved_data["n"] = n;
-        ctx->saved_data["hop"] = hop;
-        ctx->saved_data["center"] = center;
-        ctx->saved_data["length"] = x.size(1);
-        ctx->save_for_backward({window});
-        return execStft(x, n, hop, center, window);
+        saveFrames(ctx, w, n, hop, center, x.size(1), 1.0);
+        return execStft(x, n, hop, center, w.value_or(Tensor()));
     }
-    static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
-        const Tensor g = dense(grads[0]), window = ctx->get_saved_variables()[0];
-        const int64_t n = savedInt(ctx, "n"), hop = savedInt(ctx, "hop"), length = savedInt(ctx, "length");
-        const int64_t signals = g.size(0);
-        Tensor gx = at::empty({signals, length}, g.options().dtype(at::kFloat));
-        const Plan p = planFor(g.get_device(), true, n);
-        check(bfly_plan_exec_stft_backward_async(p->plan, g.data_ptr(), gx.data_ptr(), (uint32_t)n, (uint64_t)signals,
-                                                 (uint64_t)length, (uint32_t)hop, ctx->saved_data["center"].toBool(),
-                                                 windowPtr(window), streamOf(g)),
-              frameText("exec_stft_backward", n, "signals", signals, "length", length, hop));
-        return {gx, Tensor(), Tensor(), Tensor(), Tensor()};
+    static variable_list backward(AutogradContext* ctx, const variable_list& g) {
+        return {stftAdjoint(g[0], savedInt(ctx, "n"), savedInt(ctx, "hop"), ctx->saved_data["center"].toBool(),
+                            savedWindow(ctx), savedInt(ctx, "size")),
+                Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+};
+
+struct StftAdjointNode : Function<StftAdjointNode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& g, const Maybe& w, int64_t n, int64_t hop, bool center,
+                          int64_t length) {
+        saveFrames(ctx, w, n, hop, center, length, 1.0);
+        return execStftAdjoint(g, n, hop, center, w.value_or(Tensor()), length);
+    }
+    static variable_list backward(AutogradContext* ctx, const variable_list& h) {
+        return {stftOf(dense(h[0]), savedInt(ctx, "n"), savedInt(ctx, "hop"), ctx->saved_data["center"].toBool(),
+                       savedWindow(ctx)),
+                Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
 
 struct IstftNode : Function<IstftNode> {
     static Tensor forward(AutogradContext* ctx, const Tensor& spec, const Maybe& w, int64_t n, int64_t hop, bool center,
                           int64_t outLen, double scale) {
-        const Tensor window = w.value_or(Tensor());
-        ctx->saved_data["n"] = n;
-        ctx->saved_data["hop"] = hop;
-        ctx->saved_data["center"] = center;
-        ctx->saved_data["scale"] = scale;
-        ctx->saved_data["frames"] = spec.size(1);
-        ctx->save_for_backward({window});
-        return execIstft(spec, n, hop, center, window, outLen, scale);
+        saveFrames(ctx, w, n, hop, center, spec.size(1), scale);
+        return execIstft(spec, n, hop, center, w.value_or(Tensor()), outLen, scale);
     }
-    static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
-        const Tensor g = dense(grads[0]), window = ctx->get_saved_variables()[0];
-        const int64_t n = savedInt(ctx, "n"), hop = savedInt(ctx, "hop"), frames = savedInt(ctx, "frames");
-        Tensor gs = at::empty({g.size(0), frames, n / 2 + 1}, g.options().dtype(at::kComplexFloat));
-        const Plan p = planFor(g.get_device(), true, n);
-        check(bfly_plan_exec_istft_backward_async(p->plan, g.data_ptr(), gs.data_ptr(), (uint32_t)n,
-                                                  (uint64_t)g.size(0), (uint32_t)frames, (uint32_t)hop,
-                                                  ctx->saved_data["center"].toBool(), windowPtr(window),
-                                                  (uint64_t)g.size(1), (float)savedDouble(ctx, "scale"), streamOf(g)),
-              "exec_istft_backward(n=" + std::to_string(n) + ", frames=" + std::to_string(frames) + ", hop=" +
-                  std::to_string(hop) + ")");
-        return {gs, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    static variable_list backward(AutogradContext* ctx, const variable_list& g) {
+        return {istftAdjoint(g[0], savedInt(ctx, "n"), savedInt(ctx, "hop"), ctx->saved_data["center"].toBool(),
+                             savedWindow(ctx), savedInt(ctx, "size"), savedDouble(ctx, "scale")),
+                Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
+
+struct IstftAdjointNode : Function<IstftAdjointNode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& g, const Maybe& w, int64_t n, int64_t hop, bool center,
+                          int64_t frames, double scale) {
+        saveFrames(ctx, w, n, hop, center, g.size(1), scale);
+        return execIstftAdjoint(g, n, hop, center, w.value_or(Tensor()), frames, scale);
+    }
+    static variable_list backward(AutogradContext* ctx, const variable_list& h) {
+        return {istftOf(dense(h[0]), savedInt(ctx, "n"), savedInt(ctx, "hop"), ctx->saved_data["center"].toBool(),
+                        savedWindow(ctx), savedInt(ctx, "size"), savedDouble(ctx, "scale")),
+                Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+};
+
+Tensor c2cAxis(const Tensor& x, int64_t dim, int64_t direction, double scale) {
+    return wantsGrad(x) ? C2CNode::apply(x, dim, direction, scale) : execAxis(x, dim, direction, scale);
+}
+Tensor c2c2D(const Tensor& x, int64_t direction, double scale) {
+    return wantsGrad(x) ? C2C2DNode::apply(x, direction, scale) : exec2D(x, direction, scale);
+}
+Tensor r2c(const Tensor& x, double scale, double edge, double inside) {
+    return wantsGrad(x) ? R2CNode::apply(x, scale, edge, inside) : execR2C(x, scale * edge, scale * inside);
+}
+Tensor c2r(const Tensor& x, int64_t n, double scale, double edge, double inside) {
+    return wantsGrad(x) ? C2RNode::apply(x, n, scale, edge, inside) : execC2R(x, n, edge, inside, scale);
+}
+Tensor stftOf(const Tensor& x, int64_t n, int64_t hop, bool center, const Maybe& w) {
+    return wantsFrames(x, w) ? StftNode::apply(x, w, n, hop, center) : execStft(x, n, hop, center, w.value_or(Tensor()));
+}
+Tensor istftOf(const Tensor& spec, int64_t n, int64_t hop, bool center, const Maybe& w, int64_t outLen, double scale) {
+    return wantsFrames(spec, w) ? IstftNode::apply(spec, w, n, hop, center, outLen, scale)
+                                : execIstft(spec, n, hop, center, w.value_or(Tensor()), outLen, scale);
+}
+Tensor stftAdjoint(const Tensor& g, int64_t n, int64_t hop, bool center, const Maybe& w, int64_t length) {
+    return wantsGrad(g) ? StftAdjointNode::apply(g, w, n, hop, center, length)
+                        : execStftAdjoint(g, n, hop, center, w.value_or(Tensor()), length);
+}
+Tensor istftAdjoint(const Tensor& g, int64_t n, int64_t hop, bool center, const Maybe& w, int64_t frames, double scale) {
+    return wantsGrad(g) ? IstftAdjointNode::apply(g, w, n, hop, center, frames, scale)
+                        : execIstftAdjoint(g, n, hop, center, w.value_or(Tensor()), frames, scale);
+}
 
 // ------------------------------------------------------------------ entry points
 double scaleOf(int norm, double n, bool forward) {   // norm: 0 backward, 1 ortho, 2 forward
@@ -415,26 +500,24 @@ Maybe fft(const Tensor& x, int64_t dim, int64_t direction, int64_t norm) {
     dim = dim < 0 ? dim + x.dim() : dim;
     if (dim < 0 || dim >= x.dim()) return std::nullopt;
     const double s = scaleOf((int)norm, (double)x.size(dim), direction < 0);
-    return wantsGrad(x) ? C2CNode::apply(x, dim, direction, s) : execAxis(x, dim, direction, s);
+    return c2cAxis(x, dim, direction, s);
 }
 
 Maybe fft2(const Tensor& x, int64_t direction, int64_t norm) {
     if (!takes(x, at::kComplexFloat) || !plainMode() || x.dim() < 2) return std::nullopt;
     const double s = scaleOf((int)norm, (double)x.size(-2) * (double)x.size(-1), direction < 0);
-    return wantsGrad(x) ? C2C2DNode::apply(x, direction, s) : exec2D(x, direction, s);
+    return c2c2D(x, direction, s);
 }
 
 Maybe rfft(const Tensor& x, int64_t norm) {
     if (!takes(x, at::kFloat) || !plainMode() || x.dim() < 1) return std::nullopt;
-    const double s = scaleOf((int)norm, (double)x.size(-1), true);
-    return wantsGrad(x) ? R2CNode::apply(x, s) : execR2C(x, s, s);
+    return r2c(x, scaleOf((int)norm, (double)x.size(-1), true));
 }
 
 Maybe irfft(const Tensor& x, int64_t n, int64_t norm) {
     if (!takes(x, at::kComplexFloat) || !plainMode() || x.dim() < 1 || n < 1 || x.size(-1) != n / 2 + 1)
         return std::nullopt;
-    const double s = scaleOf((int)norm, (double)n, false);
-    return wantsGrad(x) ? C2RNode::apply(x, n, s) : execC2R(x, n, 1.0, 1.0, s);
+    return c2r(x, n, scaleOf((int)norm, (double)n, false));
 }
 
 Maybe rfft2(const Tensor& x, int64_t norm) {
@@ -453,24 +536,19 @@ Maybe irfft2(const Tensor& x, int64_t nx, int64_t norm) {
 bool oneKernelFrames(int64_t n) { return n >= 64 && n <= 8192 && (n & (n - 1)) == 0; }
 
 Maybe stft(const Tensor& x, int64_t n, int64_t hop, bool center, const Maybe& w) {
-    const Tensor window = w.value_or(Tensor());
     if (!takes(x, at::kFloat) || !plainMode() || x.dim() != 2 || !x.is_contiguous() || x.is_neg() || hop < 1 ||
         !oneKernelFrames(n) || x.size(1) < (center ? n + 2 : n) || x.size(0) < 1 ||
-        (window.defined() && !takes(window, at::kFloat)))
+        (w && !takes(*w, at::kFloat)))
         return std::nullopt;
-    return wantsGrad(x) || (window.defined() && wantsGrad(window)) ? StftNode::apply(x, w, n, hop, center)
-                                                                   : execStft(x, n, hop, center, window);
+    return stftOf(x, n, hop, center, w);
 }
 
 Maybe istft(const Tensor& spec, int64_t n, int64_t hop, bool center, const Maybe& w, int64_t outLen, double scale) {
-    const Tensor window = w.value_or(Tensor());
     if (!takes(spec, at::kComplexFloat) || !plainMode() || spec.dim() != 3 || !spec.is_contiguous() ||
         spec.is_conj() || spec.is_neg() ||
-        !oneKernelFrames(n) || (window.defined() && !takes(window, at::kFloat)))
+        !oneKernelFrames(n) || (w && !takes(*w, at::kFloat)))
         return std::nullopt;
-    return wantsGrad(spec) || (window.defined() && wantsGrad(window))
-               ? IstftNode::apply(spec, w, n, hop, center, outLen, scale)
-               : execIstft(spec, n, hop, center, window, outLen, scale);
+    return istftOf(spec, n, hop, center, w, outLen, scale);
 }
 
 }  // namespace
