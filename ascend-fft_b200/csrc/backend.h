@@ -78,9 +78,9 @@ int launchLongB(const void* in, void* out, uint32_t n1, uint32_t n2, uint64_t ba
 // memory, so that later launches neither load device code nor set kernel attributes.
 int prepareLongKernels();
 
-// C2C of n = 1024 and 8192..65536 in one pass, no workspace: directTableBytes(n) bytes of twiddle
-// table (0: no such kernel), in == out allowed.  Optional entries: with a seam that lacks them
-// (null addresses) those lengths run the kernels below and the single-CTA variants.
+// C2C of n = 32768 and 65536 in one pass, a thread-block cluster per row, no workspace:
+// directTableBytes(n) bytes of twiddle table (0: no such kernel), in == out allowed.  Optional
+// entries: with a seam that lacks them (null addresses) those lengths run the kernels below.
 __attribute__((weak)) size_t directTableBytes(uint32_t n);
 __attribute__((weak)) int buildDirectTable(void* table, uint32_t n, void* stream);
 __attribute__((weak)) int launchDirect(const void* in, void* out, uint32_t n, uint64_t batch, bool inverse,

@@ -160,7 +160,7 @@ int buildLinearTwiddles(void* tw, int count, long long stride, long long n, void
 int launchC2C(const void* in, void* out, uint32_t n, uint64_t batch, bool inverse, float scale,
               const void* tw, int e, int cta, void* stream) {
     const Entry* x = findEntry(kC2C, n, e, cta, inverse ? 1 : 0);
-    if (!x || !x->fn) return (int)cudaErrorInvalidDeviceFunction;
+    if (!x) return (int)cudaErrorInvalidDeviceFunction;
     if (int err = prepareEntry(x)) return err;
     return rc(launchPdl(x->fn, gridFor(batch, x->rows), x->cta, x->smem, S(stream), static_cast<const float2*>(in),
                         static_cast<float2*>(out), static_cast<const float2*>(tw), batch, scale));

@@ -1,5 +1,6 @@
 // C2C kernel instantiations (inverse).  Variant list: N in 32..16384, E in {8,16},
-// CTA in {128,256,512} (1024 only for one-transform-per-CTA lengths), shared memory <= 227 KB.
+// CTA in {128,256,512} (1024 only for one-transform-per-CTA lengths), shared memory <= 227 KB; E = 32
+// at 1024, 8192 and 16384 (k_c2c_fwd.cu).
 #include "fft_kernels.cuh"
 #include "registry.cuh"
 
@@ -8,8 +9,6 @@ namespace dev {
 
 #define E_(N, E, CTA) {N, E, CTA, 1, (const void*)&k_c2c<N, E, BFLY_ROWS(N, E, CTA), true>, \
     BFLY_ROWS(N, E, CTA), BFLY_ROWS(N, E, CTA) * smem_stride<N, E, false>() * 8}
-// Radix 16 served by k_long_direct.cu; listed for the candidates' limits.
-#define D_(N, CTA) {N, 16, CTA, 1, nullptr, BFLY_ROWS(N, 16, CTA), BFLY_ROWS(N, 16, CTA) * smem_stride<N, 16, false>() * 8}
 static const Entry kTable[] = {
     E_(32, 8, 128),
     E_(32, 8, 256),
@@ -44,9 +43,9 @@ static const Entry kTable[] = {
     E_(1024, 8, 128),
     E_(1024, 8, 256),
     E_(1024, 8, 512),
-    D_(1024, 128),
-    D_(1024, 256),
-    D_(1024, 512),
+    E_(1024, 16, 128),
+    E_(1024, 16, 512),
+    E_(1024, 32, 64),
     E_(2048, 8, 256),
     E_(2048, 8, 512),
     E_(2048, 16, 128),
@@ -56,10 +55,9 @@ static const Entry kTable[] = {
     E_(4096, 16, 256),
     E_(4096, 16, 512),
     E_(8192, 8, 1024),
-    D_(8192, 512),
-    D_(16384, 1024),
+    E_(8192, 32, 256),
+    E_(16384, 32, 512),
 };
-#undef D_
 #undef E_
 
 const Entry* findC2CInv(uint32_t n, int e, int cta) {

@@ -1,12 +1,6 @@
-// C2C of n = 1024 and 8192 .. 65536 in one HBM pass without a workspace.
+// C2C of n = 32768 and 65536 in one HBM pass without a workspace.
 //
-// n = 1024, 8192, 16384: rows in one CTA, 32 values a thread (k_c2c): a pass and an exchange fewer
-// than with 16.  n = 1024 (two passes, two rows to a 64-thread CTA), us at 256 / 2048 / 6144 rows: 2.93 /
-// 7.03 / 16.9 with 16 values, 2.25 / 6.01 / 15.4 with 32; 512 points gained nothing.  8192 and 16384
-// (three passes; GB/s at 2^25 points): 4354 / 3295 with 16, 5049 / 3755 with 32, 5433 / 4322 with the
-// next rows on their way into L2 meanwhile (prefetch_l2).
-//
-// n = 32768, 65536 = N1 * 256: one thread-block cluster per row, 4096 points per CTA.  The row
+// n = N1 * 256: one thread-block cluster per row, 4096 points per CTA.  The row
 // is the N1 x 256 matrix x[256*n1 + n2] of the four-step decomposition
 //   X[k1 + N1*k2] = sum_n2 W_256^(n2*k2) * W_n^(n2*k1) * sum_n1 W_N1^(n1*k1) x[256*n1 + n2].
 // CTA `rank` owns columns n2 in [rank*COLS, (rank+1)*COLS) for the N1-point FFTs and rows k1 in
@@ -106,24 +100,6 @@ namespace backend {
 
 namespace {
 
-constexpr int kSingleE = 32;   // values per thread of the single-CTA rows
-
-template <int N, int ROWS = 1>
-int launchSingle(const float2* in, float2* out, uint64_t batch, bool inverse, float scale, const float2* table,
-                 cudaStream_t s) {
-    constexpr int smem = ROWS * dev::smem_stride<N, kSingleE, false>() * 8;
-    const void* fn = inverse ? (const void*)dev::k_c2c<N, kSingleE, ROWS, true> : (const void*)dev::k_c2c<N, kSingleE, ROWS, false>;
-    if (batch > 0x7fffffffull) return (int)cudaErrorInvalidValue;
-    if (int e = optInSharedMemory(fn, smem)) return e;
-    return (int)launchPdl(fn, (unsigned)((batch + ROWS - 1) / ROWS), ROWS * (N / kSingleE), smem, s, in, out, table, batch, scale);
-}
-template <int N>
-int buildSingle(float2* t, cudaStream_t s) {
-    constexpr int c = dev::Sched<N, kSingleE>::TWSIZE;
-    dev::k_tw_stockham<N, kSingleE><<<(c + 255) / 256, 256, 0, s>>>(t);
-    return (int)cudaGetLastError();
-}
-
 template <int N1>
 int buildTable(float2* t, cudaStream_t s) {
     using L = dev::LongDirect<N1>;
@@ -150,9 +126,6 @@ int launchRows(const float2* in, float2* out, uint64_t batch, bool inverse, floa
 
 size_t directTableBytes(uint32_t n) {
     switch (n) {
-        case 1024: return dev::Sched<1024, kSingleE>::TWSIZE * 8;
-        case 8192: return dev::Sched<8192, kSingleE>::TWSIZE * 8;
-        case 16384: return dev::Sched<16384, kSingleE>::TWSIZE * 8;
         case 32768: return dev::LongDirect<128>::TABLE * 8;
         case 65536: return dev::LongDirect<256>::TABLE * 8;
         default: return 0;
@@ -163,9 +136,6 @@ int buildDirectTable(void* table, uint32_t n, void* stream) {
     float2* t = static_cast<float2*>(table);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     switch (n) {
-        case 1024: return buildSingle<1024>(t, s);
-        case 8192: return buildSingle<8192>(t, s);
-        case 16384: return buildSingle<16384>(t, s);
         case 32768: return buildTable<128>(t, s);
         case 65536: return buildTable<256>(t, s);
         default: return (int)cudaErrorInvalidValue;
@@ -179,9 +149,6 @@ int launchDirect(const void* in, void* out, uint32_t n, uint64_t batch, bool inv
     const float2* t = static_cast<const float2*>(table);
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     switch (n) {
-        case 1024: return launchSingle<1024, 2>(x, y, batch, inverse, scale, t, s);
-        case 8192: return launchSingle<8192>(x, y, batch, inverse, scale, t, s);
-        case 16384: return launchSingle<16384>(x, y, batch, inverse, scale, t, s);
         case 32768: return launchRows<128>(x, y, batch, inverse, scale, t, s);
         case 65536: return launchRows<256>(x, y, batch, inverse, scale, t, s);
         default: return (int)cudaErrorInvalidValue;

@@ -89,6 +89,25 @@ void stringAxis(const json::Node& obj, const char* key, std::vector<std::string>
     }
 }
 
+// Threads per CTA of the C2C kernel with 32 values a thread (two rows of 1024, one longer row); 0
+// where there is none.
+int wideCta(uint32_t n) {
+    if (n < 1024 || n > kMaxSinglePass) return 0;
+    const int cta = n == 1024 ? 64 : (int)(n / 32);
+    return backend::hasVariant(backend::kC2C, n, 32, cta) ? cta : 0;
+}
+
+// The single-pass kernel that a stockham candidate names at n: its radix and CTA size, except that
+// radix 16 with 4096 values a CTA at 1024, and with one row a CTA at 8192 and 16384, names the kernel
+// with 32 values a thread, which replaced the one of 16 there (k_c2c_fwd.cu has both times).
+bool stockhamVariant(uint32_t n, int radix, int ctaThreads, int* e, int* cta) {
+    const int wide = radix == 16 && ctaThreads == (n == 1024 ? 256 : (int)(n / 16)) ? wideCta(n) : 0;
+    if (!wide && !backend::hasVariant(backend::kC2C, n, radix, ctaThreads)) return false;
+    *e = wide ? 32 : radix;
+    *cta = wide ? wide : ctaThreads;
+    return true;
+}
+
 enum ShapeKind { kRunC2C, kRunR2C, kRunC2R, kRunLong, kPrepare, kMeasure, kExecC2C, kExecR2C, kExecC2R };
 
 // Real transforms run an n/2-point complex FFT.
@@ -307,6 +326,7 @@ std::vector<Candidate> enumerate(const DesignSpace& sp, const Hardware& hw, uint
             else c.state = State::Unverified;
         } else {   // stockham single pass
             const size_t smem = c.p.smemBytes(n, cta);
+            int ve = 0, vcta = 0;
             if (n > kMaxSinglePass) {
                 infeasible("single-pass stockham holds at most 16384 points in shared memory");
             } else if ((uint32_t)radix > n / 2) {
@@ -318,7 +338,7 @@ std::vector<Candidate> enumerate(const DesignSpace& sp, const Hardware& hw, uint
                 std::snprintf(buf, sizeof(buf), "shared memory %.1f KiB > %d KiB per CTA (radix=%d, n=%u)",
                               smem / 1024.0, hw.smemPerCta / 1024, radix, n);
                 infeasible(buf);
-            } else if (!backend::hasVariant(backend::kC2C, n, radix, cta)) {
+            } else if (!stockhamVariant(n, radix, cta, &ve, &vcta)) {
                 std::snprintf(buf, sizeof(buf), "no compiled kernel for (n=%u, radix=%d, cta=%d)", n, radix, cta);
                 infeasible(buf);
             } else {
@@ -490,26 +510,27 @@ bool Plan::validShape(uint32_t n, uint32_t batch, int kind) const {
     return resolve(rk, n, &e, &cta) == 0;
 }
 
-// Kernel variant for (kind, n): the candidate's radix/cta when compiled for n (one CTA per
-// transform, e = radix); otherwise, for long C2C lengths, the one-pass kernels (e = -3), the L2
-// ring (e = -2), one persistent thread-block cluster per row (e = -1) or the four-step kernels
-// (e = 0), by the candidate's schedule.  The one-pass kernels take "stockham" candidates of radix 16
-// at 1024 and at every long length: they run 1.1x (1024) to 1.3x (8192, 32768) as fast as what served
-// those before, radix-16 single CTAs up to 16384 and four-step above (k_long_direct.cu).
+// Kernel variant for (kind, n): the single-CTA kernel that the candidate names (stockhamVariant; e =
+// its values per thread); otherwise, for long C2C lengths and by the candidate's schedule, the kernel
+// with 32 values a thread up to 16384 or the one-pass cluster kernel above (e = -3, "stockham"), the
+// L2 ring (e = -2), one persistent thread-block cluster per row (e = -1) or the four-step kernels
+// (e = 0).
 int Plan::resolve(int kind, uint32_t n, int* e, int* cta) const {
     const int r = cand_.p.radix, c = cand_.a.ctaThreads;
     if (kind == backend::kC2C) {
         const std::string& sched = cand_.f.schedule;
-        if (sched == "stockham" && (r == 16 || !backend::hasVariant(backend::kC2C, n, r, c)) &&
-            backend::directTableBytes && backend::directTableBytes(n)) {
-            *e = -3;
-            *cta = 256;
-            return 0;
-        }
-        if (sched == "stockham" && n <= kMaxSinglePass && backend::hasVariant(backend::kC2C, n, r, c)) {
-            *e = r;
-            *cta = c;
-            return 0;
+        if (sched == "stockham") {
+            if (n <= kMaxSinglePass && stockhamVariant(n, r, c, e, cta)) return 0;
+            if (n > 4096 && wideCta(n)) {
+                *e = 32;
+                *cta = wideCta(n);
+                return 0;
+            }
+            if (backend::directTableBytes && backend::directTableBytes(n)) {
+                *e = -3;
+                *cta = 256;
+                return 0;
+            }
         }
         if (sched == "ring" && backend::hasLongRing(n)) {
             *e = -2;
@@ -668,7 +689,7 @@ int Plan::prepare(uint32_t n, uint32_t batch) {
     tf_.push_back({Transform::GenTwiddles, "FP64 twiddle tables built on the device, rounded to fp32"});
     tf_.push_back({Transform::LaunchKernel, e > 0 ? "stockham single-pass kernel on the context stream"
                                             : e == -1 ? "one thread-block cluster per row (on-chip transpose)"
-                                            : e == -3 ? "one pass, a CTA or a thread-block cluster per row"
+                                            : e == -3 ? "one pass, a thread-block cluster per row"
                                             : e == -2 ? "one persistent four-step launch, intermediate in an L2 ring"
                                                       : "four-step column + row kernels on the context stream"});
     return 0;
