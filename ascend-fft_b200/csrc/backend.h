@@ -79,7 +79,8 @@ int launchLongB(const void* in, void* out, uint32_t n1, uint32_t n2, uint64_t ba
 int prepareLongKernels();
 
 // C2C of n = 32768 and 65536 in one pass, a thread-block cluster per row, no workspace:
-// directTableBytes(n) bytes of twiddle table (0: no such kernel), in == out allowed.  Optional
+// directTableBytes(n) bytes of twiddle table (0: no such kernel, or one that the current device cannot
+// hold: 65536 points are a cluster of 16 CTAs, beyond the portable 8), in == out allowed.  Optional
 // entries: with a seam that lacks them (null addresses) those lengths run the kernels below.
 __attribute__((weak)) size_t directTableBytes(uint32_t n);
 __attribute__((weak)) int buildDirectTable(void* table, uint32_t n, void* stream);

@@ -19,6 +19,9 @@
 // at four 64-register CTAs per SM.
 #include <cuda_runtime.h>
 
+#include <mutex>
+#include <vector>
+
 #include "backend.h"
 #include "fft_kernels.cuh"
 #include "launch.cuh"
@@ -100,6 +103,48 @@ namespace backend {
 
 namespace {
 
+// Whether the current device can hold a cluster beyond the portable size; allows the kernel that
+// size.  Asked once per device and kernel.
+bool wideClusterFits(const void* fn, unsigned cluster, int block, int smem) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return false;
+    struct Answer {
+        int device;
+        const void* fn;
+        bool fits;
+    };
+    static std::mutex mu;
+    static std::vector<Answer> known;
+    std::lock_guard<std::mutex> lock(mu);
+    for (const Answer& a : known)
+        if (a.device == device && a.fn == fn) return a.fits;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = cluster;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cluster);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    const bool fits = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                      cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters > 0;
+    cudaGetLastError();   // a refusal is an answer, not an error of the calls that follow
+    known.push_back({device, fn, fits});
+    return fits;
+}
+
+template <int N1>
+size_t tableBytes() {
+    using L = dev::LongDirect<N1>;
+    if (L::C > 8)
+        for (const void* fn : {(const void*)dev::k_long_direct<N1, false>, (const void*)dev::k_long_direct<N1, true>})
+            if (!wideClusterFits(fn, L::C, L::NT, L::SMEM)) return 0;
+    return L::TABLE * 8;
+}
+
 template <int N1>
 int buildTable(float2* t, cudaStream_t s) {
     using L = dev::LongDirect<N1>;
@@ -117,8 +162,7 @@ int launchRows(const float2* in, float2* out, uint64_t batch, bool inverse, floa
     using L = dev::LongDirect<N1>;
     const void* fn = inverse ? (const void*)dev::k_long_direct<N1, true> : (const void*)dev::k_long_direct<N1, false>;
     if (batch > 0x7fffffffull / L::C) return (int)cudaErrorInvalidValue;
-    if (L::C > 8)   // beyond the portable cluster size
-        if (cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) return (int)e;
+    if (L::C > 8 && !wideClusterFits(fn, L::C, L::NT, L::SMEM)) return (int)cudaErrorInvalidConfiguration;
     return (int)launchPdlCluster(fn, (unsigned)(batch * L::C), L::NT, L::SMEM, L::C, s, in, out, table, scale);
 }
 
@@ -126,8 +170,8 @@ int launchRows(const float2* in, float2* out, uint64_t batch, bool inverse, floa
 
 size_t directTableBytes(uint32_t n) {
     switch (n) {
-        case 32768: return dev::LongDirect<128>::TABLE * 8;
-        case 65536: return dev::LongDirect<256>::TABLE * 8;
+        case 32768: return tableBytes<128>();
+        case 65536: return tableBytes<256>();
         default: return 0;
     }
 }

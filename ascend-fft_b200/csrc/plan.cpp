@@ -514,7 +514,7 @@ bool Plan::validShape(uint32_t n, uint32_t batch, int kind) const {
 // its values per thread); otherwise, for long C2C lengths and by the candidate's schedule, the kernel
 // with 32 values a thread up to 16384 or the one-pass cluster kernel above (e = -3, "stockham"), the
 // L2 ring (e = -2), one persistent thread-block cluster per row (e = -1) or the four-step kernels
-// (e = 0).
+// (e = 0), which also take a "stockham" candidate where the device cannot hold the cluster.
 int Plan::resolve(int kind, uint32_t n, int* e, int* cta) const {
     const int r = cand_.p.radix, c = cand_.a.ctaThreads;
     if (kind == backend::kC2C) {

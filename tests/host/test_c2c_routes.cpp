@@ -14,6 +14,7 @@ namespace fake {
 extern int allocations, releases, launches, syncs, failAllocation, failLaunch, failSync;
 extern int lastE, lastCta, directTables;
 extern uint32_t clusterUnavailable;
+extern int longLaunches;
 }  // namespace fake
 
 #define CHECK(cond)                                                                    \
@@ -108,6 +109,19 @@ int main(int argc, char** argv) {
     std::vector<float> a(2 * 1024, 1.f), b(2 * 1024);
     const bfly::HostRequest reqs[2] = {{x.data(), y.data(), 65536, 1, 1, 2.f}, {a.data(), b.data(), 1024, 1, -1, 1.f}};
     CHECK(p->runMany(reqs, 2) == 0 && y[9] == -2.f * x[9] && b[0] == 1024.f);
+    // a device that cannot hold the cluster of 65536: every entry takes the four-step kernels
+    fake::clusterUnavailable = 65536;
+    auto q = make(context, 1024, "r16_cta256_shared_fp32_stockham");
+    CHECK(q);
+    const int before = fake::directTables;
+    for (int k = 0; k < 2; ++k) {
+        fake::lastE = 0;
+        if (k == 0) CHECK(q->execC2C(x.data(), y.data(), 65536, 1, -1, 1.f, nullptr) == 0);
+        if (k == 1) CHECK(q->runLong(x.data(), y.data(), 65536, 1, -1) == 0 && q->runMany(reqs, 2) == 0);
+        CHECK(fake::longLaunches > 0 && fake::lastE != -3 && fake::directTables == before);
+        fake::longLaunches = 0;
+    }
+    CHECK(q->execC2C(x.data(), y.data(), 32768, 1, -1, 1.f, nullptr) == 0 && fake::lastE == -3);
     std::printf("all checks passed\n");
     return 0;
 }
