@@ -3,8 +3,9 @@
 CUDA translation units are compiled by nvcc with `-gencode arch=compute_100a,code=sm_100a`,
 host units by g++, and everything is linked into bfly/_lib/libbfly_b200.so next to the Python
 package (the CUDA runtime is linked statically); csrc_torch/ becomes the Python module
-bfly/_lib/_torch_ops.so on top of it.  Objects go to _build/; a unit is rebuilt only
-when it or a header is newer than its object.
+bfly/_lib/_torch_ops.so on top of it where torch is installed (the library itself needs none).
+Objects go to _build/; a unit is rebuilt only when it or a header is newer than its object, the module
+also when it was built for another torch or Python.
 
     python ascend-fft_b200/build.py [--force] [--jobs N]
 """
@@ -63,6 +64,16 @@ def compile_one(cmd):
     return r.stderr
 
 
+def torch_abi() -> str | None:
+    """What the torch module is built against; None without torch."""
+    import importlib.metadata
+    import sysconfig
+    try:
+        return f"torch {importlib.metadata.version('torch')} {sysconfig.get_config_var('SOABI')}"
+    except importlib.metadata.PackageNotFoundError:
+        return None
+
+
 def torch_cmd(obj: Path):
     """Compile and link commands of the torch module (C++ against the installed torch)."""
     import sysconfig
@@ -77,6 +88,25 @@ def torch_cmd(obj: Path):
             ["g++", "-shared", "-o", str(TORCH_LIB.with_suffix(".so.tmp")), str(obj), *[f"-L{d}" for d in dirs],
              f"-L{LIBDIR}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", f"-l:{LIB.name}",
              "-Wl,-rpath,$ORIGIN"])
+
+
+def build_torch_object(force: bool):
+    """Compile the torch module where it is stale; its link command where that has to run."""
+    abi = torch_abi()
+    if abi is None:
+        print("torch is not installed: the module of bfly's torch functions is not built", file=sys.stderr)
+        return None
+    obj, stamp = BUILD / (TORCH_SRC.stem + ".torch.o"), BUILD / (TORCH_SRC.stem + ".torch.abi")
+    fresh = stamp.exists() and stamp.read_text() == abi and not force and \
+        not stale(TORCH_SRC, obj, [ROOT / "include" / "bfly_b200.h"])
+    if fresh and TORCH_LIB.exists() and TORCH_LIB.stat().st_mtime >= obj.stat().st_mtime:
+        return None
+    compile_cmd, link_cmd = torch_cmd(obj)
+    if not fresh:
+        stamp.unlink(missing_ok=True)
+        compile_one(compile_cmd)
+        stamp.write_text(abi)
+    return link_cmd
 
 
 def build(force: bool = False, jobs: int | None = None, verbose: bool = False) -> Path:
@@ -97,23 +127,21 @@ def build(force: bool = False, jobs: int | None = None, verbose: bool = False) -
         if force or stale(src, obj, deps):
             cmds.append(["g++", "-std=c++17", "-O2", "-fPIC", "-Wall", "-Wextra", *INCLUDES,
                          "-c", str(src), "-o", str(obj)])
-    torch_obj = BUILD / (TORCH_SRC.stem + ".torch.o")
-    torch_compile, torch_link = torch_cmd(torch_obj)
-    if force or stale(TORCH_SRC, torch_obj, [ROOT / "include" / "bfly_b200.h"]):
-        cmds.append(torch_compile)
-    if cmds:
-        with cf.ThreadPoolExecutor(max_workers=jobs or min(len(cmds), os.cpu_count() or 4)) as ex:
-            for out in ex.map(compile_one, cmds):
-                if verbose and out:
-                    print(out, file=sys.stderr)
-    if cmds or not LIB.exists() or any(o.stat().st_mtime > LIB.stat().st_mtime for o in objs):
-        tmp = LIB.with_suffix(".so.tmp")
-        compile_one([nvcc(), "-shared", *ARCH, "-cudart", "static", "-o", str(tmp),
-                     *[str(o) for o in objs], "-lpthread", "-ldl", "-lrt"])
-        os.replace(tmp, LIB)
-    if not TORCH_LIB.exists() or torch_obj.stat().st_mtime > TORCH_LIB.stat().st_mtime:
-        compile_one(torch_link)
-        os.replace(torch_link[3], TORCH_LIB)
+    workers = jobs or min(len(cmds) + 1, os.cpu_count() or 4)
+    with cf.ThreadPoolExecutor(max_workers=workers) as ex:
+        module = ex.submit(build_torch_object, force)   # the longest of them
+        for out in ex.map(compile_one, cmds):
+            if verbose and out:
+                print(out, file=sys.stderr)
+        if cmds or not LIB.exists() or any(o.stat().st_mtime > LIB.stat().st_mtime for o in objs):
+            tmp = LIB.with_suffix(".so.tmp")
+            compile_one([nvcc(), "-shared", *ARCH, "-cudart", "static", "-o", str(tmp),
+                         *[str(o) for o in objs], "-lpthread", "-ldl", "-lrt"])
+            os.replace(tmp, LIB)
+        link = module.result()
+    if link:
+        compile_one(link)
+        os.replace(TORCH_LIB.with_suffix(".so.tmp"), TORCH_LIB)
     return LIB
 
 
