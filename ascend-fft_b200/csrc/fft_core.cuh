@@ -553,11 +553,11 @@ __device__ __forceinline__ float2 ld_stream(const float2* p) { return __ldcs(p);
 // keep several twiddle tables in L1 (the ragged launch over many lengths) lost with it and keep
 // ld_stream.
 __device__ __forceinline__ float2 ld_once_ca(const float2* p) { return __ldca(p); }
-// A caller's array of which a kernel reads elements more than once (the overlapping frames of a
-// signal, a window): through L1 by the same coherent load, for the same reason.  Read-only loads are
-// for the tables, which are complete before any kernel that reads them is launched.
-template <class T>
-__device__ __forceinline__ T ld_reused(const T* p) { return __ldca(p); }
+// Arrays of the caller of which a kernel reads elements more than once (the overlapping frames of a
+// signal, a window) are read by plain loads through pointers without __restrict__: coherent for the
+// same reason, and free for the compiler to unroll and to issue together, which inline assembly
+// (__ldca among it) is not: with that the edge envelopes of a short-time transform, chains of window
+// loads, took up to seven times as long.
 __device__ __forceinline__ void st_stream(float2* p, float2 v) { __stcs(p, v); }
 
 // Loading ahead into L2: a CTA asks for the lines of the tile that the CTA `ahead` places later

@@ -72,7 +72,7 @@ struct IstftSegment {
         for (int r = threadIdx.x; r < (int)hop; r += CTA) {
             float e = 0.f;
             for (int j = r; j < N; j += (int)hop) {
-                const float w = window ? ld_reused(window + j) : 1.f;
+                const float w = window ? window[j] : 1.f;
                 e += w * w;
             }
             rinv[r] = e > 0.f ? 1.f / e : 0.f;
@@ -132,7 +132,7 @@ struct IstftSegment {
         for (int64_t f = fh - K + 1 > 0 ? fh - K + 1 : 0; f <= fh && f < (int64_t)frames; ++f) {
             const int64_t j = p - f * hop;
             if (j < N) {
-                const float w = window ? ld_reused(window + j) : 1.f;
+                const float w = window ? window[j] : 1.f;
                 e += w * w;
             }
         }

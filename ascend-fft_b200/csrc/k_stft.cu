@@ -3,7 +3,7 @@
 //   frame f of signal s:  y[j] = w[j] * x_s[f*hop + j - (center ? N/2 : 0)],  j < N,
 //   positions outside [0, L) reflected (x[-i] = x[i], x[L-1+i] = x[L-1-i]) as torch.stft's
 //   default pad_mode="reflect";  out[s][f][k] = sum_j y[j] exp(-2*pi*i*j*k/N), k <= N/2.
-// Frames overlap, so samples are read through L1 (ld_reused: reuse across the N/hop frames that
+// Frames overlap, so samples are read through L1 (reuse across the N/hop frames that
 // cover them) instead of the streaming path of the batched transforms.
 // The reference runs its STFT cases as a dense-frame R2C proxy (docs/testing.md:118,
 // config/test_matrix.json "stft": R2C with batch = frames); framing, windowing and overlap
@@ -25,8 +25,8 @@ namespace dev {
 // bins are weighted s_edge (k = 0, N/2) and s_int (the rest).
 template <int N, int E, int ROWS, bool ADJ>
 __global__ void __launch_bounds__((N / 2 / E) * ROWS, min_blocks<E>((N / 2 / E) * ROWS))
-k_stft(const float* __restrict__ sig, float2* __restrict__ out, const float2* __restrict__ tw,
-       const float2* __restrict__ twr, const float* __restrict__ window, uint64_t rows,
+k_stft(const float* sig, float2* __restrict__ out, const float2* __restrict__ tw,
+       const float2* __restrict__ twr, const float* window, uint64_t rows,
        uint32_t framesPerSignal, int64_t sigLen, uint64_t sigStride, uint32_t hop, int center, int64_t gStart,
        float s_edge, float s_int) {
     constexpr int M = N / 2;
@@ -53,7 +53,7 @@ k_stft(const float* __restrict__ sig, float2* __restrict__ out, const float2* __
         for (int r = threadIdx.x; r < (int)hop; r += blockDim.x) {
             float e = 0.f;
             for (int j = r; j < N; j += (int)hop) {
-                const float w = window ? ld_reused(window + j) : 1.f;
+                const float w = window ? window[j] : 1.f;
                 e += w * w;
             }
             rinv[r] = e > 0.f ? 1.f / e : 0.f;
@@ -67,7 +67,7 @@ k_stft(const float* __restrict__ sig, float2* __restrict__ out, const float2* __
         for (int64_t g = fh - K + 1 > 0 ? fh - K + 1 : 0; g <= fh && g < (int64_t)framesPerSignal; ++g) {
             const int64_t j = p - g * hop;
             if (j < N) {
-                const float w = window ? ld_reused(window + j) : 1.f;
+                const float w = window ? window[j] : 1.f;
                 e += w * w;
             }
         }
@@ -76,11 +76,11 @@ k_stft(const float* __restrict__ sig, float2* __restrict__ out, const float2* __
     auto sample = [&](int64_t i) {
         if constexpr (ADJ) {
             const int64_t k = i - gStart;
-            return k >= 0 && k < sigLen ? ld_reused(x + k) * inv(i) : 0.f;
+            return k >= 0 && k < sigLen ? x[k] * inv(i) : 0.f;
         } else {
             i = i < 0 ? -i : i;
             i = i >= sigLen ? 2 * (sigLen - 1) - i : i;
-            return ld_reused(x + i);
+            return x[i];
         }
     };
     // Interior frames starting on an 8-byte boundary (every frame of an even hop away from the
@@ -95,7 +95,7 @@ k_stft(const float* __restrict__ sig, float2* __restrict__ out, const float2* __
     // on memory per issue).
     float2 v[E];
     if (direct) {
-        TM::load_first(v, t, [&](int m) { return ld_reused(xv + m); });
+        TM::load_first(v, t, [&](int m) { return xv[m]; });
         if constexpr (ADJ) {   // start even, hop even: i mod hop and i mod hop + 1 are one pair
             const uint32_t i0 = (uint32_t)(start % hop);
             TM::for_each_in(v, t, [&](int m, float2& z) {
@@ -109,7 +109,7 @@ k_stft(const float* __restrict__ sig, float2* __restrict__ out, const float2* __
     }
     if (window) {
         float2 w[E];
-        TM::load_first(w, t, [&](int m) { return ld_reused(reinterpret_cast<const float2*>(window) + m); });
+        TM::load_first(w, t, [&](int m) { return reinterpret_cast<const float2*>(window)[m]; });
 #pragma unroll
         for (int i = 0; i < E; ++i) v[i] = __fmul2_rn(v[i], w[i]);
     }
@@ -139,7 +139,7 @@ __host__ __device__ constexpr int istft_row_stride() {
 template <int N, int E, int ROWS, int MINB, int VEC, bool ADJ>
 __global__ void __launch_bounds__((N / 2 / E) * ROWS, MINB)
 k_istft(const float2* __restrict__ spec, float* __restrict__ out, const float2* __restrict__ tw,
-        const float2* __restrict__ twr, const float* __restrict__ window, uint32_t frames, uint32_t hop, uint32_t Q,
+        const float2* __restrict__ twr, const float* window, uint32_t frames, uint32_t hop, uint32_t Q,
         uint32_t segs, int64_t start, uint64_t outLen, float out_scale, float s_edge, float s_int, int pad) {
     constexpr int M = N / 2;
     constexpr int T = M / E;
@@ -171,10 +171,9 @@ k_istft(const float2* __restrict__ spec, float* __restrict__ out, const float2* 
         RS::load(v, sm, twr, t, rl, x, ADJ ? s_edge : 1.f, ADJ ? s_int : 1.f, ADJ ? 1.f : out_scale);
         TM::template passes<0>(v, sm, tw, t, rl);
         TM::sync(rl);
-        TM::for_each_out(v, t, [&](int i, float2 z) {   // windowed frame: samples 2i, 2i+1 at sm[i]
-            const float2 w = window ? ld_reused(reinterpret_cast<const float2*>(window) + i) : make_float2(1.f, 1.f);
-            sm[i] = make_float2(z.x * w.x, z.y * w.y);
-        });
+        if (window)   // every window load ahead of the stores below
+            TM::for_each_slot(v, t, [&](int i, float2& z) { z = __fmul2_rn(z, reinterpret_cast<const float2*>(window)[i]); });
+        TM::for_each_out(v, t, [&](int i, float2 z) { sm[i] = z; });   // windowed frame: samples 2i, 2i+1 at sm[i]
         __syncthreads();
         seg.template wave<VEC, CTA, ADJ>(f0, R, reinterpret_cast<const float*>(smem), 2 * S,
                                          [](const float* p, int) { return *p; },

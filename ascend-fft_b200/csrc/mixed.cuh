@@ -385,9 +385,9 @@ __global__ void __maxnreg__(ROWS::kRegs) k_c2r_mixed(const float2* __restrict__ 
 // STFT: frame f of signal s, y[j] = w[j] x_s[f hop + j - (center ? N/2 : 0)] (reflect padding,
 // as k_stft), packed as z[m] = y[2m] + i y[2m+1] and staged unpadded; then the R2C of k_r2c_mixed.
 template <class ROWS>
-__global__ void __maxnreg__(ROWS::kRegs) k_stft_mixed(const float* __restrict__ sig, float2* __restrict__ out,
+__global__ void __maxnreg__(ROWS::kRegs) k_stft_mixed(const float* sig, float2* __restrict__ out,
                                                        const float2* __restrict__ tw, const float2* __restrict__ twr,
-                                                       const float* __restrict__ window, MixedArgs a, uint64_t frames,
+                                                       const float* window, MixedArgs a, uint64_t frames,
                                                        uint32_t framesPerSignal, int64_t sigLen, uint64_t sigStride,
                                                        uint32_t hop, int center, int T, int rows, int len) {
     extern __shared__ float2 smem[];
@@ -406,20 +406,25 @@ __global__ void __maxnreg__(ROWS::kRegs) k_stft_mixed(const float* __restrict__ 
         auto sample = [&](int64_t i) {
             i = i < 0 ? -i : i;
             i = i >= sigLen ? 2 * (sigLen - 1) - i : i;
-            return ld_reused(x + i);
+            return x[i];
         };
         // interior frames starting on an 8-byte boundary read one float2 per complex value; the
         // others sample with reflection
         const bool direct = start >= 0 && start + 2 * M <= sigLen && (reinterpret_cast<uintptr_t>(x + start) & 7u) == 0;
         const float2* xv = reinterpret_cast<const float2*>(x + (direct ? start : 0));
         const float2* wv = reinterpret_cast<const float2*>(window);
-        for (int m = t; m < M; m += T) {
-            float2 z = direct ? ld_reused(xv + m) : make_float2(sample(start + 2 * m), sample(start + 2 * m + 1));
-            if (window) {
-                const float2 w = ld_reused(wv + m);
-                z = make_float2(z.x * w.x, z.y * w.y);
+        constexpr int AHEAD = 4;   // values a thread asks for before it stores the first
+        for (int m0 = t; m0 < M; m0 += AHEAD * T) {
+            float2 z[AHEAD], w[AHEAD];
+#pragma unroll
+            for (int i = 0; i < AHEAD; ++i) {
+                const int m = min(m0 + i * T, M - 1);
+                z[i] = direct ? xv[m] : make_float2(sample(start + 2 * m), sample(start + 2 * m + 1));
+                w[i] = window ? wv[m] : make_float2(1.f, 1.f);
             }
-            buf1[m] = z;
+#pragma unroll
+            for (int i = 0; i < AHEAD; ++i)
+                if (m0 + i * T < M) buf1[m0 + i * T] = make_float2(z[i].x * w[i].x, z[i].y * w[i].y);
         }
     }
     __syncthreads();
@@ -443,7 +448,7 @@ __global__ void __maxnreg__(ROWS::kRegs) k_stft_mixed(const float* __restrict__ 
 template <class ROWS, int VEC>
 __global__ void __maxnreg__(ROWS::kRegs) k_istft_mixed(const float2* __restrict__ spec, float* __restrict__ out,
                                                         const float2* __restrict__ tw, const float2* __restrict__ twr,
-                                                        const float* __restrict__ window, MixedArgs a, uint32_t frames,
+                                                        const float* window, MixedArgs a, uint32_t frames,
                                                         uint32_t hop, uint32_t Q, uint32_t segs, int64_t start,
                                                         uint64_t outLen, float out_scale, int T, int rows, int len) {
     extern __shared__ float2 smem[];
@@ -470,10 +475,10 @@ __global__ void __maxnreg__(ROWS::kRegs) k_istft_mixed(const float2* __restrict_
         __syncthreads();
         seg.wave<VEC, 0>(
             f0, R, reinterpret_cast<const float*>(smem) + finOff * 2, 4 * len,
-            [&](const float* p, int j) { return (window ? ld_reused(window + j) : 1.f) * *p; },
+            [&](const float* p, int j) { return (window ? window[j] : 1.f) * *p; },
             [&](const float* p, int j) {
                 const float4 x = *reinterpret_cast<const float4*>(p);
-                const float4 w = window ? ld_reused(reinterpret_cast<const float4*>(window + j)) : make_float4(1.f, 1.f, 1.f, 1.f);
+                const float4 w = window ? *reinterpret_cast<const float4*>(window + j) : make_float4(1.f, 1.f, 1.f, 1.f);
                 return make_float4(w.x * x.x, w.y * x.y, w.z * x.z, w.w * x.w);
             });
     }
