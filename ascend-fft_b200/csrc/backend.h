@@ -217,11 +217,42 @@ int launchIstftMixed(const void* spec, void* out, const MixedRadix& half, uint64
 // or null for none), R2C of each frame into out[s][f][n/2+1].  n a power of two in
 // [kStftMinN, kStftMaxN]; twr = W_n^k, k <= n/2.
 constexpr uint32_t kStftMinN = 64, kStftMaxN = 8192;
-// Values a thread holds of a frame's n/2-point transform: 32 at 512 and 1024 points, which then take
-// two passes and one exchange instead of three and two (us, 16 and 32: launchStft, 65540 frames of
-// 1024 90.9 / 82.7, 32772 of 2048 97.7 / 84.0; launchIstft, 60008 frames of 1024 70.2 / 59.1).  tw below is
-// the Stockham table (n/2, stftE(n/2)) in all four.
-constexpr int stftE(uint32_t half) { return half == 512 || half == 1024 ? 32 : 16; }
+// Values a thread holds of a frame's n/2-point transform: 16, or 32 at 512 and 1024 points, which then
+// take two passes and one exchange instead of three and two, on half the threads: that pays where the
+// frames are many times what the GPU holds at once, and where the work beside the transform, which has
+// half the threads too, is small.  us with 16 / 32, n = 1024 unless said:
+//   forward, hop 256: 640 frames 4.4 / 4.5, 2560 6.4 / 6.3, 40960 59.6 / 54.8; n = 2048, hop 512: 160 frames 3.9 /
+//     4.2, 1200 6.8 / 6.1; an odd hop gathers sample by sample (hop 129, 40960 frames 63.7 / 75.9);
+//   inverse, hop 256: 640 frames 7.7 / 8.4, 2560 12.9 / 12.4, 40960 88.4 / 78.7; hop 1024, 2560 frames 12.6 / 13.2;
+//     scalar overlap-add: hop 129, 10240 frames 38.5 / 40.5, 20480 70.8 / 66.8, hop 513, 10240 66.6 / 58.7; n = 2048,
+//     20480 frames of hop 512 90.5 / 87.0, of 256 92.5 / 102.8;
+//   gradient of the forward, hop 256: 640 frames 7.1 / 8.6, 5120 17.6 / 16.5, 40960 96.1 / 79.2; hop 1024, 5120
+//     frames 23.6 / 25.0, 20480 68.9 / 65.1; n = 2048, hop 256: 10240 frames 57.2 / 54.1, hop 1024: 20480 109 / 110;
+//   gradient of the inverse: its envelope table and edges are most of it (640 frames 16.4 / 36.4, 40960
+//     78.3 / 113).
+// tw below is the Stockham table (n/2, stftE(the kernel, n, ...)) in all four.
+enum StftKernel { kStftFrames, kIstftFrames, kStftAdjointFrames, kIstftAdjointFrames };
+inline int stftE(StftKernel kernel, uint32_t n, uint64_t signals, uint32_t framesPerSignal, uint32_t hop) {
+    if (n != 1024 && n != 2048) return 16;
+    const uint64_t frames = signals * framesPerSignal;
+    const bool vec = hop % 4 == 0;         // overlap-add by float4
+    const bool half = 2ull * hop <= n;     // every sample in at least two frames
+    const bool quarter = 4ull * hop <= n;  // in at least four
+    bool wide = false;
+    switch (kernel) {
+        case kStftFrames: wide = hop % 2 == 0 && frames >= (n == 1024 ? 2048u : 640u); break;
+        case kIstftFrames:
+            wide = n == 1024 ? frames >= (vec ? (half ? 2048u : 8192u) : 4ull * hop < n ? 16384u : 8192u)
+                             : vec && 4ull * hop >= n && half && frames >= 16384;
+            break;
+        case kStftAdjointFrames:
+            wide = n == 1024 ? frames >= (vec && half ? 4096u : 16384u) && (vec || half)
+                             : vec && quarter && frames >= 8192;
+            break;
+        case kIstftAdjointFrames: break;
+    }
+    return wide ? 32 : 16;
+}
 bool hasStft(uint32_t n);
 int launchStft(const void* sig, void* out, uint32_t n, uint64_t signals, uint32_t framesPerSignal,
                uint64_t sigLen, uint64_t sigStride, uint32_t hop, bool center, const void* window,

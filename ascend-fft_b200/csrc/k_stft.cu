@@ -191,11 +191,11 @@ namespace backend {
 namespace {
 
 // ADJ: the inverse-STFT adjoint (uncentred frames of g / envelope, gStart = the inverse's trim).
-template <int N, bool ADJ = false>
+template <int N, int E, bool ADJ = false>
 int launchStftN(const float* sig, void* out, uint64_t rows, uint32_t framesPerSignal, uint64_t sigLen,
                 uint64_t sigStride, uint32_t hop, bool center, const float* window, const void* tw,
                 const void* twr, void* stream, int64_t gStart = 0, float sEdge = 1.f, float sInt = 1.f) {
-    constexpr int M = N / 2, E = stftE(M), T = M / E;
+    constexpr int M = N / 2, T = M / E;
     constexpr int CTA = T < 4096 / E ? 4096 / E : T;   // at least 4096 values
     constexpr int ROWS = CTA / T;
     constexpr int SMEM = ROWS * dev::smem_stride<M, E, false>() * 8;
@@ -210,10 +210,10 @@ int launchStftN(const float* sig, void* out, uint64_t rows, uint32_t framesPerSi
 }
 
 // ADJ: the STFT adjoint (start = pad = N/2 for a centred STFT, else 0), weights 1 / 1/2, scale 1.
-template <int N, bool ADJ = false>
+template <int N, int E, bool ADJ = false>
 int launchIstftN(const float2* spec, float* out, uint64_t signals, uint32_t frames, uint32_t hop, int64_t start,
                  uint64_t outLen, const float* window, const void* tw, const void* twr, float scale, void* stream) {
-    constexpr int M = N / 2, E = stftE(M), T = M / E;
+    constexpr int M = N / 2, T = M / E;
     constexpr int CTA = T < 4096 / E ? 4096 / E : T;   // at least 4096 values
     constexpr int ROWS = CTA / T;
     constexpr int ROWBYTES = ROWS * dev::istft_row_stride<M, E>() * 8;
@@ -260,19 +260,19 @@ int launchIstftAdjoint(const void* gradOut, void* gradSpec, uint32_t n, uint64_t
     const float* w = static_cast<const float*>(window);
     const uint64_t rows = signals * frames;
     const float c = scale / (float)n;   // irfft's weights: c at DC and Nyquist, 2c between
-#define BFLY_IA(N)                                                                                            \
-    case N:                                                                                                   \
-        return launchStftN<N, true>(g, gradSpec, rows, frames, outLen, outLen, hop, false, w, tw, twr, stream, \
+#define BFLY_IA(N, E)                                                                                            \
+    case N + E:                                                                                                   \
+        return launchStftN<N, E, true>(g, gradSpec, rows, frames, outLen, outLen, hop, false, w, tw, twr, stream, \
                                     start, c, 2.f * c)
-    switch (n) {
-        BFLY_IA(64);
-        BFLY_IA(128);
-        BFLY_IA(256);
-        BFLY_IA(512);
-        BFLY_IA(1024);
-        BFLY_IA(2048);
-        BFLY_IA(4096);
-        BFLY_IA(8192);
+    switch (n + (uint32_t)stftE(kIstftAdjointFrames, n, signals, frames, hop)) {
+        BFLY_IA(64, 16);
+        BFLY_IA(128, 16);
+        BFLY_IA(256, 16);
+        BFLY_IA(512, 16);
+        BFLY_IA(1024, 16);
+        BFLY_IA(2048, 16);
+        BFLY_IA(4096, 16);
+        BFLY_IA(8192, 16);
         default: return (int)cudaErrorInvalidValue;
     }
 #undef BFLY_IA
@@ -287,17 +287,19 @@ int launchStftAdjoint(const void* gradSpec, void* gradSig, uint32_t n, uint64_t 
     float* y = static_cast<float*>(gradSig);
     const float* w = static_cast<const float*>(window);
     const int64_t start = center ? (int64_t)(n / 2) : 0;
-#define BFLY_SA(N) \
-    case N: return launchIstftN<N, true>(x, y, signals, frames, hop, start, sigLen, w, tw, twr, 1.f, stream)
-    switch (n) {
-        BFLY_SA(64);
-        BFLY_SA(128);
-        BFLY_SA(256);
-        BFLY_SA(512);
-        BFLY_SA(1024);
-        BFLY_SA(2048);
-        BFLY_SA(4096);
-        BFLY_SA(8192);
+#define BFLY_SA(N, E) \
+    case N + E: return launchIstftN<N, E, true>(x, y, signals, frames, hop, start, sigLen, w, tw, twr, 1.f, stream)
+    switch (n + (uint32_t)stftE(kStftAdjointFrames, n, signals, frames, hop)) {
+        BFLY_SA(64, 16);
+        BFLY_SA(128, 16);
+        BFLY_SA(256, 16);
+        BFLY_SA(512, 16);
+        BFLY_SA(1024, 16);
+        BFLY_SA(1024, 32);
+        BFLY_SA(2048, 16);
+        BFLY_SA(2048, 32);
+        BFLY_SA(4096, 16);
+        BFLY_SA(8192, 16);
         default: return (int)cudaErrorInvalidValue;
     }
 #undef BFLY_SA
@@ -336,17 +338,19 @@ int launchStft(const void* sig, void* out, uint32_t n, uint64_t signals, uint32_
     const float* x = static_cast<const float*>(sig);
     const float* w = static_cast<const float*>(window);
     const uint64_t rows = signals * framesPerSignal;
-#define BFLY_ST(N) \
-    case N: return launchStftN<N>(x, out, rows, framesPerSignal, sigLen, sigStride, hop, center, w, tw, twr, stream)
-    switch (n) {
-        BFLY_ST(64);
-        BFLY_ST(128);
-        BFLY_ST(256);
-        BFLY_ST(512);
-        BFLY_ST(1024);
-        BFLY_ST(2048);
-        BFLY_ST(4096);
-        BFLY_ST(8192);
+#define BFLY_ST(N, E) \
+    case N + E: return launchStftN<N, E>(x, out, rows, framesPerSignal, sigLen, sigStride, hop, center, w, tw, twr, stream)
+    switch (n + (uint32_t)stftE(kStftFrames, n, signals, framesPerSignal, hop)) {
+        BFLY_ST(64, 16);
+        BFLY_ST(128, 16);
+        BFLY_ST(256, 16);
+        BFLY_ST(512, 16);
+        BFLY_ST(1024, 16);
+        BFLY_ST(1024, 32);
+        BFLY_ST(2048, 16);
+        BFLY_ST(2048, 32);
+        BFLY_ST(4096, 16);
+        BFLY_ST(8192, 16);
         default: return (int)cudaErrorInvalidValue;
     }
 #undef BFLY_ST
@@ -359,17 +363,19 @@ int launchIstft(const void* spec, void* out, uint32_t n, uint64_t signals, uint3
     const float2* x = static_cast<const float2*>(spec);
     float* y = static_cast<float*>(out);
     const float* w = static_cast<const float*>(window);
-#define BFLY_IS(N) \
-    case N: return launchIstftN<N>(x, y, signals, frames, hop, start, outLen, w, tw, twr, scale, stream)
-    switch (n) {
-        BFLY_IS(64);
-        BFLY_IS(128);
-        BFLY_IS(256);
-        BFLY_IS(512);
-        BFLY_IS(1024);
-        BFLY_IS(2048);
-        BFLY_IS(4096);
-        BFLY_IS(8192);
+#define BFLY_IS(N, E) \
+    case N + E: return launchIstftN<N, E>(x, y, signals, frames, hop, start, outLen, w, tw, twr, scale, stream)
+    switch (n + (uint32_t)stftE(kIstftFrames, n, signals, frames, hop)) {
+        BFLY_IS(64, 16);
+        BFLY_IS(128, 16);
+        BFLY_IS(256, 16);
+        BFLY_IS(512, 16);
+        BFLY_IS(1024, 16);
+        BFLY_IS(1024, 32);
+        BFLY_IS(2048, 16);
+        BFLY_IS(2048, 32);
+        BFLY_IS(4096, 16);
+        BFLY_IS(8192, 16);
         default: return (int)cudaErrorInvalidValue;
     }
 #undef BFLY_IS

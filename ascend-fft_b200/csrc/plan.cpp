@@ -875,9 +875,10 @@ int Plan::execStft(const void* dSig, void* dOut, uint32_t n, uint64_t signals, u
             return -5;
         return 0;
     }
-    if (prepareC2C(n / 2, backend::stftE(n / 2)) || prepareReal(n)) return -2;
+    const int e = backend::stftE(backend::kStftFrames, n, signals, (uint32_t)frames, hop);
+    if (prepareC2C(n / 2, e) || prepareReal(n)) return -2;
     if (backend::launchStft(dSig, dOut, n, signals, (uint32_t)frames, sigLen, sigLen, hop, center, dWindow,
-                            impl_->twC2C[{n / 2, backend::stftE(n / 2)}], impl_->twReal[n], stream))
+                            impl_->twC2C[{n / 2, e}], impl_->twReal[n], stream))
         return -5;
     return 0;
 }
@@ -889,9 +890,10 @@ int Plan::execStftBackward(const void* dGradSpec, void* dGradSig, uint32_t n, ui
     if (center ? sigLen < (uint64_t)n + 2 : sigLen < n) return -8;
     const uint64_t frames = center ? 1 + sigLen / hop : 1 + (sigLen - n) / hop;
     if (frames > 0xFFFFFFFFull || signals > 0xFFFFFFFFull / frames) return -8;
-    if (prepareC2C(n / 2, backend::stftE(n / 2)) || prepareReal(n)) return -2;
+    const int e = backend::stftE(backend::kStftAdjointFrames, n, signals, (uint32_t)frames, hop);
+    if (prepareC2C(n / 2, e) || prepareReal(n)) return -2;
     if (backend::launchStftAdjoint(dGradSpec, dGradSig, n, signals, (uint32_t)frames, hop, center, sigLen, dWindow,
-                                   impl_->twC2C[{n / 2, backend::stftE(n / 2)}], impl_->twReal[n], stream))
+                                   impl_->twC2C[{n / 2, e}], impl_->twReal[n], stream))
         return -5;
     return 0;
 }
@@ -904,9 +906,10 @@ int Plan::execIstftBackward(const void* dGradOut, void* dGradSpec, uint32_t n, u
         return -8;
     if (signals > 0xFFFFFFFFull / frames || outLen == 0 || outLen > (1ull << 62)) return -8;
     if (reinterpret_cast<uintptr_t>(dWindow) & 7u) return -8;
-    if (prepareC2C(n / 2, backend::stftE(n / 2)) || prepareReal(n)) return -2;
+    const int e = backend::stftE(backend::kIstftAdjointFrames, n, signals, frames, hop);
+    if (prepareC2C(n / 2, e) || prepareReal(n)) return -2;
     if (backend::launchIstftAdjoint(dGradOut, dGradSpec, n, signals, frames, hop, center ? (int64_t)(n / 2) : 0,
-                                    outLen, dWindow, impl_->twC2C[{n / 2, backend::stftE(n / 2)}], impl_->twReal[n], scale, stream))
+                                    outLen, dWindow, impl_->twC2C[{n / 2, e}], impl_->twReal[n], scale, stream))
         return -5;
     return 0;
 }
@@ -927,9 +930,10 @@ int Plan::execIstft(const void* dSpec, void* dOut, uint32_t n, uint64_t signals,
             return -5;
         return 0;
     }
-    if (prepareC2C(n / 2, backend::stftE(n / 2)) || prepareReal(n)) return -2;
+    const int e = backend::stftE(backend::kIstftFrames, n, signals, frames, hop);
+    if (prepareC2C(n / 2, e) || prepareReal(n)) return -2;
     if (backend::launchIstft(dSpec, dOut, n, signals, frames, hop, center ? (int64_t)(n / 2) : 0, outLen, dWindow,
-                             impl_->twC2C[{n / 2, backend::stftE(n / 2)}], impl_->twReal[n], scale, stream))
+                             impl_->twC2C[{n / 2, e}], impl_->twReal[n], scale, stream))
         return -5;
     return 0;
 }
