@@ -56,7 +56,8 @@ k_c2c(const float2* __restrict__ in, float2* __restrict__ out, const float2* __r
     float2 v[E];
     TM::load_first(v, t, [&](int i) { return ok ? ld_once_ca(src + i) : make_float2(0.f, 0.f); });
     constexpr unsigned AHEAD = prefetch_ahead(min_blocks<E>(T * ROWS));
-    if (blockIdx.x + AHEAD < gridDim.x)
+    // (rows of 32 fill the memory pipeline by themselves: 524288 of them 55.5 us with, 53.5 without)
+    if (N > 32 && blockIdx.x + AHEAD < gridDim.x)
         prefetch_span<ROWS * N * 8, T * ROWS>(in + ((uint64_t)blockIdx.x + AHEAD) * (ROWS * N), in + batch * N);
     TM::template passes<0>(v, smem + rl * S, tw, t, rl);
     pdl_trigger();

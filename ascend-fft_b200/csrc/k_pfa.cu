@@ -160,7 +160,9 @@ k_pfa(const float2* __restrict__ in, float2* __restrict__ out, const float2* __r
         }
     }
     __syncthreads();
-    pdl_trigger();
+    // no early trigger: with one the next launch's CTAs double up beside this one's on the SMs that have
+    // room first, which costs launches of about one wave more than the earlier start gives (us without a
+    // dependent launch / with the trigger here: n = 7680 x 137 rows 9.0 / 10.1, 48 x 21846 7.7 / 8.7)
     // 4. coalesced stores of X[k] = Y[k1][k2]; across lanes k2 steps by the odd A^-1 mod B,
     //    a permutation of the banks
     if (ok) {
