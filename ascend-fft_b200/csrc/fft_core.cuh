@@ -533,8 +533,9 @@ struct Team {
 // on its stream drains: pdl_wait(), before a kernel's first global access, blocks until the
 // previous grid has finished and its writes are visible, so a chain of such launches overlaps
 // only launch latency, never data; pdl_trigger(), just before a CTA's final stores, lets the
-// next kernel launch once every CTA of this grid has reached that point (triggering at entry
-// placed the next grid's CTAs beside this one's and unbalanced one-wave launches).  Without
+// next kernel launch once every CTA of this grid has reached that point or ended (triggering at entry
+// placed the next grid's CTAs beside this one's and unbalanced one-wave launches; k_pfa and the
+// mixed-radix C2C kernels have no trigger).  Without
 // the launch attribute both are no-ops.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -566,7 +567,7 @@ __device__ __forceinline__ void st_stream(float2* p, float2 v) { __stcs(p, v); }
 // residency costs 1-5 % of the gain and 1.5 residencies most of it.  Plain launches, 2^25 points,
 // without and with: k_c2c n = 4096: 6178 -> 6300 GB/s, 8192: 5049 -> 5433, 16384: 3755 -> 4322;
 // k_cols NY = 512: 5798 -> 6410, 1024: 4002 -> 4928.  The fewer CTAs share an SM, the more it
-// gives.  kSms sets a distance only.
+// gives.  kSms sets this distance, and the grid and least size of k_staged: no result depends on it.
 constexpr unsigned kSms = 148;
 __host__ __device__ constexpr unsigned prefetch_ahead(int perSm) { return perSm * kSms / 2; }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }

@@ -80,7 +80,7 @@ MixedShape mixedShape(const MixedRadix& plan) {
     m.args = mixedArgs(plan);
     // about one butterfly of the largest radix per thread and pass (more of the smaller radices);
     // measured on B200 over n = 12..12000: n / R_max threads per row with ~200-300 threads per CTA
-    // beat n/8 threads per row, larger CTAs, and an 80-register budget
+    // beat n/8 threads per row and larger CTAs (registers: GenericRows::kRegs)
     for (int p = 0; p < plan.passes; ++p)
         m.cls = std::max(m.cls, plan.radix[p] == 11 || plan.radix[p] == 13 ? 2 : plan.radix[p] > 10 ? 1 : 0);
     m.T = dev::mixedThreads(plan.n, plan.radix, plan.passes);

@@ -1,5 +1,5 @@
-// C2C of n = A*B (A in {3, 5, 9, 15}, B a power of two >= 16, n <= 12288) by the Good-Thomas
-// prime-factor mapping, one HBM pass.  With gcd(A, B) = 1,
+// C2C of n = A*B (A in {3, 5, 9, 15}, B a power of two >= 16, n <= 12288, of these the lengths that
+// pfaTaken() names) by the Good-Thomas prime-factor mapping, one HBM pass.  With gcd(A, B) = 1,
 //   input  j <-> (j1, j2) = (j mod A, j mod B)          (Chinese-remainder map)
 //   output k  =  (B*k1 + A*k2) mod n                     (Ruritanian map)
 // gives W_n^(j*k) = W_A^(j1*k1) * W_B^(j2*k2), so the n-point DFT is an A x B two-dimensional

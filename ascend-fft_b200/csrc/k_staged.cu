@@ -131,7 +131,10 @@ int launchStaged(const float2* in, float2* out, const float2* tw, uint64_t strip
 }
 }  // namespace
 
-// Taken for strips enough to have a next one on every SM, with rows on 16-byte boundaries.
+// Taken from the first strip past one per SM on, with rows on 16-byte boundaries: with a second round
+// most SMs have a next strip or idle through it either way.  us, k_cols of 16 values a thread and this:
+// NY = 2048: 149 strips 24.1 / 21.6, 296 27.9 / 25.5, 297 36.2 / 32.3, 1100 103.7 / 89.4; 4096: 149 34.8 / 24.4,
+// 296 39.5 / 28.4, 1100 156 / 108.  148 strips, k_cols both: 14.4 / 13.8 and 20.1 / 20.1.
 bool launchColsStaged(const void* in, void* out, uint32_t ny, uint32_t ncols, uint64_t pitch, uint64_t matStride,
                       uint64_t mats, bool inverse, float scale, const void* tw, void* stream, int* rc) {
     if ((ny != 2048 && ny != 4096) || reinterpret_cast<uintptr_t>(in) % 16 || pitch % 2 || matStride % 2) return false;

@@ -1,6 +1,7 @@
 // Kernel launch with programmatic stream serialisation (programmatic dependent launch): the
-// kernel may begin launching while the previous kernel on the stream drains; kernels launched
-// this way call pdl_trigger() and pdl_wait() (fft_core.cuh) before their first global access.
+// kernel may begin launching while the previous kernel on the stream drains; every kernel launched
+// this way calls pdl_wait() before its first global access, and most call pdl_trigger() before their
+// last stores (fft_core.cuh).
 // BFLY_PDL=0 in the environment launches them plainly instead (read once per process).
 #pragma once
 #include <cuda_runtime.h>
