@@ -14,6 +14,7 @@
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/custom_class.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/utils/pybind.h>
 
@@ -321,15 +322,22 @@ Tensor istftOf(const Tensor& spec, int64_t n, int64_t hop, bool center, const Ma
 Tensor stftAdjoint(const Tensor& g, int64_t n, int64_t hop, bool center, const Maybe& w, int64_t length);
 Tensor istftAdjoint(const Tensor& g, int64_t n, int64_t hop, bool center, const Maybe& w, int64_t frames, double scale);
 
-int64_t savedInt(AutogradContext* c, const char* k) { return c->saved_data[k].toInt(); }
-double savedDouble(AutogradContext* c, const char* k) { return c->saved_data[k].toDouble(); }
-// What the four nodes of the short-time transforms keep; `size`: the signal's length or the frames.
+// What a node keeps for its backward pass, in one entry of saved_data: each entry is a string, a hash and
+// an allocation (rfft of 1024 rows of 4096 with its gradient: 52.0 us with an entry per value, 50.0 so).
+struct Saved : torch::CustomClassHolder {
+    int64_t n = 0, hop = 0, size = 0, direction = 0;   // n: length or dimension; size: signal length or frames
+    double scale = 1.0, edge = 1.0, inside = 1.0;
+    bool center = false;
+};
+void save(AutogradContext* ctx, Saved s) {
+    ctx->saved_data["p"] = c10::IValue::make_capsule(c10::make_intrusive<Saved>(std::move(s)));
+}
+Saved saved(AutogradContext* ctx) { return static_cast<const Saved&>(*ctx->saved_data["p"].toCapsule()); }
+// The nodes of the short-time transforms keep their window too.
 void saveFrames(AutogradContext* ctx, const Maybe& w, int64_t n, int64_t hop, bool center, int64_t size, double scale) {
-    ctx->saved_data["n"] = n;
-    ctx->saved_data["hop"] = hop;
-    ctx->saved_data["center"] = center;
-    ctx->saved_data["size"] = size;
-    ctx->saved_data["scale"] = scale;
+    Saved s;
+    s.n = n, s.hop = hop, s.size = size, s.scale = scale, s.center = center;
+    save(ctx, s);
     ctx->save_for_backward({w.value_or(Tensor())});
 }
 Maybe savedWindow(AutogradContext* ctx) {
@@ -339,74 +347,78 @@ Maybe savedWindow(AutogradContext* ctx) {
 
 struct C2CNode : Function<C2CNode> {   // dim: the transformed dimension
     static Tensor forward(AutogradContext* ctx, const Tensor& x, int64_t dim, int64_t direction, double scale) {
-        ctx->saved_data["dim"] = dim;
-        ctx->saved_data["direction"] = direction;
-        ctx->saved_data["scale"] = scale;
+        Saved s;
+        s.n = dim, s.direction = direction, s.scale = scale;
+        save(ctx, s);
         return execAxis(x, dim, direction, scale);
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-        return {c2cAxis(g[0], savedInt(ctx, "dim"), -savedInt(ctx, "direction"), savedDouble(ctx, "scale")), Tensor(),
-                Tensor(), Tensor()};
+        const Saved s = saved(ctx);
+        return {c2cAxis(g[0], s.n, -s.direction, s.scale), Tensor(), Tensor(), Tensor()};
     }
 };
 
 struct C2C2DNode : Function<C2C2DNode> {
     static Tensor forward(AutogradContext* ctx, const Tensor& x, int64_t direction, double scale) {
-        ctx->saved_data["direction"] = direction;
-        ctx->saved_data["scale"] = scale;
+        Saved s;
+        s.direction = direction, s.scale = scale;
+        save(ctx, s);
         return exec2D(x, direction, scale);
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-        return {c2c2D(g[0], -savedInt(ctx, "direction"), savedDouble(ctx, "scale")), Tensor(), Tensor()};
+        const Saved s = saved(ctx);
+        return {c2c2D(g[0], -s.direction, s.scale), Tensor(), Tensor()};
     }
 };
 
 struct R2CNode : Function<R2CNode> {
     static Tensor forward(AutogradContext* ctx, const Tensor& x, double scale, double edge, double inside) {
-        ctx->saved_data["scale"] = scale;
-        ctx->saved_data["edge"] = edge;
-        ctx->saved_data["inside"] = inside;
-        ctx->saved_data["n"] = x.size(-1);
+        Saved s;
+        s.n = x.size(-1), s.scale = scale, s.edge = edge, s.inside = inside;
+        save(ctx, s);
         return execR2C(x, scale * edge, scale * inside);
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-        return {c2r(g[0], savedInt(ctx, "n"), savedDouble(ctx, "scale"), savedDouble(ctx, "edge"),
-                    0.5 * savedDouble(ctx, "inside")),
-                Tensor(), Tensor(), Tensor()};
+        const Saved s = saved(ctx);
+        return {c2r(g[0], s.n, s.scale, s.edge, 0.5 * s.inside), Tensor(), Tensor(), Tensor()};
     }
 };
 
 struct C2RNode : Function<C2RNode> {
     static Tensor forward(AutogradContext* ctx, const Tensor& x, int64_t n, double scale, double edge, double inside) {
-        ctx->saved_data["scale"] = scale;
-        ctx->saved_data["edge"] = edge;
-        ctx->saved_data["inside"] = inside;
+        Saved s;
+        s.scale = scale, s.edge = edge, s.inside = inside;
+        save(ctx, s);
         return execC2R(x, n, edge, inside, scale);
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-        return {r2c(g[0], savedDouble(ctx, "scale"), savedDouble(ctx, "edge"), 2.0 * savedDouble(ctx, "inside")),
-                Tensor(), Tensor(), Tensor(), Tensor()};
+        const Saved s = saved(ctx);
+        return {r2c(g[0], s.scale, s.edge, 2.0 * s.inside), Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
 
 struct R2C2DNode : Function<R2C2DNode> {
     static Tensor forward(AutogradContext* ctx, const Tensor& x, double scale) {
-        ctx->saved_data["scale"] = scale;
-        ctx->saved_data["nx"] = x.size(-1);
+        Saved s;
+        s.n = x.size(-1), s.scale = scale;
+        save(ctx, s);
         return execR2C2D(x, scale);
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-        return {c2r(c2cAxis(g[0], -2, 1, 1.0), savedInt(ctx, "nx"), savedDouble(ctx, "scale"), 1.0, 0.5), Tensor()};
+        const Saved s = saved(ctx);
+        return {c2r(c2cAxis(g[0], -2, 1, 1.0), s.n, s.scale, 1.0, 0.5), Tensor()};
     }
 };
 
 struct C2R2DNode : Function<C2R2DNode> {
     static Tensor forward(AutogradContext* ctx, const Tensor& x, int64_t nx, double scale) {
-        ctx->saved_data["scale"] = scale;
+        Saved s;
+        s.scale = scale;
+        save(ctx, s);
         return execC2R2D(x, nx, scale);
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-        return {c2cAxis(r2c(g[0], savedDouble(ctx, "scale"), 1.0, 2.0), -2, -1, 1.0), Tensor(), Tensor()};
+        return {c2cAxis(r2c(g[0], saved(ctx).scale, 1.0, 2.0), -2, -1, 1.0), Tensor(), Tensor()};
     }
 };
 
@@ -417,9 +429,8 @@ struct StftNode : Function<StftNode> {
         return execStft(x, n, hop, center, w.value_or(Tensor()));
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-        return {stftAdjoint(g[0], savedInt(ctx, "n"), savedInt(ctx, "hop"), ctx->saved_data["center"].toBool(),
-                            savedWindow(ctx), savedInt(ctx, "size")),
-                Tensor(), Tensor(), Tensor(), Tensor()};
+        const Saved s = saved(ctx);
+        return {stftAdjoint(g[0], s.n, s.hop, s.center, savedWindow(ctx), s.size), Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
 
@@ -430,9 +441,9 @@ struct StftAdjointNode : Function<StftAdjointNode> {
         return execStftAdjoint(g, n, hop, center, w.value_or(Tensor()), length);
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& h) {
-        return {stftOf(dense(h[0]), savedInt(ctx, "n"), savedInt(ctx, "hop"), ctx->saved_data["center"].toBool(),
-                       savedWindow(ctx)),
-                Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+        const Saved s = saved(ctx);
+        return {stftOf(dense(h[0]), s.n, s.hop, s.center, savedWindow(ctx)), Tensor(), Tensor(), Tensor(), Tensor(),
+                Tensor()};
     }
 };
 
@@ -443,9 +454,9 @@ struct IstftNode : Function<IstftNode> {
         return execIstft(spec, n, hop, center, w.value_or(Tensor()), outLen, scale);
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& g) {
-        return {istftAdjoint(g[0], savedInt(ctx, "n"), savedInt(ctx, "hop"), ctx->saved_data["center"].toBool(),
-                             savedWindow(ctx), savedInt(ctx, "size"), savedDouble(ctx, "scale")),
-                Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+        const Saved s = saved(ctx);
+        return {istftAdjoint(g[0], s.n, s.hop, s.center, savedWindow(ctx), s.size, s.scale), Tensor(), Tensor(), Tensor(),
+                Tensor(), Tensor(), Tensor()};
     }
 };
 
@@ -456,9 +467,9 @@ struct IstftAdjointNode : Function<IstftAdjointNode> {
         return execIstftAdjoint(g, n, hop, center, w.value_or(Tensor()), frames, scale);
     }
     static variable_list backward(AutogradContext* ctx, const variable_list& h) {
-        return {istftOf(dense(h[0]), savedInt(ctx, "n"), savedInt(ctx, "hop"), ctx->saved_data["center"].toBool(),
-                        savedWindow(ctx), savedInt(ctx, "size"), savedDouble(ctx, "scale")),
-                Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+        const Saved s = saved(ctx);
+        return {istftOf(dense(h[0]), s.n, s.hop, s.center, savedWindow(ctx), s.size, s.scale), Tensor(), Tensor(), Tensor(),
+                Tensor(), Tensor(), Tensor()};
     }
 };
 
