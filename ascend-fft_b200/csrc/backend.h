@@ -232,8 +232,9 @@ constexpr uint32_t kStftMinN = 64, kStftMaxN = 8192;
 //     78.3 / 113).
 // tw below is the Stockham table (n/2, stftE(the kernel, n, ...)) in all four.
 enum StftKernel { kStftFrames, kIstftFrames, kStftAdjointFrames, kIstftAdjointFrames };
+inline bool stftMayWiden(uint32_t n) { return n == 1024 || n == 2048; }
 inline int stftE(StftKernel kernel, uint32_t n, uint64_t signals, uint32_t framesPerSignal, uint32_t hop) {
-    if (n != 1024 && n != 2048) return 16;
+    if (!stftMayWiden(n)) return 16;
     const uint64_t frames = signals * framesPerSignal;
     const bool vec = hop % 4 == 0;         // overlap-add by float4
     const bool half = 2ull * hop <= n;     // every sample in at least two frames

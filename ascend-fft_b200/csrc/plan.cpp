@@ -586,6 +586,14 @@ int Plan::prepareReal(uint32_t n) {
     return 0;
 }
 
+// Tables of the short-time transforms of a power of two n: of every count of values a thread that stftE
+// may choose, so that a captured call needs no more than an earlier one of its length has built.
+int Plan::prepareFrames(uint32_t n) {
+    for (int e : {16, 32})
+        if ((e == 16 || backend::stftMayWiden(n)) && prepareC2C(n / 2, e)) return -1;
+    return prepareReal(n);
+}
+
 int Plan::prepareLong(uint32_t n) {
     uint32_t n1 = 0, n2 = 0;
     backend::longSplit(n, &n1, &n2);
@@ -876,7 +884,7 @@ int Plan::execStft(const void* dSig, void* dOut, uint32_t n, uint64_t signals, u
         return 0;
     }
     const int e = backend::stftE(backend::kStftFrames, n, signals, (uint32_t)frames, hop);
-    if (prepareC2C(n / 2, e) || prepareReal(n)) return -2;
+    if (prepareFrames(n)) return -2;
     if (backend::launchStft(dSig, dOut, n, signals, (uint32_t)frames, sigLen, sigLen, hop, center, dWindow,
                             impl_->twC2C[{n / 2, e}], impl_->twReal[n], stream))
         return -5;
@@ -891,7 +899,7 @@ int Plan::execStftBackward(const void* dGradSpec, void* dGradSig, uint32_t n, ui
     const uint64_t frames = center ? 1 + sigLen / hop : 1 + (sigLen - n) / hop;
     if (frames > 0xFFFFFFFFull || signals > 0xFFFFFFFFull / frames) return -8;
     const int e = backend::stftE(backend::kStftAdjointFrames, n, signals, (uint32_t)frames, hop);
-    if (prepareC2C(n / 2, e) || prepareReal(n)) return -2;
+    if (prepareFrames(n)) return -2;
     if (backend::launchStftAdjoint(dGradSpec, dGradSig, n, signals, (uint32_t)frames, hop, center, sigLen, dWindow,
                                    impl_->twC2C[{n / 2, e}], impl_->twReal[n], stream))
         return -5;
@@ -907,7 +915,7 @@ int Plan::execIstftBackward(const void* dGradOut, void* dGradSpec, uint32_t n, u
     if (signals > 0xFFFFFFFFull / frames || outLen == 0 || outLen > (1ull << 62)) return -8;
     if (reinterpret_cast<uintptr_t>(dWindow) & 7u) return -8;
     const int e = backend::stftE(backend::kIstftAdjointFrames, n, signals, frames, hop);
-    if (prepareC2C(n / 2, e) || prepareReal(n)) return -2;
+    if (prepareFrames(n)) return -2;
     if (backend::launchIstftAdjoint(dGradOut, dGradSpec, n, signals, frames, hop, center ? (int64_t)(n / 2) : 0,
                                     outLen, dWindow, impl_->twC2C[{n / 2, e}], impl_->twReal[n], scale, stream))
         return -5;
@@ -931,7 +939,7 @@ int Plan::execIstft(const void* dSpec, void* dOut, uint32_t n, uint64_t signals,
         return 0;
     }
     const int e = backend::stftE(backend::kIstftFrames, n, signals, frames, hop);
-    if (prepareC2C(n / 2, e) || prepareReal(n)) return -2;
+    if (prepareFrames(n)) return -2;
     if (backend::launchIstft(dSpec, dOut, n, signals, frames, hop, center ? (int64_t)(n / 2) : 0, outLen, dWindow,
                              impl_->twC2C[{n / 2, e}], impl_->twReal[n], scale, stream))
         return -5;

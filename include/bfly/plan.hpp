@@ -312,6 +312,7 @@ private:
     bool validShape(uint32_t n, uint32_t batch, int kind) const;
     int prepareC2C(uint32_t n, int e);
     int prepareReal(uint32_t n);
+    int prepareFrames(uint32_t n);
     int prepareLong(uint32_t n);
     int prepareDirect(uint32_t n);
     int prepareBluestein(uint32_t n);

@@ -47,3 +47,34 @@ def test_against_fp64(cuda, n, hop, frames, signals):
     got = torch.autograd.grad(z, X, gz)[0]
     want = torch.autograd.grad(zr, Xd, gz.double())[0]
     assert _rel(torch, got, want) <= 1e-5
+
+
+@pytest.mark.parametrize("n", [1024, 2048])
+def test_capture_on_the_other_side(ctx, cuda, n):
+    """A call with few frames is all the warm-up that a captured one with many needs, on every kernel."""
+    import torch
+    plan = ctx.make_plan()
+    hop, few, many = n // 4, 40, 20000
+    w = torch.hann_window(n, device=cuda)
+    x = torch.randn(1, hop * (many - 1), device=cuda)
+    spec = torch.empty(1, many, n // 2 + 1, dtype=torch.complex64, device=cuda)
+    y, gx, gs = torch.empty_like(x), torch.empty_like(x), torch.empty_like(spec)
+
+    def run(frames, s):
+        length = hop * (frames - 1)
+        assert plan.exec_stft(x.data_ptr(), spec.data_ptr(), n, 1, length, hop, True, w.data_ptr(), s)[0] == 0
+        assert plan.exec_istft(spec.data_ptr(), y.data_ptr(), n, 1, frames, hop, True, w.data_ptr(), length, 1.0, s) == 0
+        assert plan.exec_stft_backward(spec.data_ptr(), gx.data_ptr(), n, 1, length, hop, True, w.data_ptr(), s) == 0
+        assert plan.exec_istft_backward(x.data_ptr(), gs.data_ptr(), n, 1, frames, hop, True, w.data_ptr(), length, 1.0,
+                                        s) == 0
+
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        run(few, stream.cuda_stream)
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            run(many, stream.cuda_stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert ((y - x).norm() / x.norm()).item() <= 2e-6
