@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -14,6 +15,7 @@ struct bfly_context {
 };
 struct bfly_plan {
     std::unique_ptr<bfly::Plan> plan;
+    std::mutex turn;   // held by a call: a plan builds tables and grows workspaces at first use
 };
 struct bfly_ragged {
     std::unique_ptr<bfly::Ragged> ragged;
@@ -115,6 +117,7 @@ int bfly_plan_candidate_id(bfly_plan* plan, char* buf, size_t cap) {
 
 #define PLAN_OR_FAIL()                  \
     if (!plan || !plan->plan) return -10; \
+    std::lock_guard<std::mutex> turn(plan->turn); \
     bfly::Plan& p = *plan->plan
 
 int bfly_plan_prepare(bfly_plan* plan, uint32_t n, uint32_t batch) {
@@ -267,6 +270,7 @@ int bfly_ragged_create(bfly_plan* plan, const bfly_ragged_request* reqs, size_t 
     if (!reqs || count == 0) return -8;
     const auto rs = raggedRequests(reqs, count);
     int status = 0;
+    std::lock_guard<std::mutex> turn(plan->turn);
     auto r = plan->plan->makeRagged(rs.data(), count, &status);
     if (!r) return status ? status : -1;
     *out = new bfly_ragged{std::move(r)};
@@ -283,6 +287,7 @@ int bfly_ragged_create_config(bfly_plan* plan, const bfly_ragged_request* reqs, 
     cfg.mode = mode;
     cfg.radix8 = radix8;
     int status = 0;
+    std::lock_guard<std::mutex> turn(plan->turn);
     auto r = plan->plan->makeRagged(rs.data(), count, &status, &cfg);
     if (!r) return status ? status : -1;
     *out = new bfly_ragged{std::move(r)};
@@ -297,6 +302,7 @@ int bfly_context_tune_ragged(bfly_context* ctx, bfly_plan* plan, const bfly_ragg
     const auto rs = raggedRequests(reqs, count);
     std::string text;
     int status = 0;
+    std::lock_guard<std::mutex> turn(plan->turn);
     auto r = ctx->ctx.tuneRagged(*plan->plan, rs.data(), count, &status, log ? &text : nullptr);
     if (log) copyOut(text, log, log_cap, nullptr);
     if (!r) return status ? status : -1;

@@ -12,7 +12,9 @@
  *
  * Layouts: complex data is interleaved fp32 [re, im]; C2C rows are [batch][2n] floats,
  * R2C output / C2R input rows are [batch][n+2] floats (n/2+1 complex bins).
- * Threading: one thread at a time per plan; a context owns one CUDA stream.
+ * Threading: calls on one plan take turns, since a plan builds tables at the first use of a length;
+ * a context owns one CUDA stream.  Work that a call leaves in a plan-owned workspace (four_step and
+ * ring schedules, exec_c2r_2d) is ordered by its stream: put such calls of one plan on one stream.
  */
 #ifndef BFLY_B200_H
 #define BFLY_B200_H
