@@ -630,14 +630,12 @@ class _IRFFT2(torch.autograd.Function):
         if X.shape[-1] != nx // 2 + 1:
             raise ValueError(f"irfft2: last dimension {X.shape[-1]} != nx/2+1 = {nx // 2 + 1}")
         batch = X.numel() // (ny * X.shape[-1]) if X.numel() else 0
-        y = torch.empty(*X.shape[:-1], nx, dtype=torch.float32, device=X.device)
         ctx.scale = scale
         if batch == 0:
-            return y
-        rc = plan_for(X.device, nx, "real").exec_c2r_2d(X.data_ptr(), y.data_ptr(), ny, nx, batch, scale, _stream(X))
-        if rc:
-            raise BflyError(f"exec_c2r_2d(ny={ny}, nx={nx}, batch={batch})", rc)
-        return y
+            return torch.empty(*X.shape[:-1], nx, dtype=torch.float32, device=X.device)
+        # the column pass goes to a tensor of the call's own: the plan's buffer (exec_c2r_2d) would be
+        # shared with calls on other streams and with captured graphs
+        return c2r(c2c_axis(X, -2, 1, 1.0), nx, 1.0, 1.0, scale)
 
     @staticmethod
     def backward(ctx, g):

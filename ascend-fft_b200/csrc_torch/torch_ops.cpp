@@ -238,18 +238,10 @@ Tensor execR2C2D(const Tensor& in, double scale) {
     return y;
 }
 
+// The column pass goes to a tensor of the call's own, not to the plan's buffer (exec_c2r_2d's), which
+// calls on other streams and captured graphs would share.
 Tensor execC2R2D(const Tensor& in, int64_t nx, double scale) {
-    const Tensor x = dense(in);
-    const int64_t ny = x.size(-2);
-    Tensor y = emptyLast(x, nx, at::kFloat);
-    if (!x.numel()) return y;
-    const int64_t batch = x.numel() / (ny * x.size(-1));
-    const Plan p = planFor(x.get_device(), true, nx);
-    check(bfly_plan_exec_c2r_2d_async(p->plan, x.data_ptr(), y.data_ptr(), (uint32_t)ny, (uint32_t)nx,
-                                      (uint64_t)batch, (float)scale, streamOf(x)),
-          "exec_c2r_2d(ny=" + std::to_string(ny) + ", nx=" + std::to_string(nx) + ", batch=" +
-              std::to_string(batch) + ")");
-    return y;
+    return execC2R(execAxis(in, -2, 1, 1.0), nx, 1.0, 1.0, scale);
 }
 
 const void* windowPtr(const Tensor& w) { return w.defined() ? w.data_ptr() : nullptr; }
