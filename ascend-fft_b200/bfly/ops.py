@@ -43,7 +43,7 @@ from . import _lib
 from .core import DEFAULT_CANDIDATE, BflyError, Context
 
 _native = _lib.load_torch_ops()
-_NORM = {"backward": 0, "ortho": 1, "forward": 2}
+_NORM = {None: 0, "backward": 0, "ortho": 1, "forward": 2}
 
 _lock = threading.Lock()
 _state = {}   # device index -> {"ctx": Context, "plans": {candidate id: Plan}, "tuned": {...}}
@@ -140,11 +140,12 @@ def _stream(t: torch.Tensor) -> int:
 
 
 def _norm_code(norm: str | None) -> int:
-    norm = norm or "backward"
-    code = _NORM.get(norm) if isinstance(norm, str) else None
-    if code is None:
-        raise ValueError(f"invalid norm {norm!r}")
-    return code
+    try:
+        return _NORM[norm]
+    except (KeyError, TypeError):
+        if not norm:   # "", False, 0
+            return 0
+    raise ValueError(f"invalid norm {norm!r}")
 
 
 def _scale(norm: str | None, n: int, forward: bool) -> float:

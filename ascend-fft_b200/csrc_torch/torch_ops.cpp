@@ -114,8 +114,7 @@ void bind(py::object find, py::object error) {
     table().error = error.release().ptr();
 }
 
-void check(int rc, const std::string& what) {
-    if (!rc) return;
+[[noreturn]] void raiseStatus(int rc, const std::string& what) {
     py::gil_scoped_acquire gil;
     PyObject* e = PyObject_CallFunction(table().error, "si", what.c_str(), rc);
     if (e) {
@@ -123,6 +122,10 @@ void check(int rc, const std::string& what) {
         Py_DECREF(e);
     }
     raisePython();
+}
+template <class What>   // what(): the call's text, made for a failure alone
+void check(int rc, What&& what) {
+    if (rc) raiseStatus(rc, what());
 }
 
 // ------------------------------------------------------------------ what is taken here
@@ -159,7 +162,7 @@ Tensor execC2C(const Tensor& in, int64_t direction, double scale) {
     const Plan p = planFor(x.get_device(), false, n);
     check(bfly_plan_exec_c2c_async(p->plan, x.data_ptr(), y.data_ptr(), (uint32_t)n, (uint64_t)batch, (int)direction,
                                    (float)scale, streamOf(x)),
-          text("exec_c2c", n, batch));
+          [&] { return text("exec_c2c", n, batch); });
     return y;
 }
 
@@ -176,8 +179,8 @@ Tensor execAxis(const Tensor& in, int64_t dim, int64_t direction, double scale) 
     const Plan p = planFor(x.get_device(), false, n);
     check(bfly_plan_exec_c2c_axis_async(p->plan, x.data_ptr(), y.data_ptr(), (uint32_t)n, (uint64_t)outer,
                                         (uint64_t)inner, (int)direction, (float)scale, streamOf(x)),
-          "exec_c2c_axis(n=" + std::to_string(n) + ", outer=" + std::to_string(outer) + ", inner=" +
-              std::to_string(inner) + ")");
+          [&] { return "exec_c2c_axis(n=" + std::to_string(n) + ", outer=" + std::to_string(outer) + ", inner=" +
+              std::to_string(inner) + ")"; });
     return y;
 }
 
@@ -189,8 +192,8 @@ Tensor exec2D(const Tensor& in, int64_t direction, double scale) {
     const Plan p = planFor(x.get_device(), false, nx);
     check(bfly_plan_exec_c2c_2d_async(p->plan, x.data_ptr(), y.data_ptr(), (uint32_t)ny, (uint32_t)nx,
                                       (uint64_t)batch, (int)direction, (float)scale, streamOf(x)),
-          "exec_c2c_2d(ny=" + std::to_string(ny) + ", nx=" + std::to_string(nx) + ", batch=" +
-              std::to_string(batch) + ")");
+          [&] { return "exec_c2c_2d(ny=" + std::to_string(ny) + ", nx=" + std::to_string(nx) + ", batch=" +
+              std::to_string(batch) + ")"; });
     return y;
 }
 
@@ -209,7 +212,7 @@ Tensor execR2C(const Tensor& in, double edge, double inside) {
     const Plan p = planFor(x.get_device(), true, n);
     check(bfly_plan_exec_r2c_async(p->plan, x.data_ptr(), y.data_ptr(), (uint32_t)n, (uint64_t)batch, (float)edge,
                                    (float)inside, streamOf(x)),
-          text("exec_r2c", n, batch));
+          [&] { return text("exec_r2c", n, batch); });
     return y;
 }
 
@@ -221,7 +224,7 @@ Tensor execC2R(const Tensor& in, int64_t n, double edge, double inside, double s
     const Plan p = planFor(x.get_device(), true, n);
     check(bfly_plan_exec_c2r_async(p->plan, x.data_ptr(), y.data_ptr(), (uint32_t)n, (uint64_t)batch, (float)edge,
                                    (float)inside, (float)scale, streamOf(x)),
-          text("exec_c2r", n, batch));
+          [&] { return text("exec_c2r", n, batch); });
     return y;
 }
 
@@ -233,8 +236,8 @@ Tensor execR2C2D(const Tensor& in, double scale) {
     const Plan p = planFor(x.get_device(), true, nx);
     check(bfly_plan_exec_r2c_2d_async(p->plan, x.data_ptr(), y.data_ptr(), (uint32_t)ny, (uint32_t)nx,
                                       (uint64_t)(x.numel() / (ny * nx)), (float)scale, streamOf(x)),
-          "exec_r2c_2d(ny=" + std::to_string(ny) + ", nx=" + std::to_string(nx) + ", batch=" +
-              std::to_string(x.numel() / (ny * nx)) + ")");
+          [&] { return "exec_r2c_2d(ny=" + std::to_string(ny) + ", nx=" + std::to_string(nx) + ", batch=" +
+              std::to_string(x.numel() / (ny * nx)) + ")"; });
     return y;
 }
 
@@ -258,7 +261,7 @@ Tensor execStft(const Tensor& x, int64_t n, int64_t hop, bool center, const Tens
     uint64_t got = 0;
     check(bfly_plan_exec_stft_async(p->plan, x.data_ptr(), y.data_ptr(), (uint32_t)n, (uint64_t)signals,
                                     (uint64_t)length, (uint32_t)hop, center, windowPtr(window), &got, streamOf(x)),
-          frameText("exec_stft", n, "signals", signals, "length", length, hop));
+          [&] { return frameText("exec_stft", n, "signals", signals, "length", length, hop); });
     return y;
 }
 
@@ -270,7 +273,7 @@ Tensor execIstft(const Tensor& spec, int64_t n, int64_t hop, bool center, const 
     check(bfly_plan_exec_istft_async(p->plan, spec.data_ptr(), y.data_ptr(), (uint32_t)n, (uint64_t)signals,
                                      (uint32_t)frames, (uint32_t)hop, center, windowPtr(window), (uint64_t)outLen,
                                      (float)scale, streamOf(spec)),
-          frameText("exec_istft", n, "signals", signals, "frames", frames, hop));
+          [&] { return frameText("exec_istft", n, "signals", signals, "frames", frames, hop); });
     return y;
 }
 
@@ -282,7 +285,7 @@ Tensor execStftAdjoint(const Tensor& grad, int64_t n, int64_t hop, bool center, 
     const Plan p = planFor(g.get_device(), true, n);
     check(bfly_plan_exec_stft_backward_async(p->plan, g.data_ptr(), gx.data_ptr(), (uint32_t)n, (uint64_t)signals,
                                              (uint64_t)length, (uint32_t)hop, center, windowPtr(window), streamOf(g)),
-          frameText("exec_stft_backward", n, "signals", signals, "length", length, hop));
+          [&] { return frameText("exec_stft_backward", n, "signals", signals, "length", length, hop); });
     return gx;
 }
 
@@ -294,8 +297,8 @@ Tensor execIstftAdjoint(const Tensor& grad, int64_t n, int64_t hop, bool center,
     check(bfly_plan_exec_istft_backward_async(p->plan, g.data_ptr(), gs.data_ptr(), (uint32_t)n, (uint64_t)g.size(0),
                                               (uint32_t)frames, (uint32_t)hop, center, windowPtr(window),
                                               (uint64_t)g.size(1), (float)scale, streamOf(g)),
-          "exec_istft_backward(n=" + std::to_string(n) + ", frames=" + std::to_string(frames) + ", hop=" +
-              std::to_string(hop) + ")");
+          [&] { return "exec_istft_backward(n=" + std::to_string(n) + ", frames=" + std::to_string(frames) + ", hop=" +
+              std::to_string(hop) + ")"; });
     return gs;
 }
 
