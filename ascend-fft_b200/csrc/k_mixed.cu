@@ -100,8 +100,11 @@ MixedShape mixedShape(const MixedRadix& plan) {
     m.smem = m.rows * 2 * m.len * 8;
     const int warps = (m.rows * m.T + 31) / 32;   // at 64 registers a thread 32 warps per SM
     // short rows, whose threads do little but load and store, ask for nothing ahead (us at 2^23 values
-    // with and without: n = 7 41.5 / 39.0, 10 47.3 / 45.2, 18 39.1 / 36.5, 30 47.6 / 45.2; n = 60 34.0 / 38.1)
-    m.args.ahead = plan.n < 32 ? 0 : dev::prefetch_ahead(std::max(1, std::min(32 / warps, kMixedMaxSmem / m.smem)));
+    // with and without: n = 7 41.5 / 39.0, 10 47.3 / 45.2, 18 39.1 / 36.5, 30 47.6 / 45.2; n = 60 34.0 / 38.1), but
+    // for the shortest (n = 3 33.9 / 35.3, 4 28.8 / 30.9, 5 27.2 / 28.9)
+    m.args.ahead = plan.n >= 6 && plan.n < 32
+                       ? dev::kNoAhead
+                       : dev::prefetch_ahead(std::max(1, std::min(32 / warps, kMixedMaxSmem / m.smem)));
     return m;
 }
 

@@ -44,7 +44,7 @@ struct MixedArgs {
     // R_0 < 16, meet a second one in a half-warp), and a pad would cost two instructions an access
     int pad0;
     unsigned magic0;   // ceil(2^32 / pad0), 0 when pad0 = 0
-    unsigned ahead;    // CTAs between a CTA and the one whose input it asks for (prefetch_l2); 0: none
+    unsigned ahead;    // CTAs between a CTA and the one whose input it asks for (prefetch_l2), or kNoAhead
 };
 
 // Threads per row: T butterflies at a time, so a pass of n/R takes ceil(n / (R T)) rounds of which
@@ -81,10 +81,12 @@ constexpr int mixedThreads(int n, const int* radix, int passes) {
     return best;
 }
 
+// Past the end of every grid: a test of its own in the kernels cost 4 % at n = 297.
+constexpr unsigned kNoAhead = 0x7fffffffu;
 // A CTA's share of a later CTA's input: `rows` rows of `bytes` bytes, the array ending at `end`.
 __device__ __forceinline__ void mixed_load_ahead(const void* in, const MixedArgs& a, int rows, size_t bytes,
                                                  uint64_t batch) {
-    if (!a.ahead || blockIdx.x + a.ahead >= gridDim.x) return;
+    if (blockIdx.x + a.ahead >= gridDim.x) return;
     const char* base = static_cast<const char*>(in);
     const char* p = base + ((uint64_t)blockIdx.x + a.ahead) * rows * bytes;
     const char* last = p + rows * bytes < base + batch * bytes ? p + rows * bytes : base + batch * bytes;
